@@ -662,3 +662,43 @@ def test_scf_ne_sor_reproduces_reference_trajectory():
     """Ne (ne/set-01): 4 orbitals incl. 1pi, SOR for orbitals and potentials,
     1432 printed orbital-energy lines and 52540 sweeps."""
     test_scf_sor_decks_reproduce_reference_trajectory("ne_set01", None)
+
+
+def _grid_deck(nnu, nmu):
+    """He on an nnu x nmu grid."""
+    lines = [ln for ln in golden_deck("he_set01").splitlines() if not ln.strip().lower().startswith(("grid", "stop"))]
+    return "\n".join(lines + [f"grid {nnu} {nmu} 25.0", "stop"]) + "\n"
+
+
+# one job (four lanes per point in a step) and 40 (two launches; one lane per
+# point on the larger grid), the smallest grid, more sweeps than a warp has lanes
+@pytest.mark.parametrize("nnu,nmu,njobs,nsweeps", [(31, 31, 1, 1), (31, 31, 40, 3), (31, 61, 3, 35), (91, 121, 40, 10),
+                                                   (121, 91, 7, 2)])
+@pytest.mark.parametrize("form", ["sor", "fp64"])
+@pytest.mark.parametrize("isym", [1, -1])
+def test_wavefront_sweeps_bitexact(ctx, nnu, nmu, njobs, nsweeps, form, isym):
+    """The FP64 wavefront sweeps against the oracle's sequential ones, bit for
+    bit, on functions of no symmetry and every magnitude."""
+    torch = pytest.importorskip("torch")
+    oc = Case(_grid_deck(nnu, nmu))
+    c, g = _grid(ctx, _grid_deck(nnu, nmu))
+    assert (c.nnu, c.nmu) == (nnu, nmu)
+    rng = np.random.default_rng(nnu * nmu + njobs)
+    omega, dev = oc.omega()[0], torch.device("cuda:0")
+    lhs = oc.fock(1)[0] + oc.coeffs()[5]
+    kept, jobs, refs = [], [], []
+    for k in range(njobs):
+        u = oc.putin(isym, rng.standard_normal(nnu * nmu) * 10.0 ** rng.integers(-200, 3))
+        rhs = rng.standard_normal(nnu * nmu)
+        refs.append(oc.sweep(0 if form == "sor" else 1, isym, nsweeps, omega, u, lhs, rhs, oc.suppl(0), oc.suppl(2)))
+        kept.append([torch.tensor(x, device=dev) for x in (u, lhs, rhs)])
+        jobs.append(xg.Job(u=kept[-1][0].data_ptr(), lhs=kept[-1][1].data_ptr(), rhs=kept[-1][2].data_ptr(), omega=omega,
+                           isym=isym, kind=0))
+    torch.cuda.synchronize()
+    xg.relax(ctx, g, jobs, nsweeps, xg.SOR if form == "sor" else xg.FP64)
+    ctx.synchronize()
+    sl = np.s_[4:nmu + 4, 4:nnu + 4]
+    for k, (b, ref) in enumerate(zip(kept, refs)):
+        got, exp = (x.reshape(nmu + 8, nnu + 8)[sl] for x in (b[0].cpu().numpy(), ref))
+        assert np.array_equal(got, exp), (k, np.abs(got - exp).max())
+    g.close()

@@ -336,14 +336,15 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
     }
   const void *tmp;
   int rc = X2G_OK;
-#define UP(vec, field)                                                                  \
+#define UPTO(vec, dest)                                                                 \
   do {                                                                                  \
     if ((rc = upload(gr, vec.data(), vec.size() * sizeof(vec[0]), &tmp)) != X2G_OK) { \
       x2g_grid_destroy(gr);                                                             \
       return rc;                                                                        \
     }                                                                                   \
-    d.field = static_cast<decltype(d.field)>(tmp);                                     \
+    dest = static_cast<decltype(dest)>(tmp);                                          \
   } while (0)
+#define UP(vec, field) UPTO(vec, d.field)
   UP(h.borb_mu, borb_mu);
   UP(h.bpot_mu, bpot_mu);
   UP(h.f3_mu, f3_mu);
@@ -377,13 +378,21 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
   UP(h.pts_rc, pts_rc);
   UP(h.st_pts, st_pts);
   UP(h.st_off, st_off);
-  UP(h.sor_pts, sor_pts);
-  UP(h.sor_off, sor_off);
-  UP(h.sor_bpts, sor_bpts);
-  UP(h.sor_boff, sor_boff);
-  d.sor_nlev = h.sor_nlev;
-  d.sor_nblev = h.sor_nblev;
-  d.sor_delta = h.sor_delta;
+  const WaveHost *waves[2] = {&h.sor, &h.mcsor};
+  WaveDev *wave_dev[2] = {&d.sor, &d.mcsor};
+  for (int k = 0; k < 2; ++k) {
+    const WaveHost &w = *waves[k];
+    WaveDev &wd = *wave_dev[k];
+    std::vector<int2> e(w.pts.size());
+    for (size_t q = 0; q < e.size(); ++q) e[q] = make_int2(w.pts[q], w.mask[q]);
+    UPTO(e, wd.pts);
+    UPTO(w.off, wd.off);
+    UPTO(w.bpts, wd.bpts);
+    UPTO(w.boff, wd.boff);
+    wd.nlev = w.nlev;
+    wd.nblev = w.nblev;
+    wd.delta = w.delta;
+  }
   for (int k = 0; k <= HostGrid::kBandRuns; ++k) d.st_rows[k] = h.st_rows[k];
   d.cl_size = h.cl_size;
   d.cl_maxrows = h.cl_maxrows;
@@ -418,6 +427,7 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
   UP(cmp, cmu_pot);
   UP(cnu, cnu);
 #undef UP
+#undef UPTO
   {
     double *exm = nullptr, *asy = nullptr;
     cudaError_t e = cudaMalloc(&exm, size_t(40) * h.mxsize * sizeof(double));

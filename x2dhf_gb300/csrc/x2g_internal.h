@@ -30,6 +30,24 @@ constexpr int kPhaseWords = 352, kPhaseBlocks = 320, kPhaseStride = 32;
 constexpr int kBarWords = kPhaseWords + kPhaseBlocks * kPhaseStride;
 
 // ----------------------------------------------------------------------
+// A sequential sweep over a list of points as a pipelined wavefront: an
+// interior point's level is 1 + the largest level of its stencil neighbours
+// earlier in the list (their new values are read), an axis point's level 1 +
+// the largest level of the points its extrapolation reads (the corners read
+// the mu=1 row); sweep s of a point runs at step level + s * delta.  pts /
+// bpts hold the interior / axis points by level, packed (ext row << 16) | ext
+// col, with offsets off[nlev + 1] / boff[nblev + 1].
+// ----------------------------------------------------------------------
+struct WaveHost {
+  int nlev = 0, nblev = 0, delta = 0;
+  std::vector<int> pts, off, bpts, boff;
+  // per entry of pts the stencil neighbours earlier in the list, bit 4 (k-1)
+  // + {0: -k, 1: +k, 2: -k rows, 3: +k rows}; bits 16..18: the point is the
+  // fifth of the extrapolation of the mu=1 row, nu=1 or nu=nni column
+  std::vector<int> mask;
+};
+
+// ----------------------------------------------------------------------
 // Host-side grid: every table the relaxation path reads, built with the
 // reference's formulas (initCBAllocArrays.F90 initCBlocks:813-858,
 // initSuppl:1636-2051).  Indices are 0-based: nu j in [0,nni), mu i in
@@ -88,19 +106,24 @@ struct HostGrid {
   static constexpr int kBandRuns = 16;
   std::vector<int> st_pts, st_off;
   int st_rows[kBandRuns + 1] = {};
-  // list-order SOR (sor, sormcsor.F90:20-132) as a pipelined wavefront: an
-  // interior point's SOR level is 1 + the largest level of its stencil
-  // neighbours earlier in the list (their new values are read), an axis
-  // point's level 1 + the largest level of the points its extrapolation
-  // reads (the corners read the mu=1 row); sweep s of a point runs at step
-  // level + s * sor_delta.  sor_pts / sor_bpts hold the interior / axis
-  // points by level, packed (ext row << 16) | ext col, with offsets
-  // sor_off[sor_nlev + 1] / sor_boff[sor_nblev + 1]
-  int sor_nlev = 0, sor_nblev = 0, sor_delta = 0;
-  std::vector<int> sor_pts, sor_off, sor_bpts, sor_boff;
+  // the FP64 sweeps' wavefront schedules (build_wave_schedule): list-order
+  // SOR over the "middle" list (sor, sormcsor.F90:20-132), and MCSOR as the
+  // same sweep over the list colour after colour (mcsor, :143-386)
+  WaveHost sor, mcsor;
 };
 
 std::string build_host_grid(HostGrid &g, int nni, int nmu, double r, double rinf, double z1, double z2, int mpole);
+
+// ----------------------------------------------------------------------
+// Wavefront schedule on the device: interior points by level ((ext row << 16)
+// | ext col, and the bits of the neighbours earlier in the list) and axis
+// points by level, with their offsets.
+// ----------------------------------------------------------------------
+struct WaveDev {
+  const int2 *pts;
+  const int *off, *bpts, *boff;
+  int nlev, nblev, delta;
+};
 
 // ----------------------------------------------------------------------
 // Device view of a grid, passed by value to kernels.
@@ -121,8 +144,7 @@ struct GridDev {
   const int *cl_tile0, *cl_row0, *cl_pts, *cl_off;
   const int *st_pts, *st_off;
   int st_rows[17];
-  const int *sor_pts, *sor_off, *sor_bpts, *sor_boff;
-  int sor_nlev, sor_nblev, sor_delta;
+  WaveDev sor, mcsor;
   // FP32 copies of the coefficient tables for the mixed form
   const float *borb_mu32, *bpot_mu32, *d_nu32;
   const double *e_mu, *e_nu;
@@ -149,8 +171,14 @@ struct JobDev {
   const double *lhs;
   const double *rhs;
   const double *psa, *psb;
-  double *rhs_buf;  // materialised rhs for potentials
-  float *e32;       // mixed: FP32 extended correction
+  union {
+    double *rhs_buf;  // FP64: materialised rhs of a potential
+    double *pairs;    // wavefront: (lhs, rhs) by plain index
+  };
+  union {
+    float *e32;          // mixed: FP32 extended correction
+    ulonglong2 *tagged;  // wavefront: (value, sweeps done) by ext index
+  };
   float *r32, *w32; // mixed: FP32 residual and omega / diagonal
   float2 *rw;       // mixed, persistent-band sweep: (residual, omega / diagonal) in st_pts order
   double omega;
@@ -214,7 +242,7 @@ struct x2g_ctx {
   int band_blocks = 0;          // co-resident blocks for that size
   int band_sm_smem = 0;         // shared memory per SM
   int f64_blocks = -1;          // co-resident blocks of the cooperative FP64 sweep on this device
-  int sor_blocks = -1;          // co-resident blocks of the cooperative list-order SOR sweep
+  int wave_ok = -1;             // the wavefront kernels can be co-resident, one block per SM
   int ortho_blocks = -1;        // co-resident blocks of the one-launch orthonormalisation
   int gram_blocks = -1;         // co-resident blocks of its Gram-matrix form
   int gram_ortho = 0;           // batch mode 2: orthonormalise in rounds (0) or through the Gram matrix (1)

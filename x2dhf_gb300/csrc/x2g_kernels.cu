@@ -372,77 +372,431 @@ __global__ void __launch_bounds__(kThreads) k_mcsor_f64(GridDev g, const __grid_
 }
 
 // ----------------------------------------------------------------------
-// List-order SOR (sormcsor.F90:20-132) as a pipelined wavefront over all
-// jobs of the launch: step t updates, for every sweep s still running, the
-// interior points of SOR level t - s * delta and the axis points whose
+// FP64 sweeps as a dataflow wavefront (list-order SOR, sormcsor.F90:20-132,
+// over the reference's list): step t holds, for every sweep s still running,
+// the interior points of level t - s * delta and the axis points whose
 // extrapolation after sweep s belongs to that level (the host schedule,
-// build_sor_schedule, proves these updates independent and every read
-// value current), then all blocks meet at the grid barrier.  Reference
-// arithmetic order (relax_f64); a potential's rhs = psa psb g and lhs = f3
-// (+ idel^2 e) are formed per point with the same roundings as
-// relaxPots.F90:81-95.  Ghost cells are refreshed once before the first
-// sweep (putin) and stay fixed, as in the reference.
+// build_wave_schedule, proves the updates of a step independent and every
+// read value current).  Reference arithmetic order, as relax_f64.
+//
+// There is no barrier between steps.  The launch keeps every value together
+// with its tag, the number of sweeps it has been through, in one 16-byte
+// word that is read and written whole; an update waits until the values it
+// reads carry the tags its list position asks for (the number of the sweep,
+// one more for the points earlier in the list).  Values are not overwritten
+// too early: a stencil neighbour reads and is read, so the tags that order
+// the new values order the old ones too; the only reads that go one way, the
+// fifth point of an axis extrapolation and the mu=1 row's corner, are
+// checked in the opposite direction as well (wait_value).  Every warp takes
+// its items in step order, so the earliest unfinished update never waits.
+//
+// What bounds it: the dependent chain of a step.  One FP64 instruction of a
+// warp takes ~64 cycles here whatever its active lanes, so kSplit = 4 lanes
+// share one point of a narrow step: each forms one of the four derivative
+// sums (11 instructions instead of 44 in a row) and the shuffled sums are
+// combined in the reference's order; wide steps (kSplit = 1) take a point
+// per lane, which issues the fewest FP64 instructions.  SOR, 10 sweeps of one
+// 331 x 481 orbital (481 steps): 2.26 ms, 9400 cycles a step of which 2240
+// are its FP64 chain, most of the rest the way of a value through L2; 21.8 ms
+// with a grid barrier after every step and the sweeps of a step looked up one
+// after the other.
 // ----------------------------------------------------------------------
-__device__ __forceinline__ void sor_point(const GridDev &g, const JobDev &J, int rc) {
-  const int row = rc >> 16, col = rc & 0xffff, ij = row * g.n8 + col;
-  const int mu = row - 4, nu = col - 4, ik = mu * g.nni + nu;
-  double lhs, rhs;
-  if (J.kind == 1) {
-    lhs = (J.idel2 == 0.0) ? g.f3_mu[mu] : A(g.f3_mu[mu], M(J.idel2, g.e[ik]));
-    rhs = M(M(ldcg(J.psa + ij), ldcg(J.psb + ij)), g.g[ik]);
-  } else {
-    lhs = J.lhs[ik];
-    rhs = J.rhs[ik];
-  }
-  const double *bt = (J.kind >= 1) ? g.bpot_mu : g.borb_mu;
-  relax_f64(J.u, ij, g, bt[mu], g.d_nu[nu], lhs, rhs, J.omega, 1.0 - J.omega);
+constexpr int kWaveThreads = 512;
+constexpr size_t kWaveSmem = 47 * 1024;  // level offsets held in shared memory, within the default cap
+constexpr unsigned kTagFixed = 0x7fffffffu;  // values no sweep changes
+
+struct Tagged {
+  double v;
+  int tag;
+};
+
+__device__ __forceinline__ Tagged ld_tagged(const ulonglong2 *p) {
+  unsigned long long lo, hi;
+  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  return Tagged{__longlong_as_double((long long)lo), int(unsigned(hi))};
 }
 
-__device__ __forceinline__ void sor_axis(const GridDev &g, const JobDev &J, int rc) {
-  const int row = rc >> 16, col = rc & 0xffff, ij = row * g.n8 + col;
-  // the mu=1 row extrapolates along mu, the nu=1 / nu=nni columns along nu
-  const int st = (col == 4) ? 1 : (col == g.nni + 3) ? -1 : g.n8;
-  double *u = J.u;
-  double v = 0.0;
-  if (J.isym == 1)
-    v = A(A(A(A(M(g.exeven[0], ldcg(u + ij + st)), M(g.exeven[1], ldcg(u + ij + 2 * st))),
-              M(g.exeven[2], ldcg(u + ij + 3 * st))),
-            M(g.exeven[3], ldcg(u + ij + 4 * st))),
-          M(g.exeven[4], ldcg(u + ij + 5 * st)));
-  u[ij] = v;
+__device__ __forceinline__ void st_tagged(ulonglong2 *p, double v, int tag) {
+  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%0, %1};\n\tst.relaxed.gpu.global.b128 [%2], q;\n\t}" ::"l"(
+                   __double_as_longlong(v)),
+               "l"((unsigned long long)(unsigned)tag), "l"(p)
+               : "memory");
 }
 
-__global__ void __launch_bounds__(kThreads) k_sor_f64(GridDev g, const __grid_constant__ JobTable jobs, int njobs,
-                                                      int nsweeps, BarrierDev bar, unsigned nblocks) {
-  for (int item = blockIdx.x; item < njobs * g.ntiles; item += gridDim.x) {
-    const int jb = item / g.ntiles;
-    tile_ghosts(g, jobs.j[jb].u, item - jb * g.ntiles, jobs.j[jb].isym);
+// Bounded wait bookkeeping of one warp: false when the launch must stop (its
+// own wait ran out, or another block's did).
+struct WaveWait {
+  unsigned spins = 0;
+  unsigned long long t0 = 0;
+  __device__ __forceinline__ bool again(const BarrierDev &b) {
+    if ((++spins & 63u) != 0 && b.limit_ns != 0) return true;
+    if (*(volatile int *)b.err) return false;
+    const unsigned long long now = globaltimer();
+    if (t0 == 0) t0 = now;
+    if (now - t0 >= b.limit_ns) {
+      atomicCAS(b.err, 0, X2G_ERR_TIMEOUT);
+      return false;
+    }
+    return true;
   }
-  if (!grid_barrier(bar, nblocks)) return;
-  const int D = g.sor_delta, NL = g.sor_nlev, NB = g.sor_nblev;
-  const int T = (nsweeps - 1) * D + (NL > NB ? NL : NB);
-  const int gt = int(blockIdx.x * blockDim.x + threadIdx.x), gs = int(gridDim.x * blockDim.x);
-  for (int t = 0; t < T; ++t) {
-    // the (sweep, level) pairs of this step as one index space over all jobs
-    for (int s = 0; s < nsweeps; ++s) {
-      const int l = t - s * D;
-      if (l < 0) break;
-      if (l < NL) {
-        const int b0 = g.sor_off[l], n = g.sor_off[l + 1] - b0;
-        for (int k = gt; k < n * njobs; k += gs) {
-          const int jb = k / n;
-          sor_point(g, jobs.j[jb], g.sor_pts[b0 + k - jb * n]);
-        }
+};
+
+// One warp's next piece of work: kind 0 interior points, 1 axis points, -1
+// none left.  Every lane (of a group of kSplit) has its own point; lanes
+// past the end of the list have s = -1.
+struct WaveItem {
+  int kind, jb, s;
+  int rc;         // (ext row << 16) | ext col
+  unsigned mask;  // interior points: the bits of HostGrid::sor_mask
+  __device__ __forceinline__ int row() const { return rc >> 16; }
+  __device__ __forceinline__ int col() const { return rc & 0xffff; }
+};
+
+// Walks the steps of the schedule, handing this warp groups wid, wid + nw,
+// ... of each step: first groups of 32 / kSplit interior points, then groups
+// of 32 axis points.  The sweeps that run in a step are looked at by the
+// lanes at once, 32 at a time (counts summed and searched with shuffles): a
+// loop over the sweeps by every lane took longer than the updates
+// themselves (7.3 us a step of 10 sweeps on 331 x 481, all of it here).
+template <int kSplit>
+struct WaveWalk {
+  const int *off, *boff;  // shared memory copies
+  int nlev, nblev, most, delta, nsweeps, njobs, T, wid, nw;
+  int t, lo, hi, grp, ni, na, gi;  // step, its sweeps, next group, interior and axis points, interior groups
+  __device__ __forceinline__ int count(const int *o, int levels, int s) const {
+    const int l = t - s * delta;
+    return (s <= hi && l < levels) ? o[l + 1] - o[l] : 0;
+  }
+  __device__ __forceinline__ void open() {
+    while (hi < nsweeps - 1 && (hi + 1) * delta <= t) ++hi;
+    while (lo * delta + most <= t) ++lo;
+    const int lane = threadIdx.x & 31;
+    ni = na = 0;
+    for (int s = lo; s <= hi; s += 32) {
+      ni += __reduce_add_sync(0xffffffffu, count(off, nlev, s + lane));
+      na += __reduce_add_sync(0xffffffffu, count(boff, nblev, s + lane));
+    }
+    ni *= njobs;
+    na *= njobs;
+    gi = (ni * kSplit + 31) / 32;
+    grp = wid;
+  }
+  __device__ __forceinline__ void start() {
+    t = lo = hi = 0;
+    open();
+  }
+  __device__ __forceinline__ WaveItem next(const WaveDev &w) {
+    WaveItem it;
+    it.kind = -1;
+    it.s = -1;
+    it.jb = 0;
+    it.rc = (4 << 16) | 4;
+    it.mask = 0;
+    while (t < T && grp >= gi + (na + 31) / 32) {
+      if (++t < T) open();
+    }
+    if (t >= T) return it;
+    const int lane = threadIdx.x & 31;
+    const bool axis = grp >= gi;
+    it.kind = axis ? 1 : 0;
+    const int *o = axis ? boff : off;
+    const int levels = axis ? nblev : nlev;
+    // this lane's point: index q of the step, in sweep s and job jb
+    int q = axis ? (grp - gi) * 32 + lane : (grp * 32 + lane) / kSplit;
+    grp += nw;
+    bool found = false;
+    for (int s0 = lo; s0 <= hi; s0 += 32) {
+      int sum = count(o, levels, s0 + lane) * njobs;  // points up to and with sweep s0 + lane
+#pragma unroll
+      for (int d = 1; d < 32; d *= 2) {
+        const int x = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += x;
       }
-      if (l < NB) {
-        const int b0 = g.sor_boff[l], n = g.sor_boff[l + 1] - b0;
-        for (int k = gt; k < n * njobs; k += gs) {
-          const int jb = k / n;
-          sor_axis(g, jobs.j[jb], g.sor_bpts[b0 + k - jb * n]);
-        }
+      // the first sweep whose sum is beyond q
+      int f = 0;
+#pragma unroll
+      for (int d = 16; d > 0; d /= 2)
+        if (__shfl_sync(0xffffffffu, sum, (f + d - 1) & 31) <= q) f += d;
+      const int before = __shfl_sync(0xffffffffu, sum, (f + 31) & 31), all = __shfl_sync(0xffffffffu, sum, 31);
+      if (!found && q < all) {
+        found = true;
+        const int s = s0 + f, l = t - s * delta, k0 = q - (f > 0 ? before : 0), n = o[l + 1] - o[l];
+        const int jb = njobs > 1 ? k0 / n : 0, k = o[l] + k0 - jb * n;
+        it.s = s;
+        it.jb = jb;
+        // the entry is first used when this item's turn comes
+        const int2 e = axis ? make_int2(__ldg(w.bpts + k), 0) : __ldg(w.pts + k);
+        it.rc = e.x;
+        it.mask = unsigned(e.y);
+      }
+      q -= all;
+    }
+    return it;
+  }
+};
+
+// Final value of an update: kept with its tag, and in u after the last sweep.
+__device__ __forceinline__ void wave_store(const JobDev &J, int ij, double v, int s, int nsweeps) {
+  st_tagged(J.tagged + ij, v, s + 1);
+  if (s == nsweeps - 1) J.u[ij] = v;
+}
+
+// Axis extrapolation (sormcsor.F90:94-129): the mu=1 row along mu, the nu=1
+// and nu=nni columns along nu; five values of this sweep.  The mu=1 row's
+// points next to a corner also wait until that corner has read their last
+// value.
+__device__ __forceinline__ bool wave_axis(const GridDev &g, const JobTable &jobs, const WaveItem &it, int nsweeps,
+                                          const BarrierDev &bar) {
+  const JobDev &J = jobs.j[it.jb];
+  const bool on = it.s >= 0;
+  const int row = it.row(), col = it.col(), ij = row * g.n8 + col;
+  const int st = (col == 4) ? 1 : (col == g.nni + 3) ? -1 : g.n8;
+  int back = 0;  // a corner that reads this point
+  if (on && row == 4 && col != 4 && col != g.nni + 3) {
+    if (col <= 9) back = 4 * g.n8 + 4;
+    else if (col >= g.nni - 2) back = 4 * g.n8 + g.nni + 3;
+  }
+  double v[5];
+  bool got = !on;
+  WaveWait ww;
+  for (;;) {
+    if (!got) {
+      bool ok = true;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        const Tagged x = ld_tagged(J.tagged + ij + (k + 1) * st);
+        v[k] = x.v;
+        ok = ok && x.tag > it.s;
+      }
+      if (back) ok = ok && ld_tagged(J.tagged + back).tag >= it.s;
+      got = ok;
+    }
+    if (__all_sync(0xffffffffu, got)) break;
+    if (!__all_sync(0xffffffffu, ww.again(bar))) return false;
+  }
+  if (on) {
+    double r = 0.0;
+    if (J.isym == 1)
+      r = A(A(A(A(M(g.exeven[0], v[0]), M(g.exeven[1], v[1])), M(g.exeven[2], v[2])), M(g.exeven[3], v[3])),
+            M(g.exeven[4], v[4]));
+    wave_store(J, ij, r, it.s, nsweeps);
+  }
+  return true;
+}
+
+// the axis value five points from a point, or 0: an extrapolation's last
+// point is the only one that does not read it back (flags of
+// HostGrid::sor_mask); which: 0 along mu, 1 along nu
+__device__ __forceinline__ int fifth_reader(const GridDev &g, unsigned mask, int ij, int which) {
+  if (which == 0) return (mask & 0x10000u) ? ij - 5 * g.n8 : 0;
+  return (mask & 0x20000u) ? ij - 5 : (mask & 0x40000u) ? ij + 5 : 0;
+}
+
+// (lhs, rhs), b(mu) and d(nu) of an interior point
+struct WaveCoef {
+  double2 lr;
+  double b, d;
+  __device__ __forceinline__ WaveCoef(const GridDev &g, const JobDev &J, const WaveItem &it) {
+    const int mu = it.row() - 4, nu = it.col() - 4;
+    lr = __ldcg(reinterpret_cast<const double2 *>(J.pairs) + mu * g.nni + nu);
+    b = __ldg((J.kind >= 1 ? g.bpot_mu : g.borb_mu) + mu);
+    d = __ldg(g.d_nu + nu);
+  }
+};
+
+// interior points, four lanes each: roles 0 / 1 the second / first mu
+// derivative, 2 / 3 the nu derivatives
+__device__ __forceinline__ bool wave_points4(const GridDev &g, const JobTable &jobs, const WaveItem &it, int nsweeps,
+                                             const BarrierDev &bar, const double (&cf)[4]) {
+  const JobDev &J = jobs.j[it.jb];
+  const bool on = it.s >= 0;
+  const int role = threadIdx.x & 3, st = (role < 2) ? g.n8 : 1, bit = (role < 2) ? 2 : 0;
+  double m[4], p[4], uc = 0.0;
+  unsigned miss = on ? 0x3ffu : 0u;  // values still to come: 8 neighbours, the centre, a fifth reader
+  const int ij = it.row() * g.n8 + it.col();
+  const WaveCoef co(g, J, it);
+  const int fifth = (role == 1) ? 0 : fifth_reader(g, it.mask, ij, role == 0 ? 0 : 1);
+  if (!fifth) miss &= ~0x200u;
+  WaveWait ww;
+  for (;;) {
+    Tagged x[4], y[4], c;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (miss & (1u << q)) x[q] = ld_tagged(J.tagged + ij - (4 - q) * st);
+      if (miss & (16u << q)) y[q] = ld_tagged(J.tagged + ij + (4 - q) * st);
+    }
+    if (miss & 256u) c = ld_tagged(J.tagged + ij);
+    if (miss & 512u) {
+      if (ld_tagged(J.tagged + fifth).tag >= it.s) miss &= ~512u;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = 4 * (3 - q) + bit;
+      if ((miss & (1u << q)) && x[q].tag >= it.s + int((it.mask >> e) & 1u)) {
+        m[q] = x[q].v;
+        miss &= ~(1u << q);
+      }
+      if ((miss & (16u << q)) && y[q].tag >= it.s + int((it.mask >> (e + 1)) & 1u)) {
+        p[q] = y[q].v;
+        miss &= ~(16u << q);
       }
     }
-    if (t + 1 < T && !grid_barrier(bar, nblocks)) return;
+    if ((miss & 256u) && c.tag >= it.s) {
+      uc = c.v;
+      miss &= ~256u;
+    }
+    if (__all_sync(0xffffffffu, miss == 0)) break;
+    if (!__all_sync(0xffffffffu, ww.again(bar))) return false;
+    // values at distance 3 or 4 still missing: this warp is steps early and
+    // must not take the load units from the warps whose turn it is
+    if (__any_sync(0xffffffffu, miss & 0x33u)) __nanosleep(400);
+    else if (__any_sync(0xffffffffu, miss & 0x44u)) __nanosleep(100);
+  }
+  // a - b as a + (-b): the same rounding
+  const long long flip = (role & 1) ? (1ll << 63) : 0;
+  double a[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) a[q] = A(m[q], __longlong_as_double(__double_as_longlong(p[q]) ^ flip));
+  double t = A(A(A(M(cf[0], a[0]), M(cf[1], a[1])), M(cf[2], a[2])), M(cf[3], a[3]));
+  t = M(role == 1 ? co.b : role == 3 ? co.d : 1.0, t);
+  const int base = threadIdx.x & 28;
+  const double ddmi2 = __shfl_sync(0xffffffffu, t, base), bddmi1 = __shfl_sync(0xffffffffu, t, base + 1);
+  const double ddni2 = __shfl_sync(0xffffffffu, t, base + 2), dddni1 = __shfl_sync(0xffffffffu, t, base + 3);
+  if (on) {
+    const double omega = J.omega, omega1 = 1.0 - J.omega;
+    const double cc = A(A(A(ddmi2, bddmi1), ddni2), dddni1);
+    const double v = A(D(M(omega, S(co.lr.y, cc)), co.lr.x), M(omega1, uc));
+    if (role == 0) wave_store(J, ij, v, it.s, nsweeps);
+  }
+  return true;
+}
+
+// interior points, one lane each
+__device__ __forceinline__ bool wave_points1(const GridDev &g, const JobTable &jobs, const WaveItem &it, int nsweeps,
+                                             const BarrierDev &bar) {
+  const JobDev &J = jobs.j[it.jb];
+  const bool on = it.s >= 0;
+  double n[16], uc = 0.0;
+  const int ij = it.row() * g.n8 + it.col();
+  const WaveCoef co(g, J, it);
+  const int f0 = fifth_reader(g, it.mask, ij, 0), f1 = fifth_reader(g, it.mask, ij, 1);
+  bool got = !on;
+  WaveWait ww;
+  for (;;) {
+    if (!got) {
+      bool ok = true;
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const int k = e / 4 + 1, st = (e & 2) ? k * g.n8 : k;
+        const Tagged x = ld_tagged(J.tagged + ((e & 1) ? ij + st : ij - st));
+        n[e] = x.v;
+        ok = ok && x.tag >= it.s + int((it.mask >> e) & 1u);
+      }
+      const Tagged c = ld_tagged(J.tagged + ij);
+      uc = c.v;
+      ok = ok && c.tag >= it.s;
+      if (f0) ok = ok && ld_tagged(J.tagged + f0).tag >= it.s;
+      if (f1) ok = ok && ld_tagged(J.tagged + f1).tag >= it.s;
+      got = ok;
+    }
+    if (__all_sync(0xffffffffu, got)) break;
+    if (!__all_sync(0xffffffffu, ww.again(bar))) return false;
+  }
+  if (on) {
+    const double ddmi2 = A(A(A(M(g.dmu2[0], A(n[14], n[15])), M(g.dmu2[1], A(n[10], n[11]))),
+                             M(g.dmu2[2], A(n[6], n[7]))), M(g.dmu2[3], A(n[2], n[3])));
+    const double ddmi1 = A(A(A(M(g.dmu1[0], S(n[14], n[15])), M(g.dmu1[1], S(n[10], n[11]))),
+                             M(g.dmu1[2], S(n[6], n[7]))), M(g.dmu1[3], S(n[2], n[3])));
+    const double ddni2 = A(A(A(M(g.dni2[0], A(n[12], n[13])), M(g.dni2[1], A(n[8], n[9]))),
+                             M(g.dni2[2], A(n[4], n[5]))), M(g.dni2[3], A(n[0], n[1])));
+    const double ddni1 = A(A(A(M(g.dni1[0], S(n[12], n[13])), M(g.dni1[1], S(n[8], n[9]))),
+                             M(g.dni1[2], S(n[4], n[5]))), M(g.dni1[3], S(n[0], n[1])));
+    const double omega = J.omega, omega1 = 1.0 - J.omega;
+    const double cc = A(A(A(ddmi2, M(co.b, ddmi1)), ddni2), M(co.d, ddni1));
+    wave_store(J, ij, A(D(M(omega, S(co.lr.y, cc)), co.lr.x), M(omega1, uc)), it.s, nsweeps);
+  }
+  return true;
+}
+
+template <int kSplit>
+__global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev w, const __grid_constant__ JobTable jobs,
+                                                             int njobs, int nsweeps, BarrierDev bar, unsigned nblocks) {
+  extern __shared__ int s_off[];
+  const int nt = int(gridDim.x * blockDim.x), id = int(blockIdx.x * blockDim.x + threadIdx.x);
+  for (int k = threadIdx.x; k <= w.nlev; k += blockDim.x) s_off[k] = w.off[k];
+  for (int k = threadIdx.x; k <= w.nblev; k += blockDim.x) s_off[w.nlev + 1 + k] = w.boff[k];
+  // the tagged copy of every function, its ghost cells refreshed as putin
+  // does (in u too), and the (lhs, rhs) pairs: a potential's lhs = f3 +
+  // idel^2 e and rhs = psa psb g with the roundings of relaxPots.F90:81-95
+  for (int jb = 0; jb < njobs; ++jb) {
+    const JobDev &J = jobs.j[jb];
+    for (int k = id; k < g.next; k += nt) {
+      const int row = k / g.n8, col = k - row * g.n8;
+      int src = k;
+      if (row >= 4 && row < g.nmu) {
+        if (col < 4) src = row * g.n8 + 8 - col;
+        else if (col > g.nni + 3) src = row * g.n8 + 2 * g.nni + 6 - col;
+      } else if (row < 4 && col >= 4 && col <= g.nni + 3) {
+        src = (8 - row) * g.n8 + col;
+      }
+      double v = ldcg(J.u + src);
+      if (src != k) {
+        if (J.isym != 1) v = -v;
+        J.u[k] = v;
+      }
+      const bool swept = row >= 4 && row < g.nmu && col >= 4 && col <= g.nni + 3;  // interior and axis
+      st_tagged(J.tagged + k, v, swept ? 0 : int(kTagFixed));
+    }
+    double2 *pairs = reinterpret_cast<double2 *>(J.pairs);
+    for (int k = id; k < g.mxsize; k += nt) {
+      double2 lr;
+      if (J.kind == 1) {
+        const int mu = k / g.nni, ij = (mu + 4) * g.n8 + (k - mu * g.nni) + 4;
+        lr.x = (J.idel2 == 0.0) ? g.f3_mu[mu] : A(g.f3_mu[mu], M(J.idel2, g.e[k]));
+        lr.y = M(M(J.psa[ij], J.psb[ij]), g.g[k]);
+      } else {
+        lr = make_double2(J.lhs[k], J.rhs[k]);
+      }
+      pairs[k] = lr;
+    }
+  }
+  if (!grid_barrier(bar, nblocks)) return;
+  WaveWalk<kSplit> walk;
+  walk.off = s_off;
+  walk.boff = s_off + w.nlev + 1;
+  walk.nlev = w.nlev;
+  walk.nblev = w.nblev;
+  walk.delta = w.delta;
+  walk.nsweeps = nsweeps;
+  walk.njobs = njobs;
+  walk.most = w.nlev > w.nblev ? w.nlev : w.nblev;
+  walk.T = (nsweeps - 1) * w.delta + walk.most;
+  walk.wid = int((threadIdx.x >> 5) * gridDim.x + blockIdx.x);  // neighbouring groups on different SMs
+  walk.nw = int(gridDim.x * (blockDim.x >> 5));
+  walk.start();
+  double cf[4];
+  {
+    const int role = threadIdx.x & 3;
+    const double *c = role == 0 ? g.dmu2 : role == 1 ? g.dmu1 : role == 2 ? g.dni2 : g.dni1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) cf[q] = c[q];
+  }
+  WaveItem it = walk.next(w);
+  while (it.kind >= 0) {
+    // the next item's list entry and pair travel while this one waits
+    const WaveItem nx = walk.next(w);
+    bool ok;
+    if (it.kind == 1)
+      ok = wave_axis(g, jobs, it, nsweeps, bar);
+    else if (kSplit == 4)
+      ok = wave_points4(g, jobs, it, nsweeps, bar, cf);
+    else
+      ok = wave_points1(g, jobs, it, nsweeps, bar);
+    if (!ok) return;
+    it = nx;
   }
 }
 
@@ -2607,39 +2961,69 @@ static int relax_batch(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, 
   return X2G_OK;
 }
 
-// List-order SOR: jobs in launches of kParamJobs, each one cooperative
-// wavefront launch; the grid holds as many blocks as the widest step needs.
-static int relax_sor(x2g_ctx *ctx, const x2g_grid *grid, const x2g_job *jobs, int njobs, int nsweeps) {
-  const GridDev &g = grid->d;
-  if (ctx->sor_blocks < 0) {
-    int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_sor_f64, kThreads, 0);
+// FP64 relaxation over the wavefront schedule w, in cooperative launches of
+// at most kParamJobs jobs and kWaveScratch bytes of scratch (the tagged copy
+// and the (lhs, rhs) pairs of a launch's jobs, used by the launches in turn;
+// 32 jobs of 331 x 481 are 167 MB, about what L2 holds, and a launch of one
+// 781 x 1201 job already has points enough in a step to fill the GPU).
+constexpr size_t kWaveScratch = size_t(256) << 20;
+static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2g_job *jobs, int njobs, int nsweeps,
+                      bool profile) {
+  const size_t tagged = (size_t(g.next) * 16 + 255) / 256 * 256, pairs = (size_t(g.mxsize) * 16 + 255) / 256 * 256;
+  const int most =
+      std::max(1, std::min(std::min(njobs, kParamJobs), int(std::min(kWaveScratch / (tagged + pairs), size_t(kParamJobs)))));
+  char *scratch = static_cast<char *>(ctx_workspace(ctx, (tagged + pairs) * size_t(most)));
+  if (!scratch) return set_status(X2G_ERR_ALLOC, "workspace allocation failed");
+  const size_t smem = size_t(w.nlev + w.nblev + 2) * sizeof(int);
+  if (smem > kWaveSmem) return set_status(X2G_ERR_ARG, "grid too large for the wavefront's level table");
+  if (ctx->wave_ok < 0) {
+    int a = 0, b = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, (const void *)k_wave_f64<4>, kWaveThreads, kWaveSmem);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void *)k_wave_f64<1>, kWaveThreads, kWaveSmem);
     if (e != cudaSuccess) return cuda_status(e, "occupancy query");
-    if (per_sm < 1) return set_status(X2G_ERR_CUDA, "cooperative SOR sweep cannot be resident");
-    ctx->sor_blocks = per_sm * ctx->num_sms;
+    ctx->wave_ok = (a >= 1 && b >= 1) ? 1 : 0;
   }
-  int widest = 0;
-  for (int l = 0; l < g.sor_nlev; ++l) widest = std::max(widest, grid->h.sor_off[l + 1] - grid->h.sor_off[l]);
-  for (int b0 = 0; b0 < njobs; b0 += kParamJobs) {
-    const int nb = (njobs - b0 < kParamJobs) ? njobs - b0 : kParamJobs;
+  if (!ctx->wave_ok) return set_status(X2G_ERR_CUDA, "cooperative FP64 sweep cannot be resident");
+  for (int b0 = 0; b0 < njobs; b0 += most) {
+    const int nb = std::min(njobs - b0, most);
     JobTable jt{};
-    for (int i = 0; i < nb; ++i)
+    for (int i = 0; i < nb; ++i) {
       if (!make_job(jobs[b0 + i], jt.j[i])) return set_status(X2G_ERR_ARG, "bad relaxation job");
+      char *p = scratch + (tagged + pairs) * size_t(i);
+      jt.j[i].tagged = reinterpret_cast<ulonglong2 *>(p);
+      jt.j[i].pairs = reinterpret_cast<double *>(p + tagged);
+    }
     cudaError_t err = cudaMemsetAsync(ctx->bar, 0, 2 * sizeof(unsigned), ctx->stream);
     if (err != cudaSuccess) return cuda_status(err, "barrier reset");
     BarrierDev bar{ctx->bar, ctx->bar + 1, reinterpret_cast<int *>(ctx->bar + 2), ctx->wait_limit_ns};
-    const int inflight = std::min(nsweeps, (std::max(g.sor_nlev, g.sor_nblev) + g.sor_delta - 1) / g.sor_delta + 1);
-    const long items = long(nb) * widest * inflight;
-    long want = (items + kThreads - 1) / kThreads;
-    want = std::max(want, long(std::min(nb * g.ntiles, ctx->sor_blocks)));  // the ghost prologue's tiles
-    unsigned nblocks = unsigned(std::min(want, long(ctx->sor_blocks)));
-    if (nblocks < 1) nblocks = 1;
+    // four lanes per point while the average step is narrow: MCSOR, 10
+    // sweeps, four lanes / one lane: 289 / 329 us at 58 points a step and SM
+    // (151 x 241, 2 jobs), 369 / 368 us at 85 (91 x 121, 10 jobs), 507 / 389
+    // us at 145 (151 x 241, 5 jobs)
+    const double steps = double(nsweeps - 1) * w.delta + std::max(w.nlev, w.nblev);
+    const double per_sm = double(nb) * nsweeps * double(g.nni - 2) * double(g.nmu - 5) / steps / ctx->num_sms;
+    x2g_ctx::Pending pe{};
+    if (profile && ctx->profiling) {
+      int rc;
+      if ((rc = take_event(ctx, &pe.a)) || (rc = take_event(ctx, &pe.b))) return rc;
+      pe.precision = 0;
+      pe.points = double(nb) * double(g.nni - 2) * double(g.nmu - 5) * double(nsweeps);
+      cudaEventRecord(pe.a, ctx->stream);
+    }
+    unsigned nblocks = unsigned(ctx->num_sms);
     int nj = nb, ns = nsweeps;
     GridDev gd = g;
-    void *args[] = {&gd, &jt, &nj, &ns, &bar, &nblocks};
-    err = cudaLaunchCooperativeKernel((const void *)k_sor_f64, dim3(nblocks), dim3(kThreads), args, 0, ctx->stream);
-    if (err != cudaSuccess) return cuda_status(err, "cooperative SOR launch");
+    WaveDev wd = w;
+    void *args[] = {&gd, &wd, &jt, &nj, &ns, &bar, &nblocks};
+    err = cudaLaunchCooperativeKernel(per_sm < 85.0 ? (const void *)k_wave_f64<4> : (const void *)k_wave_f64<1>,
+                                      dim3(nblocks), dim3(kWaveThreads), args, smem, ctx->stream);
+    if (err != cudaSuccess) return cuda_status(err, "cooperative FP64 sweep launch");
     ctx->launches += 1;
+    if (profile && ctx->profiling) {
+      cudaEventRecord(pe.b, ctx->stream);
+      ctx->pending.push_back(pe);
+    }
   }
   return X2G_OK;
 }
@@ -2658,7 +3042,7 @@ int cluster_occupancy(x2g_ctx *ctx, x2g_grid *grid, int *plain, int *pot) {
 int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, int nsweeps, int precision) {
   if (njobs <= 0) return X2G_OK;
   if (nsweeps <= 0) return set_status(X2G_ERR_ARG, "nsweeps must be positive");
-  if (precision == X2G_SOR) return relax_sor(ctx, grid, jobs, njobs, nsweeps);
+  if (precision == X2G_SOR) return relax_wave(ctx, grid->d, grid->d.sor, jobs, njobs, nsweeps, false);
   if (precision != X2G_FP64 && precision != X2G_MIXED) return set_status(X2G_ERR_ARG, "unknown relaxation form");
   const GridDev &g = grid->d;
   const bool mixed = (precision == X2G_MIXED);

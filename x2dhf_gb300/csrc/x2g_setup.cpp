@@ -33,8 +33,10 @@ std::vector<double> newton_cotes(int n, double h) {
   return w;
 }
 
-// List-order SOR as a pipelined wavefront.  Sequential SOR over the
-// "middle" list (sormcsor.F90:41-74) followed by the axis extrapolation
+// Sweeps over a list as a pipelined wavefront: list-order SOR over the
+// "middle" list, MCSOR over the same list colour after colour (mcsor's loops
+// i = c, ngrid, 5 one after the other).  A sequential sweep over the list
+// (sormcsor.F90:41-74, 170-386) followed by the axis extrapolation
 // (:94-129) after every sweep is reproduced exactly when every point update
 // and every axis extrapolation of sweep s runs at step level + s * delta and
 // the updates of one step run in any order: a point reads the new values of
@@ -44,12 +46,14 @@ std::vector<double> newton_cotes(int n, double h) {
 // overwritten.  The ghost cells and the mu >= nmu-3 rows stay fixed during a
 // relaxation call.  Every dependency is checked here; a violation refuses
 // the grid.
-std::string build_sor_schedule(HostGrid &g, const std::vector<int> &pos, const int *offs) {
-  const int npts = int(g.order.size()), n8 = g.n8, nni = g.nni, nmu = g.nmu;
+std::string build_wave_schedule(const HostGrid &g, const std::vector<int> &order, const int *offs, WaveHost &w) {
+  const int npts = int(order.size()), n8 = g.n8, nni = g.nni, nmu = g.nmu;
+  std::vector<int> pos(g.next, -1);
+  for (int p = 0; p < npts; ++p) pos[order[p]] = p;
   std::vector<int> L(npts, 0);
   int nlev = 0;
   for (int p = 0; p < npts; ++p) {
-    const int ij = g.order[p];
+    const int ij = order[p];
     int l = 0;
     for (int k = 0; k < 16; ++k) {
       const int q = ij + offs[k];
@@ -79,7 +83,7 @@ std::string build_sor_schedule(HostGrid &g, const std::vector<int> &pos, const i
     for (int k = 1; k <= 5; ++k) {
       const int q = a.ij + k * a.st;
       const int lq = (pos[q] >= 0) ? L[pos[q]] : B[q];
-      if (lq < 0) return "SOR schedule: an axis point reads neither an interior nor an axis point";
+      if (lq < 0) return "schedule: an axis point reads neither an interior nor an axis point";
       b = std::max(b, lq + 1);
     }
     B[a.ij] = b;
@@ -89,7 +93,7 @@ std::string build_sor_schedule(HostGrid &g, const std::vector<int> &pos, const i
   // not yet overwritten by the next
   int delta = 1;
   for (int p = 0; p < npts; ++p) {
-    const int ij = g.order[p];
+    const int ij = order[p];
     for (int k = 0; k < 16; ++k) {
       const int q = ij + offs[k];
       if (q < 0 || q >= g.next) continue;
@@ -105,40 +109,50 @@ std::string build_sor_schedule(HostGrid &g, const std::vector<int> &pos, const i
     }
   // check every dependency at sweeps s and s+1 (step = level + s * delta)
   for (int p = 0; p < npts; ++p) {
-    const int ij = g.order[p];
+    const int ij = order[p];
     for (int k = 0; k < 16; ++k) {
       const int q = ij + offs[k];
       if (q < 0 || q >= g.next) continue;
-      if (pos[q] >= 0 && pos[q] < p && !(L[pos[q]] < L[p])) return "SOR schedule: new value read too early";
+      if (pos[q] >= 0 && pos[q] < p && !(L[pos[q]] < L[p])) return "schedule: new value read too early";
       if (pos[q] > p && !(L[pos[q]] > L[p] && L[pos[q]] < L[p] + delta))
-        return "SOR schedule: old value of a later point not preserved";
-      if (B[q] >= 0 && !(B[q] > L[p] && B[q] < L[p] + delta)) return "SOR schedule: axis value out of order";
+        return "schedule: old value of a later point not preserved";
+      if (B[q] >= 0 && !(B[q] > L[p] && B[q] < L[p] + delta)) return "schedule: axis value out of order";
     }
   }
   for (const Axis &a : ax)
     for (int k = 1; k <= 5; ++k) {
       const int q = a.ij + k * a.st;
       const int lq = (pos[q] >= 0) ? L[pos[q]] : B[q];
-      if (!(lq < B[a.ij] && B[a.ij] < lq + delta)) return "SOR schedule: extrapolation out of order";
+      if (!(lq < B[a.ij] && B[a.ij] < lq + delta)) return "schedule: extrapolation out of order";
     }
-  g.sor_nlev = nlev;
-  g.sor_nblev = nblev;
-  g.sor_delta = delta;
-  g.sor_off.assign(nlev + 1, 0);
-  for (int p = 0; p < npts; ++p) g.sor_off[L[p] + 1]++;
-  for (int l = 0; l < nlev; ++l) g.sor_off[l + 1] += g.sor_off[l];
-  g.sor_pts.assign(npts, 0);
+  w.nlev = nlev;
+  w.nblev = nblev;
+  w.delta = delta;
+  w.off.assign(nlev + 1, 0);
+  for (int p = 0; p < npts; ++p) w.off[L[p] + 1]++;
+  for (int l = 0; l < nlev; ++l) w.off[l + 1] += w.off[l];
+  w.pts.assign(npts, 0);
   {
-    std::vector<int> fill(g.sor_off.begin(), g.sor_off.end() - 1);
-    for (int p = 0; p < npts; ++p) g.sor_pts[fill[L[p]]++] = ((g.order[p] / n8) << 16) | (g.order[p] % n8);
+    std::vector<int> fill(w.off.begin(), w.off.end() - 1);
+    w.mask.assign(npts, 0);
+    for (int p = 0; p < npts; ++p) {
+      const int ij = order[p], at = fill[L[p]]++;
+      w.pts[at] = ((ij / n8) << 16) | (ij % n8);
+      for (int k = 0; k < 16; ++k)  // an interior point's 16 neighbours all lie in the extended array
+        if (pos[ij + offs[k]] >= 0 && pos[ij + offs[k]] < p) w.mask[at] |= 1 << k;
+      // the fifth point of an axis extrapolation
+      if (ij / n8 == 9) w.mask[at] |= 1 << 16;
+      if (ij % n8 == 9) w.mask[at] |= 1 << 17;
+      if (ij % n8 == nni - 2) w.mask[at] |= 1 << 18;
+    }
   }
-  g.sor_boff.assign(nblev + 1, 0);
-  for (const Axis &a : ax) g.sor_boff[B[a.ij] + 1]++;
-  for (int l = 0; l < nblev; ++l) g.sor_boff[l + 1] += g.sor_boff[l];
-  g.sor_bpts.assign(ax.size(), 0);
+  w.boff.assign(nblev + 1, 0);
+  for (const Axis &a : ax) w.boff[B[a.ij] + 1]++;
+  for (int l = 0; l < nblev; ++l) w.boff[l + 1] += w.boff[l];
+  w.bpts.assign(ax.size(), 0);
   {
-    std::vector<int> fill(g.sor_boff.begin(), g.sor_boff.end() - 1);
-    for (const Axis &a : ax) g.sor_bpts[fill[B[a.ij]]++] = ((a.ij / n8) << 16) | (a.ij % n8);
+    std::vector<int> fill(w.boff.begin(), w.boff.end() - 1);
+    for (const Axis &a : ax) w.bpts[fill[B[a.ij]]++] = ((a.ij / n8) << 16) | (a.ij % n8);
   }
   return "";
 }
@@ -623,7 +637,13 @@ static std::string build_schedule(HostGrid &g) {
     if (band_of(ra) != band_of(rb)) return "schedule check: dependency crosses a tile";
     if (!(lev[d.second] > lev[d.first])) return "schedule check: level order violated";
   }
-  return build_sor_schedule(g, pos, offs);
+  std::string msg = build_wave_schedule(g, g.order, offs, g.sor);
+  if (!msg.empty()) return msg;
+  std::vector<int> by_colour;
+  by_colour.reserve(g.order.size());
+  for (int c = 0; c < 5; ++c)
+    for (int p = c; p < npts; p += 5) by_colour.push_back(g.order[p]);
+  return build_wave_schedule(g, by_colour, offs, g.mcsor);
 }
 
 
@@ -671,13 +691,8 @@ void copy_schedule(HostGrid &to, const HostGrid &from) {
   to.st_pts = from.st_pts;
   to.st_off = from.st_off;
   for (int k = 0; k <= HostGrid::kBandRuns; ++k) to.st_rows[k] = from.st_rows[k];
-  to.sor_nlev = from.sor_nlev;
-  to.sor_nblev = from.sor_nblev;
-  to.sor_delta = from.sor_delta;
-  to.sor_pts = from.sor_pts;
-  to.sor_off = from.sor_off;
-  to.sor_bpts = from.sor_bpts;
-  to.sor_boff = from.sor_boff;
+  to.sor = from.sor;
+  to.mcsor = from.mcsor;
 }
 constexpr size_t kScheduleCacheEntries = 8;
 }  // namespace
@@ -831,13 +846,13 @@ extern "C" int x2g_host_sor_schedule(int nnu, int nmu, int *npoints, int *nlev, 
   x2g::HostGrid g;
   std::string msg = x2g::build_host_grid(g, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
   if (!msg.empty()) return X2G_ERR_SCHEDULE;
-  if (npoints) *npoints = int(g.sor_pts.size());
-  if (nlev) *nlev = g.sor_nlev;
-  if (nblev) *nblev = g.sor_nblev;
-  if (delta) *delta = g.sor_delta;
-  if (pts) std::copy(g.sor_pts.begin(), g.sor_pts.end(), pts);
-  if (off) std::copy(g.sor_off.begin(), g.sor_off.end(), off);
-  if (bpts) std::copy(g.sor_bpts.begin(), g.sor_bpts.end(), bpts);
-  if (boff) std::copy(g.sor_boff.begin(), g.sor_boff.end(), boff);
+  if (npoints) *npoints = int(g.sor.pts.size());
+  if (nlev) *nlev = g.sor.nlev;
+  if (nblev) *nblev = g.sor.nblev;
+  if (delta) *delta = g.sor.delta;
+  if (pts) std::copy(g.sor.pts.begin(), g.sor.pts.end(), pts);
+  if (off) std::copy(g.sor.off.begin(), g.sor.off.end(), off);
+  if (bpts) std::copy(g.sor.bpts.begin(), g.sor.bpts.end(), bpts);
+  if (boff) std::copy(g.sor.boff.begin(), g.sor.boff.end(), boff);
   return X2G_OK;
 }
