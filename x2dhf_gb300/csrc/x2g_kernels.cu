@@ -317,8 +317,10 @@ __device__ void tile_rhs(const GridDev &g, const JobDev &J, int t) {
 }
 
 // ----------------------------------------------------------------------
-// Persistent cooperative MCSOR kernel: all jobs x tiles, 5 colour phases
-// per micro-sweep, grid barrier between phases.
+// Persistent cooperative MCSOR kernel of the relaxation that allocates
+// nothing (its fixed scratch has no room for the wavefront's tagged copies):
+// all jobs x tiles, 5 colour phases per micro-sweep, grid barrier between
+// phases.
 // ----------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads) k_mcsor_f64(GridDev g, const __grid_constant__ JobTable jobs, int njobs,
                                                         int nsweeps, BarrierDev bar, unsigned nblocks) {
@@ -2861,14 +2863,14 @@ static int cluster_sweep(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs
   return X2G_OK;
 }
 
-// One launch batch (at most kParamJobs jobs) of launch_relax.
-static int relax_batch(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, int nsweeps, bool mixed,
-                       bool on_chip, bool pot, int G, size_t smem) {
+// One launch batch (at most kParamJobs jobs) of launch_relax's mixed form.
+static int relax_batch(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, int nsweeps, bool on_chip, bool pot,
+                       int G, size_t smem) {
   cudaError_t err;
   x2g_ctx::Pending pe{};
   const double points = double(njobs) * double(g.nni - 2) * double(g.nmu - 5) * double(nsweeps);
   const int wave = ctx->cluster_active[1];
-  if (mixed && on_chip && pot && ctx->residual_overlap && wave > 0 && njobs > wave) {
+  if (on_chip && pot && ctx->residual_overlap && wave > 0 && njobs > wave) {
     // waves of the potentials' cluster variant: the first wave's FP64
     // residual, then the later waves' residuals on the low-priority
     // auxiliary stream, beside the sweeps (on the SMs they leave free);
@@ -2902,62 +2904,40 @@ static int relax_batch(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, 
     }
     return X2G_OK;
   }
-  if (mixed) {
-    dim3 gr(grid_blocks((g.nni - 2) * (g.nmu - 5)), njobs);
-    if (on_chip)
-      k_residual<false><<<gr, kThreads, 0, ctx->stream>>>(g, jt, 0, pot ? 0 : 1);
-    else
-      k_residual<true><<<gr, kThreads, 0, ctx->stream>>>(g, jt, 1, 1);
-    ctx->launches += 1;
-  }
+  const dim3 gr(grid_blocks((g.nni - 2) * (g.nmu - 5)), njobs);
+  if (on_chip)
+    k_residual<false><<<gr, kThreads, 0, ctx->stream>>>(g, jt, 0, pot ? 0 : 1);
+  else
+    k_residual<true><<<gr, kThreads, 0, ctx->stream>>>(g, jt, 1, 1);
+  ctx->launches += 1;
   if (on_chip) return cluster_sweep(ctx, g, jt, njobs, nsweeps, pot);
   if (ctx->profiling) {
     int rc;
     if ((rc = take_event(ctx, &pe.a)) || (rc = take_event(ctx, &pe.b))) return rc;
-    pe.precision = mixed ? 1 : 0;
+    pe.precision = 1;
     pe.points = points;
     cudaEventRecord(pe.a, ctx->stream);
   }
-  {
-    // persistent cooperative kernels: the FP64 sweep with grid barriers,
-    // the mixed form's persistent-band sweep with neighbour waits.  Only the
-    // arrival count and generation are reset: the error word keeps an
-    // earlier launch's timeout until x2g_synchronize reports it
-    err = cudaMemsetAsync(ctx->bar, 0, 2 * sizeof(unsigned), ctx->stream);
-    if (err != cudaSuccess) return cuda_status(err, "barrier reset");
-    BarrierDev bar{ctx->bar, ctx->bar + 1, reinterpret_cast<int *>(ctx->bar + 2), ctx->wait_limit_ns};
-    int nj = njobs, ns = nsweeps;
-    GridDev gd = g;
-    if (mixed) {
-      // one block per (job, run of G tiles); phase counts zeroed
-      const unsigned nb = unsigned(njobs * ((g.ntiles + G - 1) / G));
-      if (nb > unsigned(kPhaseBlocks)) return set_status(X2G_ERR_ARG, "too many blocks for the phase counts");
-      err = cudaMemsetAsync(ctx->bar + kPhaseWords, 0, size_t(kPhaseBlocks) * kPhaseStride * sizeof(unsigned),
-                            ctx->stream);
-      if (err != cudaSuccess) return cuda_status(err, "barrier reset");
-      unsigned *phase = ctx->bar + kPhaseWords;
-      void *args[] = {&gd, &jt, &ns, &G, &bar, &phase};
-      err = cudaLaunchCooperativeKernel((const void *)k_mcsor_f32p, dim3(nb), dim3(kBandThreads), args, smem,
-                                        ctx->stream);
-    } else {
-      int rc = f64_block_limit(ctx);
-      if (rc) return rc;
-      const int nitems = njobs * g.ntiles;
-      unsigned nblocks = unsigned(nitems < ctx->f64_blocks ? nitems : ctx->f64_blocks);
-      if (nblocks < 1) nblocks = 1;
-      void *args[] = {&gd, &jt, &nj, &ns, &bar, &nblocks};
-      err = cudaLaunchCooperativeKernel((const void *)k_mcsor_f64, dim3(nblocks), dim3(kThreads), args, 0,
-                                        ctx->stream);
-    }
-    if (err != cudaSuccess) return cuda_status(err, "cooperative MCSOR launch");
-    ctx->launches += 1;
-    if (ctx->profiling) {
-      cudaEventRecord(pe.b, ctx->stream);
-      ctx->pending.push_back(pe);
-    }
-    // the mixed form's update u += e and the axis of u are the
-    // persistent-band sweep's epilogue
+  // persistent-band sweep, one block per (job, run of G tiles), phase counts
+  // zeroed.  The error word keeps an earlier launch's timeout until
+  // x2g_synchronize reports it
+  const unsigned nb = unsigned(njobs * ((g.ntiles + G - 1) / G));
+  if (nb > unsigned(kPhaseBlocks)) return set_status(X2G_ERR_ARG, "too many blocks for the phase counts");
+  err = cudaMemsetAsync(ctx->bar + kPhaseWords, 0, size_t(kPhaseBlocks) * kPhaseStride * sizeof(unsigned), ctx->stream);
+  if (err != cudaSuccess) return cuda_status(err, "barrier reset");
+  BarrierDev bar{ctx->bar, ctx->bar + 1, reinterpret_cast<int *>(ctx->bar + 2), ctx->wait_limit_ns};
+  unsigned *phase = ctx->bar + kPhaseWords;
+  int ns = nsweeps;
+  GridDev gd = g;
+  void *args[] = {&gd, &jt, &ns, &G, &bar, &phase};
+  err = cudaLaunchCooperativeKernel((const void *)k_mcsor_f32p, dim3(nb), dim3(kBandThreads), args, smem, ctx->stream);
+  if (err != cudaSuccess) return cuda_status(err, "cooperative MCSOR launch");
+  ctx->launches += 1;
+  if (ctx->profiling) {
+    cudaEventRecord(pe.b, ctx->stream);
+    ctx->pending.push_back(pe);
   }
+  // the update u += e and the axis of u are that kernel's epilogue
   return X2G_OK;
 }
 
@@ -3043,10 +3023,14 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
   if (njobs <= 0) return X2G_OK;
   if (nsweeps <= 0) return set_status(X2G_ERR_ARG, "nsweeps must be positive");
   if (precision == X2G_SOR) return relax_wave(ctx, grid->d, grid->d.sor, jobs, njobs, nsweeps, false);
-  if (precision != X2G_FP64 && precision != X2G_MIXED) return set_status(X2G_ERR_ARG, "unknown relaxation form");
+  // FP64 MCSOR: the same sweep over the colour-ordered list.  The barrier
+  // sweep (k_mcsor_f64, 50 phases of three dependent levels) took 7.03 ms for
+  // 22 potentials of 331 x 481, 1.80 ms for 5 and 0.52 ms for one 91 x 121
+  // orbital; the wavefront 4.29, 1.04 and 0.25 ms
+  if (precision == X2G_FP64) return relax_wave(ctx, grid->d, grid->d.mcsor, jobs, njobs, nsweeps, true);
+  if (precision != X2G_MIXED) return set_status(X2G_ERR_ARG, "unknown relaxation form");
   const GridDev &g = grid->d;
-  const bool mixed = (precision == X2G_MIXED);
-  bool on_chip = mixed && cluster_usable(ctx, g);
+  bool on_chip = cluster_usable(ctx, g);
   // potentials built from orbitals (separable lhs): the variant at two CTAs
   // per SM when the batch is larger than the clusters co-resident at one
   bool pot = false;
@@ -3065,18 +3049,16 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
     if (persistent_shape(ctx, g, want, &nj, &G1, &sm1) == X2G_OK && nj >= want) on_chip = false;
     set_status(X2G_OK, "");
   }
-  // per-job scratch: FP64 rhs of potentials, or the mixed form's FP32
-  // correction, residual and omega/lhs
+  // per-job scratch: FP32 correction, residual and omega/lhs
   const size_t per_job =
-      (mixed ? (size_t(g.next) * sizeof(float) + 2 * size_t(g.mxsize) * sizeof(float) + 256)
-             : (size_t(g.mxsize) * sizeof(double) + 256)) / 256 * 256 + 256;
+      (size_t(g.next) * sizeof(float) + 2 * size_t(g.mxsize) * sizeof(float) + 256) / 256 * 256 + 256;
   char *scratch = static_cast<char *>(ctx_workspace(ctx, per_job * njobs + 256));
   if (!scratch) return set_status(X2G_ERR_ALLOC, "workspace allocation failed");
   // the persistent-band sweep takes as many jobs per launch as give every
   // (job, run of tiles) its own co-resident block
   int per_launch = kParamJobs, G = 0;
   size_t smem = 0;
-  if (mixed && !on_chip) {
+  if (!on_chip) {
     int rc = persistent_shape(ctx, g, njobs < kParamJobs ? njobs : kParamJobs, &per_launch, &G, &smem);
     if (rc) return rc;
   }
@@ -3087,16 +3069,12 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
       JobDev &d = jt.j[i];
       if (!make_job(jobs[b0 + i], d)) return set_status(X2G_ERR_ARG, "bad relaxation job");
       char *p = scratch + per_job * size_t(b0 + i);
-      if (mixed) {
-        d.e32 = reinterpret_cast<float *>(p);
-        d.r32 = reinterpret_cast<float *>(p + (size_t(g.next) * sizeof(float) + 127) / 128 * 128);
-        d.w32 = d.r32 + g.mxsize;
-        d.rw = reinterpret_cast<float2 *>(d.r32);  // persistent-band sweep: pairs over r32 and w32
-      } else {
-        d.rhs_buf = reinterpret_cast<double *>(p);
-      }
+      d.e32 = reinterpret_cast<float *>(p);
+      d.r32 = reinterpret_cast<float *>(p + (size_t(g.next) * sizeof(float) + 127) / 128 * 128);
+      d.w32 = d.r32 + g.mxsize;
+      d.rw = reinterpret_cast<float2 *>(d.r32);  // persistent-band sweep: pairs over r32 and w32
     }
-    int rc = relax_batch(ctx, g, jt, nb, nsweeps, mixed, on_chip, pot, G, smem);
+    int rc = relax_batch(ctx, g, jt, nb, nsweeps, on_chip, pot, G, smem);
     if (rc) return rc;
   }
   // barrier error word: checked by the caller at its next synchronisation
