@@ -473,8 +473,8 @@ def run_gpu(args):
         "gpu_launches": launches,
         "roofline": {
             "bound": "hbm",
-            "kernel": ("k_mixed_cluster (mixed-form FP32 correction sweeps, one 16-CTA cluster per relaxation job, "
-                       "band resident in shared memory)" if on_chip else
+            "kernel": ("k_columns (mixed-form FP32 correction sweeps, one cluster per relaxation job, one column of "
+                       "the band in shared memory per thread)" if on_chip else
                        "k_mcsor_f32p (mixed-form FP32 correction sweeps, persistent-band cooperative kernel: "
                        "every block keeps one band of one job in shared memory for the whole launch, halos "
                        "exchanged through L2; the grid's bands do not fit one cluster's shared memory)"),

@@ -160,9 +160,9 @@ int x2g_host_sor_schedule(int nnu, int nmu, int *npoints, int *nlev, int *nblev,
  * batches that it holds in one launch. */
 int x2g_set_mixed_on_chip(x2g_ctx *ctx, int on);
 /* Mixed form, cluster kernel, batches of potentials built from orbitals
- * (lhs = f3 + idel^2 e, separable in mu and nu): a variant that keeps only
- * the residual on chip and forms omega / lhs from a row and a column term,
- * so that two CTAs fit each SM and twice the clusters are co-resident.
+ * (lhs = f3 + idel^2 e, separable in mu and nu): a variant that forms omega /
+ * lhs from a row and a column term instead of keeping it on chip, so that two
+ * CTAs fit each SM and twice the clusters are co-resident.
  * mode 0 never, 1 always, 2 (default) for batches larger than the clusters
  * of the plain kernel co-resident on the device.  No reference counterpart. */
 int x2g_set_potential_clusters(x2g_ctx *ctx, int mode);
@@ -177,11 +177,11 @@ int x2g_set_potential_clusters(x2g_ctx *ctx, int mode);
  * an SCF near its noise floor meets the convergence test).  No reference
  * counterpart. */
 int x2g_set_gram_orthonormalise(x2g_ctx *ctx, int on);
-/* Mixed form, potential batches larger than the co-resident clusters of
- * the potentials' cluster variant: 1 (default) the batch runs in waves of
+/* Mixed form, batches larger than the co-resident clusters of the cluster
+ * kernel they run on: 1 (default) the batch runs in waves of
  * that size and the FP64 residuals of the later waves run on the context's
  * low-priority auxiliary stream beside the earlier waves' sweeps (on the SMs
- * they leave free), 0 every residual before the first sweep.  Same kernels,
+ * they leave free), 0 on the context's own stream.  Same kernels,
  * same results.  No reference counterpart. */
 int x2g_set_residual_overlap(x2g_ctx *ctx, int on);
 /* Colouring of the mixed form's on-chip cluster sweep: 0 the reference's

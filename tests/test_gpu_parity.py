@@ -702,3 +702,63 @@ def test_wavefront_sweeps_bitexact(ctx, nnu, nmu, njobs, nsweeps, form, isym):
         got, exp = (x.reshape(nmu + 8, nnu + 8)[sl] for x in (b[0].cpu().numpy(), ref))
         assert np.array_equal(got, exp), (k, np.abs(got - exp).max())
     g.close()
+
+
+# edges of the on-chip sweep's bands: the smallest grids (one CTA), a seam beside a warp's end, both row pitches
+# above 11 warps, more jobs than a launch holds, one sweep and more than the halo barriers' two parities
+@pytest.mark.parametrize("nnu,nmu,njobs,nsweeps", [(31, 31, 1, 1), (31, 31, 40, 3), (61, 31, 2, 10), (91, 121, 33, 4),
+                                                   (121, 331, 3, 7), (331, 481, 14, 2), (361, 571, 2, 5),
+                                                   (511, 301, 3, 2)])
+def test_column_sweep_matches_band_sweep(ctx, nnu, nmu, njobs, nsweeps):
+    """The on-chip sweep against the persistent-band sweep on functions of no
+    symmetry: both do the same FP32 operations in the same order, so orbitals
+    and potentials agree bit for bit.  The potentials' variant has its own
+    omega / lhs (a rounded row and column term and a fast quotient, 5e-7
+    relative per update); ten sweeps of step 2 on values that their neighbours
+    enlarge up to tenfold leave 1e-4 of the largest correction."""
+    torch = pytest.importorskip("torch")
+    g = xg.Grid(ctx, nnu, nmu, 2.0, 25.0, 1.0, 1.0)
+    dev = torch.device("cuda:0")
+    gen = torch.Generator().manual_seed(nnu * nmu + njobs)
+
+    def ext(scale=1.0, shift=0.0):
+        x = torch.zeros(nmu + 8, nnu + 8, dtype=torch.float64)
+        x[4:nmu + 4, 4:nnu + 4] = shift + scale * torch.randn(nmu, nnu, generator=gen, dtype=torch.float64)
+        return x.to(dev)
+
+    def flat(scale, shift):
+        return (shift + scale * torch.rand(nmu * nnu, generator=gen, dtype=torch.float64)).to(dev)
+
+    u0 = [ext() for _ in range(njobs)]
+    lhs, rhs = flat(-1e4, -1e4), flat(2.0, -1.0)
+    a, b = ext(1e-2), ext(1e-2)
+
+    def run(kind, **opts):
+        us = [u.clone() for u in u0]
+        jobs = [xg.Job(u=u.data_ptr(), omega=1.9, isym=1 if k % 2 == 0 else -1, kind=kind, idel=k % 3,
+                       **(dict(lhs=lhs.data_ptr(), rhs=rhs.data_ptr()) if kind == 0 else
+                          dict(psa=a.data_ptr(), psb=b.data_ptr()))) for k, u in enumerate(us)]
+        for name, value in opts.items():
+            getattr(ctx, "set_" + name)(value)
+        torch.cuda.synchronize()
+        try:
+            xg.relax(ctx, g, jobs, nsweeps, xg.MIXED)
+            ctx.synchronize()
+        finally:
+            ctx.set_mixed_on_chip(True)
+            ctx.set_potential_clusters("auto")
+            ctx.set_mixed_colouring("reference")
+        return us
+
+    for kind in (0, 1):
+        band = run(kind, mixed_on_chip=False)
+        chip = run(kind, potential_clusters=False)
+        for k, (x, y) in enumerate(zip(chip, band)):
+            assert torch.isfinite(x).all() and torch.equal(x, y), (kind, k, float((x - y).abs().max()))
+    for colouring in ("reference", "free"):
+        plain = run(1, potential_clusters=False, mixed_colouring=colouring)
+        sep = run(1, potential_clusters=True, mixed_colouring=colouring)
+        for k, (x, y, u) in enumerate(zip(sep, plain, u0)):
+            big = float((y - u).abs().max())
+            assert big > 0 and float((x - y).abs().max()) <= 1e-4 * big, (colouring, k, float((x - y).abs().max()) / big)
+    g.close()

@@ -440,7 +440,7 @@ class Context:
 
     def set_potential_clusters(self, mode):
         """Cluster sweep of potential batches: True the two-CTAs-per-SM
-        variant (residual only on chip, omega/lhs from row and column terms),
+        variant (omega/lhs from row and column terms, not kept on chip),
         False the plain kernel, "auto" the variant for batches above the
         plain kernel's co-resident clusters."""
         _check(self.L.x2g_set_potential_clusters(self.h, 2 if mode == "auto" else (1 if mode else 0)))
@@ -461,8 +461,8 @@ class Context:
         _check(self.L.x2g_set_gram_orthonormalise(self.h, 1 if on else 0))
 
     def set_residual_overlap(self, on):
-        """Potential batches beyond one wave of clusters: the later jobs' FP64
-        residual on the auxiliary stream under the first wave's sweep."""
+        """Batches beyond one wave of clusters: the later jobs' FP64 residual
+        on the auxiliary stream under the first wave's sweep."""
         _check(self.L.x2g_set_residual_overlap(self.h, 1 if on else 0))
 
     def convert_selftest(self, n, seed=1):

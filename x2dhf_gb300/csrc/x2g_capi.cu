@@ -375,7 +375,6 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
   UP(h.tile_row1, tile_row1);
   UP(h.pts, pts);
   UP(h.off, off);
-  UP(h.pts_rc, pts_rc);
   UP(h.st_pts, st_pts);
   UP(h.st_off, st_off);
   const WaveHost *waves[2] = {&h.sor, &h.mcsor};
@@ -394,32 +393,6 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
     wd.delta = w.delta;
   }
   for (int k = 0; k <= HostGrid::kBandRuns; ++k) d.st_rows[k] = h.st_rows[k];
-  d.cl_size = h.cl_size;
-  d.cl_maxrows = h.cl_maxrows;
-  d.cl_maxchunks = h.cl_maxchunks;
-  d.cl_wa = h.cl_wa;
-  d.cl_wb = h.cl_wb;
-  d.cl_ws = h.cl_ws;
-  d.cl_pa = h.cl_pa;
-  d.cf_maxchunks = h.cf_maxchunks;
-  d.cf_wa = h.cf_wa;
-  d.cf_wb = h.cf_wb;
-  d.cf_ws = h.cf_ws;
-  d.cf_pa = h.cf_pa;
-  d.cf_pb = h.cf_pb;
-  d.cf_ps = h.cf_ps;
-  d.cl_pb = h.cl_pb;
-  d.cl_ps = h.cl_ps;
-  if (h.cl_size > 0) {
-    UP(h.cl_tile0, cl_tile0);
-    UP(h.cl_row0, cl_row0);
-    UP(h.cl_pts, cl_pts);
-    UP(h.cl_off, cl_off);
-    UP(h.cf_pts, cf_pts);
-    UP(h.cf_off, cf_off);
-  } else {
-    d.cl_tile0 = d.cl_row0 = d.cl_pts = d.cl_off = d.cf_pts = d.cf_off = nullptr;
-  }
   UP(b32, borb_mu32);
   UP(p32, bpot_mu32);
   UP(d32, d_nu32);

@@ -1,0 +1,57 @@
+// Device helpers shared by the kernels of the mixed form.
+#pragma once
+
+#include "x2g_internal.h"
+
+namespace x2g {
+
+// double -> float with round to nearest even, on the integer pipes (GB300
+// issues conversion instructions on its narrow FP64 pipe); values beyond the
+// float range become infinities, values below its normal range signed zero
+__device__ __forceinline__ float narrow_f64(double x) {
+  const unsigned hi = unsigned(__double2hiint(x)), lo = unsigned(__double2loint(x));
+  const unsigned sign = hi & 0x80000000u;
+  const int dex = int((hi >> 20) & 0x7ffu);
+  if (dex == 0x7ff) return __uint_as_float(sign | 0x7f800000u | ((hi & 0xfffffu) ? 0x400000u : 0u));
+  const int fex = dex - 896;
+  if (fex >= 255) return __uint_as_float(sign | 0x7f800000u);
+  if (fex <= 0) return __uint_as_float(sign);
+  // 23 mantissa bits: 20 from hi, 3 from lo; the remaining 29 bits round
+  unsigned bits = (unsigned(fex) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+  const unsigned rest = lo & 0x1fffffffu;
+  if (rest > 0x10000000u || (rest == 0x10000000u && (bits & 1u))) ++bits;  // may carry into the exponent
+  return __uint_as_float(sign | bits);
+}
+
+// float -> double by bit manipulation on the integer pipes (GB300 issues
+// conversion instructions on its narrow FP64 pipe); exact for normal floats,
+// infinities and NaNs; float subnormals (|e| < 1.2e-38, far below any
+// correction that matters) become signed zero
+__device__ __forceinline__ double widen_f32(float f) {
+  const unsigned b = __float_as_uint(f), ex = (b >> 23) & 0xffu, m = b & 0x7fffffu;
+  const unsigned sign = b & 0x80000000u;
+  if (ex == 0) return __hiloint2double(int(sign), 0);
+  const unsigned dex = (ex == 0xffu) ? 0x7ffu : ex + 896u;
+  return __hiloint2double(int(sign | (dex << 20) | (m >> 3)), int(m << 29));
+}
+
+// FP64 axis extrapolation of one point from its 5 neighbours at stride st
+// (sormcsor.F90:94-129 order)
+__device__ __forceinline__ double extrap64(const GridDev &g, const double *u, int ij, int st) {
+  double v = __dadd_rn(__dmul_rn(g.exeven[0], u[ij + st]), __dmul_rn(g.exeven[1], u[ij + 2 * st]));
+  v = __dadd_rn(v, __dmul_rn(g.exeven[2], u[ij + 3 * st]));
+  v = __dadd_rn(v, __dmul_rn(g.exeven[3], u[ij + 4 * st]));
+  return __dadd_rn(v, __dmul_rn(g.exeven[4], u[ij + 5 * st]));
+}
+
+// axis extrapolation of the correction from the five values at stride s
+__device__ __forceinline__ float ex5f(const float *ex, const float *p, int s) {
+  return ex[0] * p[s] + ex[1] * p[2 * s] + ex[2] * p[3 * s] + ex[3] * p[4 * s] + ex[4] * p[5 * s];
+}
+
+// split cluster barrier: arrive releases this thread's earlier shared and
+// distributed-shared writes, wait acquires every CTA's released writes
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+}  // namespace x2g

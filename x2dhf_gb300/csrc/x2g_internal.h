@@ -48,6 +48,25 @@ struct WaveHost {
 };
 
 // ----------------------------------------------------------------------
+// Bands of the on-chip FP32 sweep (k_columns) for clusters of `size` CTAs:
+// CTA k owns ext rows [row0[k], row0[k+1]) of the interior rows 5..nmu-1.
+// With two threads per column (groups 2) a band is cut before its row cut[k].
+// The row seam lies inside one thread's rows; slots is the most points of one
+// colour in a thread's rows, pitch the row pitch in words (a multiple of 32),
+// warps those of a group, shift the lanes before the first column that keep
+// the column seam inside one warp.
+// ----------------------------------------------------------------------
+constexpr int kMaxCluster = 16;
+struct ColPlan {
+  int size, groups, maxrows, slots, pitch, warps, shift;
+  // set for the launch: the rows the kernel's arrays hold, the FP32 stencil
+  // weights as (mu, nu) pairs, (-1, -1)
+  int rows;
+  float2 c2[4], c1[4], neg;
+  int row0[kMaxCluster + 1], cut[kMaxCluster];
+};
+
+// ----------------------------------------------------------------------
 // Host-side grid: every table the relaxation path reads, built with the
 // reference's formulas (initCBAllocArrays.F90 initCBlocks:813-858,
 // initSuppl:1636-2051).  Indices are 0-based: nu j in [0,nni), mu i in
@@ -106,6 +125,8 @@ struct HostGrid {
   static constexpr int kBandRuns = 16;
   std::vector<int> st_pts, st_off;
   int st_rows[kBandRuns + 1] = {};
+  // bands of the on-chip FP32 sweep, by cluster size and threads per column
+  std::vector<ColPlan> columns;
   // the FP64 sweeps' wavefront schedules (build_wave_schedule): list-order
   // SOR over the "middle" list (sor, sormcsor.F90:20-132), and MCSOR as the
   // same sweep over the list colour after colour (mcsor, :143-386)
@@ -137,11 +158,7 @@ struct GridDev {
   const double *wf;  // wgt2 f4: the weight of the orbital inner products (Gram-matrix orthonormalisation)
   const double *dmu9, *dni9;
   const double *vxi, *vxisq, *veta, *vetasq;
-  const int *tile_row0, *tile_row1, *pts, *off, *pts_rc;
-  int cl_size, cl_maxrows, cl_maxchunks, cl_wa, cl_wb, cl_ws, cl_pa, cl_pb, cl_ps;
-  int cf_maxchunks, cf_wa, cf_wb, cf_ws, cf_pa, cf_pb, cf_ps;
-  const int *cf_pts, *cf_off;
-  const int *cl_tile0, *cl_row0, *cl_pts, *cl_off;
+  const int *tile_row0, *tile_row1, *pts, *off;
   const int *st_pts, *st_off;
   int st_rows[17];
   WaveDev sor, mcsor;
@@ -227,16 +244,25 @@ struct x2g_ctx {
   double *host_red = nullptr;  // pinned host buffer for small readbacks
   long long h2d_bytes = 0, d2h_bytes = 0;  // host<->device bytes copied by the library
   long launches = 0;
-  size_t cluster_smem_set = 0;  // dynamic shared memory granted to the cluster kernel
+  int cluster_smem = -1;        // largest dynamic shared memory of a cluster sweep CTA (0: none)
   int no_cluster = 0;           // 1: mixed form uses the persistent-band FP32 kernel
   int auto_band = 0;            // 1: batches beyond the co-resident clusters take the persistent-band kernel
-  int pot_clusters = 2;         // potentials' cluster variant: 0 never, 1 always, 2 batches above cluster_active[0]
+  int pot_clusters = 2;         // potentials' cluster variant: 0 never, 1 always, 2 batches beyond the plain kernel's clusters
   int mixed_free = 0;           // cluster sweep colouring: 0 the reference's list order mod 5, 1 seam-free
-  // [0] the cluster kernel, [1] its potentials' variant:
-  int cluster_active[2] = {0, 0};       // clusters co-resident on the device (last shape checked)
-  long cluster_checked_key[2] = {-1, -1};  // (shared bytes, cluster size, warps) last checked
-  int cluster_ok[2] = {0, 0};             // that cluster shape is schedulable here
-  int cluster_nonportable = 0;  // cluster kernels allowed more than 8 CTAs
+  // kernels of the cluster sweep that run a grid size's band plans here
+  struct ColumnShape {
+    int plan;  // place in HostGrid::columns
+    const void *fn;
+    bool sep;
+    int rows;
+    size_t smem;
+    int active;  // co-resident clusters
+  };
+  struct ColumnShapes {
+    int nni, nmu;
+    std::vector<ColumnShape> shapes;
+  };
+  std::vector<ColumnShapes> columns;
   int band_attr = 0;            // shared memory cap granted to the persistent-band sweep
   long band_key = -1;           // shared bytes of its last occupancy query
   int band_blocks = 0;          // co-resident blocks for that size

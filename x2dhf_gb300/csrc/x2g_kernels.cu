@@ -12,7 +12,7 @@
 #include <cstdio>
 #include <vector>
 
-#include "x2g_kernels.cuh"
+#include "x2g_columns.cuh"
 
 namespace x2g {
 
@@ -802,44 +802,6 @@ __global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev
   }
 }
 
-// double -> float with round to nearest even, on the integer pipes (GB300
-// issues conversion instructions on its narrow FP64 pipe); values beyond the
-// float range become infinities, values below its normal range signed zero
-__device__ __forceinline__ float narrow_f64(double x) {
-  const unsigned hi = unsigned(__double2hiint(x)), lo = unsigned(__double2loint(x));
-  const unsigned sign = hi & 0x80000000u;
-  const int dex = int((hi >> 20) & 0x7ffu);
-  if (dex == 0x7ff) return __uint_as_float(sign | 0x7f800000u | ((hi & 0xfffffu) ? 0x400000u : 0u));
-  const int fex = dex - 896;
-  if (fex >= 255) return __uint_as_float(sign | 0x7f800000u);
-  if (fex <= 0) return __uint_as_float(sign);
-  // 23 mantissa bits: 20 from hi, 3 from lo; the remaining 29 bits round
-  unsigned bits = (unsigned(fex) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
-  const unsigned rest = lo & 0x1fffffffu;
-  if (rest > 0x10000000u || (rest == 0x10000000u && (bits & 1u))) ++bits;  // may carry into the exponent
-  return __uint_as_float(sign | bits);
-}
-
-// float -> double by bit manipulation on the integer pipes (GB300 issues
-// conversion instructions on its narrow FP64 pipe); exact for normal floats,
-// infinities and NaNs; float subnormals (|e| < 1.2e-38, far below any
-// correction that matters) become signed zero
-__device__ __forceinline__ double widen_f32(float f) {
-  const unsigned b = __float_as_uint(f), ex = (b >> 23) & 0xffu, m = b & 0x7fffffu;
-  const unsigned sign = b & 0x80000000u;
-  if (ex == 0) return __hiloint2double(int(sign), 0);
-  const unsigned dex = (ex == 0xffu) ? 0x7ffu : ex + 896u;
-  return __hiloint2double(int(sign | (dex << 20) | (m >> 3)), int(m << 29));
-}
-
-// FP64 axis extrapolation of one point from its 5 neighbours at stride st
-// (sormcsor.F90:94-129 order)
-__device__ __forceinline__ double extrap64(const GridDev &g, const double *u, int ij, int st) {
-  return A(A(A(A(M(g.exeven[0], u[ij + st]), M(g.exeven[1], u[ij + 2 * st])), M(g.exeven[2], u[ij + 3 * st])),
-             M(g.exeven[3], u[ij + 4 * st])),
-           M(g.exeven[4], u[ij + 5 * st]));
-}
-
 // Axis extrapolation of the correction (tile_boundary<float>) for tiles
 // [t0, t1) computed in the band sb held in shared memory (indexed by ext
 // index).
@@ -1038,383 +1000,6 @@ __global__ void __launch_bounds__(kBandThreads) k_mcsor_f32p(GridDev g, const __
       u[ij] = even ? extrap64(g, u, ij, threadIdx.x == 0 ? 1 : -1) : 0.0;
     }
   }
-}
-
-// ----------------------------------------------------------------------
-// On-chip FP32 correction sweep of the mixed form: one relaxation job per
-// thread-block cluster.  CTA k of the cluster keeps ext rows
-// [cl_row0[k]-4, cl_row0[k+1]+4) of the correction e in shared memory for
-// all micro-sweeps, together with the band's residual, omega/lhs, the
-// coefficient rows and its point list; after updating a point within 4 rows
-// of its band edge it also stores the value into the neighbouring CTA's halo
-// through distributed shared memory, and the colour phases are separated by
-// the cluster's hardware barrier.  Ends with u += e (FP64) on the band's
-// interior points and the FP64 axis re-extrapolation of u.
-// ----------------------------------------------------------------------
-constexpr int kClusterMaxThreads = 768;  // 24 warps: interior + edge + seam roles
-
-__device__ __forceinline__ float ex5f(const float *ex, const float *p, int s) {
-  return ex[0] * p[s] + ex[1] * p[2 * s] + ex[2] * p[3 * s] + ex[3] * p[4 * s] + ex[4] * p[5 * s];
-}
-
-// axis extrapolation of e in shared memory for the CTA's rows
-__device__ void smem_boundary(const GridDev &g, float *E, int R0, int R1, int rank, bool even, const float *ex) {
-  const int n8 = g.n8, nni = g.nni;
-  const int nrow7 = (rank == 0) ? nni - 2 : 0;
-  const int r0 = (rank == 0) ? 5 : R0;
-  const int nside = 2 * (R1 - r0);
-  for (int k = threadIdx.x; k < nrow7 + nside; k += blockDim.x) {
-    if (k < nrow7) {
-      float *p = E + (4 - R0 + 4) * n8 + 5 + k;
-      *p = even ? ex5f(ex, p, n8) : 0.0f;
-    } else {
-      const int q = k - nrow7, r = r0 + q / 2, side = q % 2;
-      float *p = E + (r - R0 + 4) * n8 + (side == 0 ? 4 : nni + 3);
-      *p = even ? ex5f(ex, p, side == 0 ? 1 : -1) : 0.0f;
-    }
-  }
-  __syncthreads();
-  if (rank == 0 && threadIdx.x < 2) {
-    float *p = E + (4 - R0 + 4) * n8 + (threadIdx.x == 0 ? 4 : nni + 3);
-    *p = even ? ex5f(ex, p, threadIdx.x == 0 ? 1 : -1) : 0.0f;
-  }
-}
-
-// dynamic shared memory of k_mixed_cluster: (residual, omega/lhs) pairs of
-// the band's points, correction band with 4-row halos, b(mu) of the band's
-// rows, d(nu) by ext column, the CTA's segment offsets, then its chunk list.
-// k_mixed_cluster_pot (potentials, lhs = f3(mu) + idel^2 (e_mu(mu) -
-// e_nu(nu))) keeps the residual alone and the lhs as a row term of the
-// band's rows and a column term by ext column, after d(nu).
-// free: the seam-free colouring's plan (one level, cf_*), else the
-// reference colouring's (cl_*)
-size_t cluster_smem_bytes(const GridDev &g, bool sep, bool free) {
-  const size_t band = size_t(g.cl_maxrows) * g.n8 * sizeof(float);
-  const int S = (free ? 1 : g.nlev) + 2, chunks = free ? g.cf_maxchunks : g.cl_maxchunks;
-  return (sep ? band : 2 * band) + size_t(g.cl_maxrows + 8) * g.n8 * sizeof(float) +
-         size_t(g.cl_maxrows + g.n8) * sizeof(float) * (sep ? 2 : 1) + size_t(5 * S + 1) * sizeof(int) +
-         size_t(chunks) * sizeof(int);
-}
-
-
-// split cluster barrier: arrive releases this thread's earlier shared and
-// distributed-shared writes, wait acquires every CTA's released writes
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
-// (row, col) of the points k, k+T, k+2T, ... of a band's interior listed
-// row by row from (ra, 5) with ncols columns per row, advanced without
-// division
-struct BandWalk {
-  int row, col, step_r, step_c, col_end, ncols;
-  __device__ BandWalk(int k, int T, int ra, int nc) : ncols(nc) {
-    row = ra + k / nc;
-    col = 5 + k % nc;
-    step_r = T / nc;
-    step_c = T % nc;
-    col_end = 5 + nc;
-  }
-  __device__ __forceinline__ void next() {
-    row += step_r;
-    col += step_c;
-    if (col >= col_end) {
-      col -= ncols;
-      ++row;
-    }
-  }
-};
-
-struct ClusterBand {
-  float *E;               // correction rows [R0-4, R1+4) of the band
-  const float2 *RW;       // (residual, omega/lhs) by band row * n8 + col
-  const float *R;         // potentials' variant: residual by band row * n8 + col
-  const float *BT, *DN;   // b(mu) by band row, d(nu) by ext column
-  const float *LP, *LQ;   // potentials' variant: lhs = LP[band row] - LQ[ext column]
-  const unsigned *PL;     // chunks (band row << 19) | (col << 2) | (count-1)
-  float *up, *dn;         // neighbours' halos addressed like E, or null
-  int n8, hdn;            // band rows >= hdn feed the lower neighbour
-  float omega, omega1;
-  CoefF cf;
-};
-
-// One chunk: up to 4 same-colour points of one band row at columns col,
-// col+5, col+10, col+15.  The row values col-4..col+19 are read once (a
-// point's left neighbours are the previous point's right ones); every read
-// precedes every write.  Positions past the chunk's count are computed but
-// not stored: their reads stay inside the CTA's shared allocation (at most
-// 10 elements past the correction band, the pairs, the residual, d(nu) or
-// the lhs column term, each followed by a larger array).  kSep: omega / lhs
-// from the row and column terms (fast reciprocal: the correction sweep is
-// the inner solver of the FP64 defect correction, whose fixed point does
-// not depend on it).
-template <bool halo, bool kSep>
-__device__ __forceinline__ void cluster_chunk(const ClusterBand &B, unsigned q) {
-  const int n8 = B.n8;
-  const int lr = int(q >> 19), col = int((q >> 2) & 0x1ffffu), n = int(q & 3u) + 1;
-  const int ls = lr * n8 + col;
-  float *const p = B.E + ls + 4 * n8;
-  const CoefF &cf = B.cf;
-  float rv[24];
-#pragma unroll
-  for (int i = 0; i < 24; ++i) rv[i] = p[i - 4];
-  const float b = B.BT[lr];
-  float out[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float *pj = p + 5 * j;
-    const float m4 = pj[-4 * n8], p4 = pj[4 * n8], m3 = pj[-3 * n8], p3 = pj[3 * n8];
-    const float m2 = pj[-2 * n8], p2 = pj[2 * n8], m1 = pj[-n8], p1 = pj[n8];
-    const float l4 = rv[5 * j], l3 = rv[5 * j + 1], l2 = rv[5 * j + 2], l1 = rv[5 * j + 3], ec = rv[5 * j + 4];
-    const float r1 = rv[5 * j + 5], r2 = rv[5 * j + 6], r3 = rv[5 * j + 7], r4 = rv[5 * j + 8];
-    float2 rw;
-    if (kSep)
-      rw = make_float2(B.R[ls + 5 * j], __fdividef(B.omega, B.LP[lr] - B.LQ[col + 5 * j]));
-    else
-      rw = B.RW[ls + 5 * j];
-    const float d = B.DN[col + 5 * j];
-    float dm2 = cf.dmu2[0] * (m4 + p4);
-    dm2 = __fmaf_rn(cf.dmu2[1], m3 + p3, dm2);
-    dm2 = __fmaf_rn(cf.dmu2[2], m2 + p2, dm2);
-    dm2 = __fmaf_rn(cf.dmu2[3], m1 + p1, dm2);
-    float dm1 = cf.dmu1[0] * (m4 - p4);
-    dm1 = __fmaf_rn(cf.dmu1[1], m3 - p3, dm1);
-    dm1 = __fmaf_rn(cf.dmu1[2], m2 - p2, dm1);
-    dm1 = __fmaf_rn(cf.dmu1[3], m1 - p1, dm1);
-    float dn2 = cf.dni2[0] * (l4 + r4);
-    dn2 = __fmaf_rn(cf.dni2[1], l3 + r3, dn2);
-    dn2 = __fmaf_rn(cf.dni2[2], l2 + r2, dn2);
-    dn2 = __fmaf_rn(cf.dni2[3], l1 + r1, dn2);
-    float dn1 = cf.dni1[0] * (l4 - r4);
-    dn1 = __fmaf_rn(cf.dni1[1], l3 - r3, dn1);
-    dn1 = __fmaf_rn(cf.dni1[2], l2 - r2, dn1);
-    dn1 = __fmaf_rn(cf.dni1[3], l1 - r1, dn1);
-    const float cc = __fmaf_rn(d, dn1, __fmaf_rn(b, dm1, dm2) + dn2);
-    out[j] = __fmaf_rn(B.omega1, ec, rw.y * (rw.x - cc));
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (j < n) p[5 * j] = out[j];
-  if (halo) {
-    if (B.up && lr < 4) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j < n) B.up[ls + 4 * n8 + 5 * j] = out[j];
-    }
-    if (B.dn && lr >= B.hdn) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j < n) B.dn[ls + 4 * n8 + 5 * j] = out[j];
-    }
-  }
-}
-
-// update chunks [b0, b1) of the CTA's list (their points are independent),
-// thread t of the n threads of a warp role taking chunks t, t+n, ...
-template <bool halo, bool kSep>
-__device__ __forceinline__ void cluster_chunks(const ClusterBand &B, int b0, int b1, int t, int n) {
-  for (int k = b0 + t; k < b1; k += n) cluster_chunk<halo, kSep>(B, B.PL[k]);
-}
-
-// barrier among the seam warps only (named barrier 1)
-__device__ __forceinline__ void seam_barrier(int nthreads) {
-  asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
-}
-
-template <bool kSep>
-__device__ __forceinline__ void mixed_cluster_body(const GridDev &g, const JobTable &jobs, int nsweeps, int free) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  const int C = int(cl.num_blocks()), rank = int(cl.block_rank());
-  const JobDev &J = jobs.j[blockIdx.x / C];
-  const float *const r32 = J.r32, *const w32 = J.w32;
-  const bool even = (J.isym == 1);
-  const float *const bt = (J.kind >= 1) ? g.bpot_mu32 : g.borb_mu32;
-  extern __shared__ float2 smem2[];
-  const int n8 = g.n8, nni = g.nni, nlev = free ? 1 : g.nlev, S = nlev + 2;
-  const int R0 = g.cl_row0[rank], R1 = g.cl_row0[rank + 1];
-  const int nloc = (g.cl_maxrows + 8) * n8;
-  const int *const plan_off = free ? g.cf_off : g.cl_off, *const plan_pts = free ? g.cf_pts : g.cl_pts;
-  float2 *const RW = smem2;
-  float *const RR = reinterpret_cast<float *>(smem2);
-  float *const E = kSep ? RR + g.cl_maxrows * n8 : reinterpret_cast<float *>(RW + g.cl_maxrows * n8);
-  float *const BT = E + nloc;
-  float *const DN = BT + g.cl_maxrows;
-  float *const LP = DN + n8;                   // kSep only
-  float *const LQ = LP + g.cl_maxrows;         // kSep only
-  int *const SO = reinterpret_cast<int *>(kSep ? LQ + n8 : DN + n8);  // segment offsets into PL
-  unsigned *const PL = reinterpret_cast<unsigned *>(SO + 5 * S + 1);
-  const int *const coff = plan_off + size_t(rank) * 5 * S;
-  const int pbase = coff[0], npl = coff[5 * S] - pbase;
-  for (int k = threadIdx.x; k <= 5 * S; k += blockDim.x) SO[k] = coff[k] - pbase;
-  for (int k = threadIdx.x; k < nloc; k += blockDim.x) E[k] = 0.0f;
-  for (int k = threadIdx.x; k < R1 - R0; k += blockDim.x) BT[k] = bt[R0 + k - 4];
-  for (int k = threadIdx.x; k < n8; k += blockDim.x) DN[k] = (k >= 4 && k < nni + 4) ? g.d_nu32[k - 4] : 0.0f;
-  if (kSep) {
-    // lhs = f3 + idel^2 e with e = e_mu - e_nu: the row term in FP64, then
-    // both terms in FP32 (the nu axis columns, never updated, get 0)
-    for (int k = threadIdx.x; k < R1 - R0; k += blockDim.x) {
-      const int mu = R0 + k - 4;
-      LP[k] = narrow_f64(fma(J.idel2, g.e_mu[mu], g.f3_mu[mu]));
-    }
-    for (int k = threadIdx.x; k < n8; k += blockDim.x)
-      LQ[k] = (k >= 4 && k < nni + 4) ? narrow_f64(J.idel2 * g.e_nu[k - 4]) : 0.0f;
-  }
-  for (int k = threadIdx.x; k < npl; k += blockDim.x) PL[k] = unsigned(plan_pts[pbase + k]);
-  const int ra = (R0 < 5) ? 5 : R0, ncols = nni - 2, nband = (R1 - ra) * ncols;
-  {
-    // four points per thread in flight: all loads before the stores
-    BandWalk w(threadIdx.x, blockDim.x, ra, ncols);
-    for (int k = threadIdx.x; k < nband; k += 4 * blockDim.x) {
-      float rv[4], wv[4];
-      int ls[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        ls[j] = -1;
-        if (k + j * int(blockDim.x) < nband) {
-          const int ik = (w.row - 4) * nni + (w.col - 4);
-          ls[j] = (w.row - R0) * n8 + w.col;
-          rv[j] = r32[ik];
-          if (!kSep) wv[j] = w32[ik];
-        }
-        w.next();
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (ls[j] >= 0) {
-          if (kSep)
-            RR[ls[j]] = rv[j];
-          else
-            RW[ls[j]] = make_float2(rv[j], wv[j]);
-        }
-    }
-  }
-  ClusterBand B;
-  B.E = E;
-  B.RW = RW;
-  B.R = RR;
-  B.BT = BT;
-  B.DN = DN;
-  B.LP = LP;
-  B.LQ = LQ;
-  B.PL = PL;
-  B.n8 = n8;
-  B.hdn = R1 - R0 - 4;
-  B.omega = J.omegaf;
-  B.omega1 = J.omega1f;
-  for (int k = 0; k < 4; ++k) {
-    B.cf.dmu1[k] = g.dmu1f[k];
-    B.cf.dmu2[k] = g.dmu2f[k];
-    B.cf.dni1[k] = g.dni1f[k];
-    B.cf.dni2[k] = g.dni2f[k];
-  }
-  float ex[5];
-  for (int k = 0; k < 5; ++k) ex[k] = g.exevenf[k];
-  // neighbours' halo rows, addressed by this CTA's band offsets
-  B.up = (rank > 0) ? cl.map_shared_rank(E, rank - 1) + (R0 - g.cl_row0[rank - 1]) * n8 : nullptr;
-  B.dn = (rank < C - 1) ? cl.map_shared_rank(E, rank + 1) + (R0 - R1) * n8 : nullptr;
-  // warp roles: interior, edge, seam
-  const int wa = free ? (kSep ? g.cf_pa : g.cf_wa) : (kSep ? g.cl_pa : g.cl_wa);
-  const int wb = free ? (kSep ? g.cf_pb : g.cf_wb) : (kSep ? g.cl_pb : g.cl_wb);
-  const int ws = free ? (kSep ? g.cf_ps : g.cf_ws) : (kSep ? g.cl_ps : g.cl_ws);
-  const int warp = threadIdx.x >> 5;
-  const int role = (warp < wa) ? 0 : (warp < wa + wb) ? 1 : 2;
-  const int rbase = (role == 0) ? 0 : (role == 1) ? wa : wa + wb;
-  const int rt = threadIdx.x - 32 * rbase;
-  const int rn = 32 * ((role == 0) ? wa : (role == 1) ? wb : ws);
-  __syncthreads();
-  cluster_arrive();  // this band is zeroed: neighbours may push into its halos
-  for (int s = 0; s < nsweeps; ++s) {
-    for (int c = 0; c < 5; ++c) {
-      if (c == 0 && s > 0) {
-        smem_boundary(g, E, R0, R1, rank, even, ex);
-        __syncthreads();
-      }
-      const int *o = SO + c * S;
-      // After the cluster wait the halos hold the neighbours' previous
-      // colour, and the neighbours no longer read the halo values this colour
-      // overwrites.  Interior points need only this CTA's values; seam points
-      // go level by level among the seam warps.
-      if (role == 0) {
-        cluster_chunks<false, kSep>(B, o[0], o[1], rt, rn);
-        cluster_wait();
-      } else if (role == 1) {
-        cluster_wait();
-        cluster_chunks<true, kSep>(B, o[1], o[2], rt, rn);
-      } else {
-        cluster_wait();
-        cluster_chunks<true, kSep>(B, o[2], o[3], rt, rn);
-        for (int l = 1; l < nlev; ++l) {
-          if (o[2 + l] == o[3 + l]) continue;
-          seam_barrier(rn);
-          cluster_chunks<true, kSep>(B, o[2 + l], o[3 + l], rt, rn);
-        }
-      }
-      __syncthreads();
-      cluster_arrive();
-    }
-  }
-  cluster_wait();  // no CTA leaves while a neighbour may still write its halo
-  // u += e on the band's interior points, then the FP64 axis of u for the
-  // band's rows (the mu=1 row and corners by the first CTA, whose band holds
-  // rows 4..9)
-  double *const u = J.u;
-  {
-    BandWalk w(threadIdx.x, blockDim.x, ra, ncols);
-    for (int k = threadIdx.x; k < nband; k += 4 * blockDim.x) {
-      double uv[4];
-      int ij[4], le[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        ij[j] = -1;
-        if (k + j * int(blockDim.x) < nband) {
-          ij[j] = w.row * n8 + w.col;
-          le[j] = (w.row - R0 + 4) * n8 + w.col;
-          uv[j] = u[ij[j]];
-        }
-        w.next();
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (ij[j] >= 0) u[ij[j]] = uv[j] + widen_f32(E[le[j]]);
-    }
-  }
-  __syncthreads();
-  const int nrow7 = (rank == 0) ? nni - 2 : 0, nside = 2 * (R1 - ra);
-  for (int k = threadIdx.x; k < nrow7 + nside; k += blockDim.x) {
-    if (k < nrow7) {
-      const int ij = 4 * n8 + 5 + k;
-      u[ij] = even ? extrap64(g, u, ij, n8) : 0.0;
-    } else {
-      const int q = k - nrow7, r = ra + q / 2, side = q % 2;
-      const int ij = r * n8 + (side == 0 ? 4 : nni + 3);
-      u[ij] = even ? extrap64(g, u, ij, side == 0 ? 1 : -1) : 0.0;
-    }
-  }
-  __syncthreads();
-  if (rank == 0 && threadIdx.x < 2) {
-    const int ij = 4 * n8 + (threadIdx.x == 0 ? 4 : nni + 3);
-    u[ij] = even ? extrap64(g, u, ij, threadIdx.x == 0 ? 1 : -1) : 0.0;
-  }
-}
-
-__global__ void __launch_bounds__(kClusterMaxThreads, 1) k_mixed_cluster(GridDev g, const __grid_constant__ JobTable jobs,
-                                                                        int nsweeps, int free) {
-  mixed_cluster_body<false>(g, jobs, nsweeps, free);
-}
-
-// Potentials only (job kind 1): two CTAs per SM, so that twice the clusters
-// are co-resident for the batches of an SCF iteration's potentials; at most
-// kWarps warps per CTA (kPotWarpsRef for the reference colouring,
-// kPotWarpsFree for the seam-free one)
-template <int kWarps>
-__global__ void __launch_bounds__(32 * kWarps, 2) k_mixed_cluster_pot(GridDev g, const __grid_constant__ JobTable jobs,
-                                                                     int nsweeps, int free) {
-  mixed_cluster_body<true>(g, jobs, nsweeps, free);
-}
-
-// the potentials' variant for a colouring
-static const void *pot_kernel(bool free) {
-  return free ? (const void *)k_mixed_cluster_pot<kPotWarpsFree> : (const void *)k_mixed_cluster_pot<kPotWarpsRef>;
 }
 
 // ----------------------------------------------------------------------
@@ -2687,73 +2272,113 @@ static int take_event(x2g_ctx *ctx, cudaEvent_t *ev) {
   return (err == cudaSuccess) ? X2G_OK : cuda_status(err, "profiling event");
 }
 
-// The cluster kernel's function attributes are shared by every context and
-// thread of the process: the dynamic shared memory cap is set once to the
-// device's opt-in maximum (never lowered, so concurrent contexts with
-// different grids cannot undercut each other) and clusters above 8 CTAs are
-// allowed.  Idempotent.
-static bool cluster_attributes(x2g_ctx *ctx) {
-  if (ctx->cluster_smem_set > 0 && ctx->cluster_nonportable) return true;
-  int optin = 0;
-  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess ||
-      cudaFuncSetAttribute((const void *)k_mixed_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute((const void *)k_mixed_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(pot_kernel(false), cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
-      cudaFuncSetAttribute(pot_kernel(false), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaFuncSetAttribute(pot_kernel(true), cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
-      cudaFuncSetAttribute(pot_kernel(true), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return false;
-  }
-  ctx->cluster_smem_set = size_t(optin);
-  ctx->cluster_nonportable = 1;
-  return true;
-}
-
-// block size of the cluster sweep (pot: the potentials' variant; free: the
-// seam-free colouring's plan)
-static int cluster_threads(const GridDev &g, bool pot, bool free) {
-  if (free) return 32 * (pot ? g.cf_pa + g.cf_pb + g.cf_ps : g.cf_wa + g.cf_wb + g.cf_ws);
-  return 32 * (pot ? g.cl_pa + g.cl_pb + g.cl_ps : g.cl_wa + g.cl_wb + g.cl_ws);
-}
-
-// whether the on-chip cluster sweep (pot: its potentials' variant) can run
-// this grid here, and how many of its clusters are co-resident (asked once
-// per shape: shared memory per CTA, cluster size, block size)
-static bool cluster_usable(x2g_ctx *ctx, const GridDev &g, bool pot = false) {
-  if (g.cl_size < 2 || ctx->no_cluster) return false;
-  const bool free = ctx->mixed_free != 0;
-  const size_t smem = cluster_smem_bytes(g, pot, free);
-  const long key = (long(smem) * 64 + g.cl_size) * 32 + cluster_threads(g, pot, free) / 32;
-  const int v = pot ? 1 : 0;
-  if (ctx->cluster_checked_key[v] != key) {
-    ctx->cluster_checked_key[v] = key;
-    ctx->cluster_ok[v] = 0;
-    const bool attr_ok = cluster_attributes(ctx) && smem <= ctx->cluster_smem_set;
-    if (attr_ok) {
-      cudaLaunchConfig_t q = {};
-      q.gridDim = dim3(unsigned(g.cl_size));
-      q.blockDim = dim3(unsigned(cluster_threads(g, pot, free)));
-      q.dynamicSmemBytes = smem;
-      cudaLaunchAttribute qa[1];
-      qa[0].id = cudaLaunchAttributeClusterDimension;
-      qa[0].val.clusterDim.x = unsigned(g.cl_size);
-      qa[0].val.clusterDim.y = 1;
-      qa[0].val.clusterDim.z = 1;
-      q.attrs = qa;
-      q.numAttrs = 1;
-      int nclusters = 0;
-      const void *fn = pot ? pot_kernel(free) : (const void *)k_mixed_cluster;
-      if (cudaOccupancyMaxActiveClusters(&nclusters, fn, &q) == cudaSuccess && nclusters > 0) {
-        ctx->cluster_ok[v] = 1;
-        ctx->cluster_active[v] = nclusters;
-      }
+// Co-resident clusters of `size` CTAs of a cluster sweep kernel on the
+// context's device (0: it cannot run).  The function's attributes are shared
+// by every context and thread of the process: its dynamic shared memory cap is
+// set to the device's opt-in maximum (never lowered, so concurrent contexts
+// cannot undercut each other) and clusters above 8 CTAs are allowed.
+static int cluster_active(x2g_ctx *ctx, const void *fn, int size, int threads, size_t smem) {
+  if (ctx->cluster_smem < 0) {
+    int optin = 0;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess) {
+      (void)cudaGetLastError();
+      optin = 0;
     }
-    (void)cudaGetLastError();
+    ctx->cluster_smem = optin;
   }
-  return ctx->cluster_ok[v] != 0;
+  if (!fn || smem > size_t(ctx->cluster_smem)) return 0;
+  int n = 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->cluster_smem) == cudaSuccess &&
+      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+    cudaLaunchConfig_t q = {};
+    q.gridDim = dim3(unsigned(size));
+    q.blockDim = dim3(unsigned(threads));
+    q.dynamicSmemBytes = smem;
+    cudaLaunchAttribute qa[1];
+    qa[0].id = cudaLaunchAttributeClusterDimension;
+    qa[0].val.clusterDim.x = unsigned(size);
+    qa[0].val.clusterDim.y = 1;
+    qa[0].val.clusterDim.z = 1;
+    q.attrs = qa;
+    q.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, fn, &q) != cudaSuccess) n = 0;
+  }
+  (void)cudaGetLastError();
+  return n;
+}
+
+// A kernel and band plan of the on-chip sweep.
+struct ColChoice {
+  const ColPlan *plan = nullptr;
+  const void *fn = nullptr;
+  bool sep = false;
+  int rows = 0;
+  size_t smem = 0;
+  int active = 0;  // co-resident clusters
+  int wave = 0;    // jobs of a launch
+};
+
+// The kernels of the on-chip sweep that can run this grid's band plans here,
+// asked once per grid size: plain, sep, sep with two CTAs per SM.
+static const std::vector<x2g_ctx::ColumnShape> &column_shapes(x2g_ctx *ctx, const HostGrid &h) {
+  for (const auto &s : ctx->columns)
+    if (s.nni == h.nni && s.nmu == h.nmu) return s.shapes;
+  x2g_ctx::ColumnShapes out{h.nni, h.nmu, {}};
+  for (size_t i = 0; i < h.columns.size(); ++i)
+    for (int kind = 0; kind < 3; ++kind) {
+      const ColPlan &p = h.columns[i];
+      const int need = std::max(p.pitch, p.warps * 32);
+      const int pitch = need <= kPitchNarrow ? kPitchNarrow : need <= kPitchWide ? kPitchWide : kPitchBroad;
+      // up to 11 warps in a row: two threads per column, or two CTAs per SM
+      if (need > pitch || p.groups != (pitch == kPitchNarrow && kind != 2 ? 2 : 1)) continue;
+      if (kind == 2 && pitch != kPitchNarrow) continue;
+      const ColKernel k = kind == 2               ? column_kernel_pair(p.slots, true)
+                          : pitch == kPitchNarrow ? column_kernel_split(p.slots, kind == 1)
+                          : pitch == kPitchWide   ? column_kernel_wide(p.slots, kind == 1)
+                                                  : column_kernel_broad(p.slots, kind == 1);
+      x2g_ctx::ColumnShape c{int(i), k.fn, kind > 0, column_rows(p, k.slots), 0, 0};
+      c.smem = column_smem(c.rows, pitch, c.sep, p.warps * p.groups * 32);
+      c.active = cluster_active(ctx, c.fn, p.size, p.warps * p.groups * 32, c.smem);
+      if (c.active > 0) out.shapes.push_back(c);
+    }
+  ctx->columns.push_back(std::move(out));
+  return ctx->columns.back().shapes;
+}
+
+// Expected time of one launch of the on-chip sweep over `jobs` jobs, in us for
+// 10 sweeps: a start-up and, per slot (point of a colour in a thread's rows),
+// the latency of a few warps or the issue slots of the warps that share an SM.
+// Clusters rarely fill more than nine tenths of the SMs (whole clusters lie in
+// one group of SMs).  Measured, us: 151x241, two threads per column: 3 slots
+// 57, 4 66, 5 74; 331x481 likewise: 4 slots 96, 5 114; one thread per column,
+// one CTA on an SM: 7 slots 117, 9 139, two: 7 160, 9 207.  So 22 potentials
+// of 331x481 run as one wave of 12-CTA clusters (209) and not as two of 16-CTA
+// ones (320), 64 of 151x241 as two launches of 32 (214; 287 on the kernel with
+// fixed clusters of 8).
+static double column_time(const ColPlan &p, int jobs, int num_sms) {
+  const int share = (jobs * p.size + num_sms * 9 / 10 - 1) / (num_sms * 9 / 10);
+  return 30.0 + p.slots * std::max(12.0, 0.8 * p.warps * p.groups * share);
+}
+
+// The on-chip sweep for njobs jobs (sep: all of them potentials with a
+// separable lhs), or none: the kernel and cluster size with the least expected
+// time for the waves of co-resident clusters they take.
+static ColChoice choose_columns(x2g_ctx *ctx, const HostGrid &h, int njobs, bool sep) {
+  ColChoice best;
+  double best_time = 0;
+  if (ctx->no_cluster) return best;
+  for (const x2g_ctx::ColumnShape &c : column_shapes(ctx, h)) {
+    if (c.sep != sep) continue;
+    const ColPlan &p = h.columns[size_t(c.plan)];
+    const int wave = std::min(c.active, kParamJobs);
+    const double time = njobs / wave * column_time(p, wave, ctx->num_sms) +
+                        (njobs % wave ? column_time(p, njobs % wave, ctx->num_sms) : 0.0);
+    if (!best.plan || time < best_time) {
+      best = {&p, c.fn, sep, c.rows, c.smem, c.active, wave};
+      best_time = time;
+    }
+  }
+  return best;
 }
 
 // Launch shape of the persistent-band sweep: the most jobs per launch (at
@@ -2822,10 +2447,9 @@ static int f64_block_limit(x2g_ctx *ctx) {
   return X2G_OK;
 }
 
-// One launch batch (at most kParamJobs jobs) of launch_relax.
 // One launch of the on-chip cluster sweep over the jobs of jt, timed with the
 // context's events when profiling.
-static int cluster_sweep(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, int nsweeps, bool pot) {
+static int cluster_sweep(x2g_ctx *ctx, const GridDev &g, const ColChoice &c, JobTable &jt, int njobs, int nsweeps) {
   x2g_ctx::Pending pe{};
   if (ctx->profiling) {
     int rc;
@@ -2834,26 +2458,30 @@ static int cluster_sweep(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs
     pe.points = double(njobs) * double(g.nni - 2) * double(g.nmu - 5) * double(nsweeps);
     cudaEventRecord(pe.a, ctx->stream);
   }
-  const int free = ctx->mixed_free;
-  const size_t smem = cluster_smem_bytes(g, pot, free != 0);
-  if (!cluster_attributes(ctx) || smem > ctx->cluster_smem_set)
-    return set_status(X2G_ERR_CUDA, "cluster kernel attributes could not be set");
+  int free = ctx->mixed_free;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(njobs * g.cl_size));
-  cfg.blockDim = dim3(unsigned(cluster_threads(g, pot, free != 0)));
-  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = dim3(unsigned(njobs * c.plan->size));
+  cfg.blockDim = dim3(unsigned(32 * c.plan->warps * c.plan->groups));
+  cfg.dynamicSmemBytes = c.smem;
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = unsigned(g.cl_size);
+  attr[0].val.clusterDim.x = unsigned(c.plan->size);
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   GridDev gd = g;
-  cudaError_t err = !pot ? cudaLaunchKernelEx(&cfg, k_mixed_cluster, gd, jt, nsweeps, free)
-                    : free ? cudaLaunchKernelEx(&cfg, k_mixed_cluster_pot<kPotWarpsFree>, gd, jt, nsweeps, free)
-                           : cudaLaunchKernelEx(&cfg, k_mixed_cluster_pot<kPotWarpsRef>, gd, jt, nsweeps, free);
+  ColPlan plan = *c.plan;
+  plan.rows = c.rows;
+  for (int k = 0; k < 4; ++k) {
+    plan.c2[k] = make_float2(g.dmu2f[k], g.dni2f[k]);
+    plan.c1[k] = make_float2(g.dmu1f[k], g.dni1f[k]);
+  }
+  plan.neg = make_float2(-1.0f, -1.0f);
+  int *err_word = reinterpret_cast<int *>(ctx->bar + 2);
+  void *args[] = {&gd, &plan, &jt, &nsweeps, &free, &err_word};
+  cudaError_t err = cudaLaunchKernelExC(&cfg, c.fn, args);
   if (err != cudaSuccess) return cuda_status(err, "cluster MCSOR launch");
   ctx->launches += 1;
   if (ctx->profiling) {
@@ -2863,59 +2491,60 @@ static int cluster_sweep(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs
   return X2G_OK;
 }
 
-// One launch batch (at most kParamJobs jobs) of launch_relax's mixed form.
-static int relax_batch(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, int nsweeps, bool on_chip, bool pot,
-                       int G, size_t smem) {
+// Mixed form on chip: the jobs in waves of the co-resident clusters.  The
+// first wave's FP64 residual, then each later wave's on the low-priority
+// auxiliary stream, beside the sweep before it (on the SMs and the FP64 pipes
+// that leaves free); each sweep waits for its own wave's residual.  The short
+// wave (the remainder) goes first: its residual is the only one on the
+// critical path.  job(i): the table entry of job i.
+template <class JobOf>
+static int relax_on_chip(x2g_ctx *ctx, const GridDev &g, const ColChoice &col, int njobs, int nsweeps, JobOf job) {
+  const unsigned nblk = unsigned(grid_blocks((g.nni - 2) * (g.nmu - 5)));
+  const bool overlap = ctx->residual_overlap != 0;
+  const int first = njobs % col.wave ? njobs % col.wave : col.wave;
+  cudaError_t err;
+  JobTable cur{}, next{};
+  auto table = [&](int i0, int n, JobTable &t) {
+    for (int i = 0; i < n; ++i) t.j[i] = job(i0 + i);
+  };
+  auto residual = [&](const JobTable &t, int n, cudaStream_t s) {
+    k_residual<false><<<dim3(nblk, unsigned(n)), kThreads, 0, s>>>(g, t, 0, col.sep ? 0 : 1);
+    ctx->launches += 1;
+  };
+  table(0, first, cur);
+  residual(cur, first, ctx->stream);
+  if (overlap && first < njobs &&
+      ((err = cudaEventRecord(ctx->ev_split[0], ctx->stream)) != cudaSuccess ||
+       (err = cudaStreamWaitEvent(ctx->aux, ctx->ev_split[0], 0)) != cudaSuccess))
+    return cuda_status(err, "residual overlap");
+  for (int i0 = 0, n = first, c = 0; i0 < njobs; i0 += n, n = col.wave, ++c) {
+    const bool more = i0 + n < njobs;
+    cudaEvent_t ev = ctx->ev_split[(c + 1) & 1];
+    if (more) {
+      table(i0 + n, col.wave, next);
+      residual(next, col.wave, overlap ? ctx->aux : ctx->stream);
+      if (overlap && (err = cudaEventRecord(ev, ctx->aux)) != cudaSuccess) return cuda_status(err, "residual overlap");
+    }
+    int rc = cluster_sweep(ctx, g, col, cur, n, nsweeps);
+    if (rc) return rc;
+    if (more && overlap && (err = cudaStreamWaitEvent(ctx->stream, ev, 0)) != cudaSuccess)
+      return cuda_status(err, "residual overlap");
+    cur = next;
+  }
+  return X2G_OK;
+}
+
+// Mixed form in persistent bands: one launch batch (at most kParamJobs jobs).
+static int relax_bands(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, int nsweeps, int G, size_t smem) {
   cudaError_t err;
   x2g_ctx::Pending pe{};
-  const double points = double(njobs) * double(g.nni - 2) * double(g.nmu - 5) * double(nsweeps);
-  const int wave = ctx->cluster_active[1];
-  if (on_chip && pot && ctx->residual_overlap && wave > 0 && njobs > wave) {
-    // waves of the potentials' cluster variant: the first wave's FP64
-    // residual, then the later waves' residuals on the low-priority
-    // auxiliary stream, beside the sweeps (on the SMs they leave free);
-    // each sweep waits for its own wave's residual.  The short wave (the
-    // remainder) goes first: its residual is the only one on the critical
-    // path, the full waves' residuals run beside sweeps
-    const int nw = (njobs + wave - 1) / wave;
-    std::vector<JobTable> w(size_t(nw), JobTable{});
-    std::vector<int> sz(size_t(nw), wave);
-    if (njobs % wave) sz[0] = njobs % wave;
-    const unsigned nblk = unsigned(grid_blocks((g.nni - 2) * (g.nmu - 5)));
-    for (int c = 0, i0 = 0; c < nw; i0 += sz[size_t(c)], ++c)
-      for (int i = 0; i < sz[size_t(c)]; ++i) w[size_t(c)].j[i] = jt.j[i0 + i];
-    auto size = [&](int c) { return sz[size_t(c)]; };
-    k_residual<false><<<dim3(nblk, size(0)), kThreads, 0, ctx->stream>>>(g, w[0], 0, 0);
-    ctx->launches += 1;
-    if ((err = cudaEventRecord(ctx->ev_split[0], ctx->stream)) != cudaSuccess ||
-        (err = cudaStreamWaitEvent(ctx->aux, ctx->ev_split[0], 0)) != cudaSuccess)
-      return cuda_status(err, "residual overlap");
-    for (int c = 0; c < nw; ++c) {
-      cudaEvent_t ev = ctx->ev_split[(c + 1) & 1];
-      if (c + 1 < nw) {
-        k_residual<false><<<dim3(nblk, size(c + 1)), kThreads, 0, ctx->aux>>>(g, w[c + 1], 0, 0);
-        ctx->launches += 1;
-        if ((err = cudaEventRecord(ev, ctx->aux)) != cudaSuccess) return cuda_status(err, "residual overlap");
-      }
-      int rc = cluster_sweep(ctx, g, w[c], size(c), nsweeps, true);
-      if (rc) return rc;
-      if (c + 1 < nw && (err = cudaStreamWaitEvent(ctx->stream, ev, 0)) != cudaSuccess)
-        return cuda_status(err, "residual overlap");
-    }
-    return X2G_OK;
-  }
-  const dim3 gr(grid_blocks((g.nni - 2) * (g.nmu - 5)), njobs);
-  if (on_chip)
-    k_residual<false><<<gr, kThreads, 0, ctx->stream>>>(g, jt, 0, pot ? 0 : 1);
-  else
-    k_residual<true><<<gr, kThreads, 0, ctx->stream>>>(g, jt, 1, 1);
+  k_residual<true><<<dim3(grid_blocks((g.nni - 2) * (g.nmu - 5)), njobs), kThreads, 0, ctx->stream>>>(g, jt, 1, 1);
   ctx->launches += 1;
-  if (on_chip) return cluster_sweep(ctx, g, jt, njobs, nsweeps, pot);
   if (ctx->profiling) {
     int rc;
     if ((rc = take_event(ctx, &pe.a)) || (rc = take_event(ctx, &pe.b))) return rc;
     pe.precision = 1;
-    pe.points = points;
+    pe.points = double(njobs) * double(g.nni - 2) * double(g.nmu - 5) * double(nsweeps);
     cudaEventRecord(pe.a, ctx->stream);
   }
   // persistent-band sweep, one block per (job, run of G tiles), phase counts
@@ -3009,13 +2638,11 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
 }
 
 // co-resident clusters of the cluster sweep and of its potentials' variant
-// for this grid on the context's device (0: that kernel cannot run it)
+// for large batches on this grid on the context's device (0: that kernel
+// cannot run it)
 int cluster_occupancy(x2g_ctx *ctx, x2g_grid *grid, int *plain, int *pot) {
-  const GridDev &g = grid->d;
-  const int a = cluster_usable(ctx, g, false) ? ctx->cluster_active[0] : 0;
-  const int b = cluster_usable(ctx, g, true) ? ctx->cluster_active[1] : 0;
-  if (plain) *plain = a;
-  if (pot) *pot = b;
+  if (plain) *plain = choose_columns(ctx, grid->h, kParamJobs, false).active;
+  if (pot) *pot = choose_columns(ctx, grid->h, kParamJobs, true).active;
   return set_status(X2G_OK, "");
 }
 
@@ -3030,23 +2657,25 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
   if (precision == X2G_FP64) return relax_wave(ctx, grid->d, grid->d.mcsor, jobs, njobs, nsweeps, true);
   if (precision != X2G_MIXED) return set_status(X2G_ERR_ARG, "unknown relaxation form");
   const GridDev &g = grid->d;
-  bool on_chip = cluster_usable(ctx, g);
-  // potentials built from orbitals (separable lhs): the variant at two CTAs
-  // per SM when the batch is larger than the clusters co-resident at one
-  bool pot = false;
-  if (on_chip && ctx->pot_clusters != 0) {
-    pot = true;
-    for (int i = 0; i < njobs && pot; ++i) pot = (jobs[i].kind == 1 && !(jobs[i].lhs && jobs[i].rhs));
-    if (pot && ctx->pot_clusters == 2) pot = njobs > ctx->cluster_active[0];
-    pot = pot && cluster_usable(ctx, g, true);
+  // potentials built from orbitals have a separable lhs: batches of them
+  // beyond the plain kernel's clusters take the kernel that forms omega / lhs
+  // itself (22 of 331x481: 210 us, the plain kernel's two waves of 13 and 9
+  // 233; 64 of 151x241 214 and 284); below that both take the same time, and
+  // the plain kernel's results are the persistent-band sweep's bit for bit
+  bool sep = ctx->pot_clusters != 0;
+  for (int i = 0; i < njobs && sep; ++i) sep = (jobs[i].kind == 1 && !(jobs[i].lhs && jobs[i].rhs));
+  ColChoice col = choose_columns(ctx, grid->h, njobs, false);
+  if (sep && (ctx->pot_clusters == 1 || njobs > col.active)) {
+    const ColChoice c = choose_columns(ctx, grid->h, njobs, true);
+    if (c.plan) col = c;
   }
-  if (on_chip && !pot && ctx->auto_band && njobs > ctx->cluster_active[0]) {
+  if (col.plan && !col.sep && ctx->auto_band && njobs > col.active) {
     // more jobs than co-resident clusters: the cluster kernel would run in
     // waves, while the persistent-band kernel may hold the whole batch
     int nj = 0, G1 = 0;
     size_t sm1 = 0;
     const int want = njobs < kParamJobs ? njobs : kParamJobs;
-    if (persistent_shape(ctx, g, want, &nj, &G1, &sm1) == X2G_OK && nj >= want) on_chip = false;
+    if (persistent_shape(ctx, g, want, &nj, &G1, &sm1) == X2G_OK && nj >= want) col = ColChoice();
     set_status(X2G_OK, "");
   }
   // per-job scratch: FP32 correction, residual and omega/lhs
@@ -3054,28 +2683,33 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
       (size_t(g.next) * sizeof(float) + 2 * size_t(g.mxsize) * sizeof(float) + 256) / 256 * 256 + 256;
   char *scratch = static_cast<char *>(ctx_workspace(ctx, per_job * njobs + 256));
   if (!scratch) return set_status(X2G_ERR_ALLOC, "workspace allocation failed");
+  {
+    JobDev d;
+    for (int i = 0; i < njobs; ++i)
+      if (!make_job(jobs[i], d)) return set_status(X2G_ERR_ARG, "bad relaxation job");
+  }
+  auto job = [&](int i) {
+    JobDev d;
+    make_job(jobs[i], d);
+    char *p = scratch + per_job * size_t(i);
+    d.e32 = reinterpret_cast<float *>(p);
+    d.r32 = reinterpret_cast<float *>(p + (size_t(g.next) * sizeof(float) + 127) / 128 * 128);
+    d.w32 = d.r32 + g.mxsize;
+    d.rw = reinterpret_cast<float2 *>(d.r32);  // persistent-band sweep: pairs over r32 and w32
+    return d;
+  };
+  if (col.plan) return relax_on_chip(ctx, g, col, njobs, nsweeps, job);
   // the persistent-band sweep takes as many jobs per launch as give every
   // (job, run of tiles) its own co-resident block
   int per_launch = kParamJobs, G = 0;
   size_t smem = 0;
-  if (!on_chip) {
-    int rc = persistent_shape(ctx, g, njobs < kParamJobs ? njobs : kParamJobs, &per_launch, &G, &smem);
-    if (rc) return rc;
-  }
+  int rc = persistent_shape(ctx, g, njobs < kParamJobs ? njobs : kParamJobs, &per_launch, &G, &smem);
+  if (rc) return rc;
   for (int b0 = 0; b0 < njobs; b0 += per_launch) {
     const int nb = (njobs - b0 < per_launch) ? njobs - b0 : per_launch;
     JobTable jt{};
-    for (int i = 0; i < nb; ++i) {
-      JobDev &d = jt.j[i];
-      if (!make_job(jobs[b0 + i], d)) return set_status(X2G_ERR_ARG, "bad relaxation job");
-      char *p = scratch + per_job * size_t(b0 + i);
-      d.e32 = reinterpret_cast<float *>(p);
-      d.r32 = reinterpret_cast<float *>(p + (size_t(g.next) * sizeof(float) + 127) / 128 * 128);
-      d.w32 = d.r32 + g.mxsize;
-      d.rw = reinterpret_cast<float2 *>(d.r32);  // persistent-band sweep: pairs over r32 and w32
-    }
-    int rc = relax_batch(ctx, g, jt, nb, nsweeps, on_chip, pot, G, smem);
-    if (rc) return rc;
+    for (int i = 0; i < nb; ++i) jt.j[i] = job(b0 + i);
+    if ((rc = relax_bands(ctx, g, jt, nb, nsweeps, G, smem))) return rc;
   }
   // barrier error word: checked by the caller at its next synchronisation
   return X2G_OK;

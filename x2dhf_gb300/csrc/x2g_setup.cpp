@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <numeric>
 
+#include "x2g_columns_plan.h"
 #include "x2g_internal.h"
 
 namespace x2g {
@@ -637,6 +638,12 @@ static std::string build_schedule(HostGrid &g) {
     if (band_of(ra) != band_of(rb)) return "schedule check: dependency crosses a tile";
     if (!(lev[d.second] > lev[d.first])) return "schedule check: level order violated";
   }
+  g.columns.clear();
+  for (int size = 1; size <= kMaxCluster; ++size)
+    for (int groups = 1; groups <= 2; ++groups) {
+      ColPlan cp;
+      if (column_plan(nni, nmu, size, groups, cp)) g.columns.push_back(cp);
+    }
   std::string msg = build_wave_schedule(g, g.order, offs, g.sor);
   if (!msg.empty()) return msg;
   std::vector<int> by_colour;
@@ -691,6 +698,7 @@ void copy_schedule(HostGrid &to, const HostGrid &from) {
   to.st_pts = from.st_pts;
   to.st_off = from.st_off;
   for (int k = 0; k <= HostGrid::kBandRuns; ++k) to.st_rows[k] = from.st_rows[k];
+  to.columns = from.columns;
   to.sor = from.sor;
   to.mcsor = from.mcsor;
 }
