@@ -762,3 +762,74 @@ def test_column_sweep_matches_band_sweep(ctx, nnu, nmu, njobs, nsweeps):
             big = float((y - u).abs().max())
             assert big > 0 and float((x - y).abs().max()) <= 1e-4 * big, (colouring, k, float((x - y).abs().max()) / big)
     g.close()
+
+
+FIXED_POINTS = 1 << 17  # fewest points of a call that take the fixed-point residual
+
+
+@pytest.mark.parametrize("nnu,nmu", [(31, 31), (61, 91), (91, 121), (151, 61)])
+@pytest.mark.parametrize("field", ["zero", "random", "steep", "large", "tiny", "spike", "solved"])
+def test_fixed_point_residual_matches_fma_residual(ctx, nnu, nmu, field):
+    """Batches of potentials built from orbitals take the fixed-point residual, the same
+    problem with explicit lhs and rhs the FMA one.  After one sweep the two
+    differ by the residual's rounding: 17 roundings of terms as large as lhs u,
+    divided by lhs and enlarged tenfold by a sweep (1e-13 of the largest u
+    around), and an FP32 unit of the residual (1e-6 of the largest correction
+    around).  Fields: smooth to the last bits, of no symmetry, falling by 2^-11
+    over the stencil's reach (values beyond the tile's units), at the ends of
+    the exponent range, zero but for single points, and at the fixed point
+    (where the residual is what rounding leaves)."""
+    torch = pytest.importorskip("torch")
+    g = xg.Grid(ctx, nnu, nmu, 2.0, 25.0, 1.0, 1.0)
+    dev = torch.device("cuda:0")
+    gen = torch.Generator().manual_seed(nnu * nmu)
+    f3, e, gg = (torch.tensor(g.table(k).reshape(nmu, nnu)) for k in (7, 3, 9))
+    rand = lambda: torch.randn(nmu, nnu, generator=gen, dtype=torch.float64)  # noqa: E731
+    a, b = rand() * 1e-3, rand() * 1e-3
+    row, col = torch.arange(nmu, dtype=torch.float64)[:, None], torch.arange(nnu, dtype=torch.float64)[None, :]
+    u0 = {"zero": 0 * rand(), "random": rand(), "steep": rand() * torch.exp(-0.95 * row - 0.5 * col), "large": rand() * 1e25,
+          "tiny": rand() * 1e-290, "spike": rand() * (torch.rand(nmu, nnu, generator=gen) < 0.01),
+          "solved": torch.exp(-0.03 * row) * torch.cos(0.01 * col)}[field]
+
+    def ext(x):
+        y = torch.zeros(nmu + 8, nnu + 8, dtype=torch.float64)
+        y[4:nmu + 4, 4:nnu + 4] = x
+        return y.to(dev)
+
+    ea, eb = ext(a), ext(b)
+    jobs_of = []
+    for idel, isym in ((0, 1), (1, -1), (2, 1)) * (FIXED_POINTS // (3 * (nnu - 2) * (nmu - 5)) + 1):
+        lhs, rhs = (f3 + idel * idel * e).reshape(-1).to(dev), (a * b * gg).reshape(-1).to(dev)
+        jobs_of.append((idel, isym, lhs, rhs))
+
+    def run(us, explicit, nsweeps):
+        jobs = [xg.Job(u=u.data_ptr(), omega=1.8, isym=isym, kind=1, idel=idel,
+                       **(dict(lhs=lhs.data_ptr(), rhs=rhs.data_ptr()) if explicit else
+                          dict(psa=ea.data_ptr(), psb=eb.data_ptr())))
+                for u, (idel, isym, lhs, rhs) in zip(us, jobs_of)]
+        ctx.set_potential_clusters(False)
+        torch.cuda.synchronize()
+        try:
+            xg.relax(ctx, g, jobs, nsweeps, xg.MIXED)
+            ctx.synchronize()
+        finally:
+            ctx.set_potential_clusters("auto")
+        return us
+
+    start = [ext(u0) for _ in jobs_of]
+    if field == "solved":
+        for _ in range(40):
+            run(start, True, 10)
+    fma = run([u.clone() for u in start], True, 1)
+    for on_chip in (True, False):
+        ctx.set_mixed_on_chip(on_chip)
+        try:
+            got = run([u.clone() for u in start], False, 1)
+        finally:
+            ctx.set_mixed_on_chip(True)
+        around = lambda x: torch.nn.functional.max_pool2d(x.abs()[None, None], 61, 1, 30)[0, 0]  # noqa: E731
+        for k, (x, y, u) in enumerate(zip(got, fma, start)):
+            bound = 1e-6 * around(y - u) + 1e-13 * around(u)
+            assert torch.isfinite(y).all()
+            assert bool(((x - y).abs() <= bound).all()), (on_chip, k, float(((x - y).abs() / (bound + 1e-300)).max()))
+    g.close()

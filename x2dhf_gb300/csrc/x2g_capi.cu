@@ -1,5 +1,7 @@
 // C ABI of the x2dhf GB300 library: context, grid, relaxation, quadrature
 // entry points and the reference-named link-compatible symbols.
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -334,6 +336,32 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
       cnu[nu * 8 + q] = h.dni2[q] + h.d_nu[nu] * h.dni1[q];
       cnu[nu * 8 + 4 + q] = h.dni2[q] - h.d_nu[nu] * h.dni1[q];
     }
+  // no weight above 2^57 and no point's weights above 2^60 together
+  double most = 0.0, mu_sum = 0.0, nu_sum = 0.0;
+  for (const auto *v : {&cmo, &cmp, &cnu})
+    for (size_t k = 8; k < v->size() - 8; k += 8) {  // the axes have no points
+      double sum = 0.0;
+      for (size_t q = k; q < k + 8; ++q) {
+        sum += std::fabs((*v)[q]);
+        most = std::max(most, std::fabs((*v)[q]));
+      }
+      double &to = v == &cnu ? nu_sum : mu_sum;
+      to = std::max(to, sum);
+    }
+  d.wscale = std::min(57 - (std::ilogb(most) + 1), 60 - (std::ilogb(mu_sum + nu_sum) + 1));
+  auto fixed = [&](const std::vector<double> &v) {
+    std::vector<int2> w(v.size());
+    for (size_t k = 8; k < v.size() - 8; ++k) {
+      const long long x = std::llrint(std::ldexp(v[k], d.wscale)), hi = (x + (1ll << 28)) >> 29;
+      w[k] = make_int2(int(hi), int(x - hi * (1ll << 29)));
+    }
+    return w;
+  };
+  std::vector<int> place(h.st_pts.size());
+  for (size_t k = 0; k < place.size(); ++k) {
+    const int row = h.st_pts[k] >> 16, col = h.st_pts[k] & 0xffff;
+    place[size_t(row - 5) * (h.nni - 2) + col - 5] = int(k);
+  }
   const void *tmp;
   int rc = X2G_OK;
 #define UPTO(vec, dest)                                                                 \
@@ -399,6 +427,11 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
   UP(cmo, cmu_orb);
   UP(cmp, cmu_pot);
   UP(cnu, cnu);
+  const std::vector<int2> fixed_mo = fixed(cmo), fixed_mp = fixed(cmp), fixed_nu = fixed(cnu);
+  UP(fixed_mo, wmu_orb);
+  UP(fixed_mp, wmu_pot);
+  UP(fixed_nu, wnu);
+  UP(place, st_place);
 #undef UP
 #undef UPTO
   {

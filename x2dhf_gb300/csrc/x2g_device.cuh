@@ -9,18 +9,15 @@ namespace x2g {
 // issues conversion instructions on its narrow FP64 pipe); values beyond the
 // float range become infinities, values below its normal range signed zero
 __device__ __forceinline__ float narrow_f64(double x) {
-  const unsigned hi = unsigned(__double2hiint(x)), lo = unsigned(__double2loint(x));
-  const unsigned sign = hi & 0x80000000u;
-  const int dex = int((hi >> 20) & 0x7ffu);
-  if (dex == 0x7ff) return __uint_as_float(sign | 0x7f800000u | ((hi & 0xfffffu) ? 0x400000u : 0u));
-  const int fex = dex - 896;
-  if (fex >= 255) return __uint_as_float(sign | 0x7f800000u);
-  if (fex <= 0) return __uint_as_float(sign);
-  // 23 mantissa bits: 20 from hi, 3 from lo; the remaining 29 bits round
-  unsigned bits = (unsigned(fex) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
-  const unsigned rest = lo & 0x1fffffffu;
-  if (rest > 0x10000000u || (rest == 0x10000000u && (bits & 1u))) ++bits;  // may carry into the exponent
-  return __uint_as_float(sign | bits);
+  const unsigned hi = unsigned(__double2hiint(x)), lo = unsigned(__double2loint(x)), mag = hi & 0x7fffffffu;
+  // 24 bits: 21 from hi, 3 from lo; the remaining 29 round (a carry may go
+  // into the exponent)
+  const unsigned long long t = ((unsigned long long)mag << 32 | lo) + (0x0fffffffu + (lo >> 29 & 1u));
+  unsigned f = unsigned(t >> 29) - (896u << 23);
+  f = mag >= (1151u << 20) ? 0x7f800000u : f;
+  f = mag > 0x7ff00000u || (mag == 0x7ff00000u && lo != 0) ? 0x7fc00000u : f;
+  f = mag < (897u << 20) ? 0u : f;
+  return __uint_as_float(hi & 0x80000000u | f);
 }
 
 // float -> double by bit manipulation on the integer pipes (GB300 issues
@@ -33,6 +30,27 @@ __device__ __forceinline__ double widen_f32(float f) {
   if (ex == 0) return __hiloint2double(int(sign), 0);
   const unsigned dex = (ex == 0xffu) ? 0x7ffu : ex + 896u;
   return __hiloint2double(int(sign | (dex << 20) | (m >> 3)), int(m << 29));
+}
+
+// u at ext (row, col) with the putin ghost cells (inout.F90:47-80) read as
+// the mirrored interior value, negated for odd functions (a sign-bit flip);
+// the corner ghosts, never filled by putin, are not reachable by the cross
+// stencil
+__device__ __forceinline__ double ghost_read(const GridDev &g, const double *u, int row, int col, int isym) {
+  bool m = false;
+  if (col < 4) {
+    col = 8 - col;
+    m = true;
+  } else if (col > g.nni + 3) {
+    col = 2 * g.nni + 6 - col;
+    m = true;
+  }
+  if (row < 4) {
+    row = 8 - row;
+    m = true;
+  }
+  const double v = u[row * g.n8 + col];
+  return (m && isym != 1) ? __longlong_as_double(__double_as_longlong(v) ^ (1ll << 63)) : v;
 }
 
 // FP64 axis extrapolation of one point from its 5 neighbours at stride st

@@ -170,6 +170,11 @@ struct GridDev {
   // q] = dmu2 + b dmu1 (q < 4, before) and dmu2 - b dmu1 (q >= 4, after) with
   // b = borb or bpot; cnu[nu * 8 + q] likewise with dni2, d(nu), dni1
   const double *cmu_orb, *cmu_pot, *cnu;
+  // the same as fixed-point numbers w 2^wscale = .x 2^29 + .y with |.x| <=
+  // 2^28, |.y| <= 2^28, and the place of interior point (mu, nu) in st_pts
+  const int2 *wmu_orb, *wmu_pot, *wnu;
+  int wscale;
+  const int *st_place;
   // per-grid moment tables (built on the device at grid creation):
   // exm[(idel * 8 + q) * mxsize + k] = wgt2 f4 P_{q+1}^idel(cos th) (r2 r)^(q+1)
   // for idel 0..4, q < mpole; asy[slot * 4 nni + p] on the 4 boundary rows

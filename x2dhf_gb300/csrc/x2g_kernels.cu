@@ -1028,98 +1028,6 @@ __device__ __forceinline__ void ghost_point(const GridDev &g, double *u, int k, 
   }
 }
 
-// u at ext (row, col) with the putin ghost cells (inout.F90:47-80) read as
-// the mirrored interior value, negated for odd functions (a sign-bit flip);
-// the corner ghosts, never filled by putin, are not reachable by the cross
-// stencil
-__device__ __forceinline__ double ghost_read(const GridDev &g, const double *u, int row, int col, int isym) {
-  bool m = false;
-  if (col < 4) {
-    col = 8 - col;
-    m = true;
-  } else if (col > g.nni + 3) {
-    col = 2 * g.nni + 6 - col;
-    m = true;
-  }
-  if (row < 4) {
-    row = 8 - row;
-    m = true;
-  }
-  const double v = u[row * g.n8 + col];
-  return (m && isym != 1) ? __longlong_as_double(__double_as_longlong(v) ^ (1ll << 63)) : v;
-}
-
-// Mixed form residual r = rhs - A u in FP64 over the interior, stored as
-// FP32 with omega / lhs; the stencil uses the grid's separable weights (one
-// FMA per neighbour) and reads the ghost cells as mirrored interior values,
-// so u needs no ghost refresh first.  kPacked: the points are taken in
-// st_pts order and stored as (r, w) pairs in that order (persistent-band
-// sweep);
-// otherwise r32 / w32 are plain nni x nmu arrays (cluster sweep; need_w 0:
-// the potentials' cluster sweep forms omega / lhs itself, only r32 is
-// stored).
-template <bool kPacked>
-__global__ void k_residual(GridDev g, const __grid_constant__ JobTable jobs, int zero_e, int need_w) {
-  const JobDev &J = jobs.j[blockIdx.y];
-  const int nint = (g.nni - 2) * (g.nmu - 5);
-  const int n8 = g.n8;
-  if (zero_e)
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < g.next; k += gridDim.x * blockDim.x) J.e32[k] = 0.0f;
-  const double *cmu = (J.kind == 0) ? g.cmu_orb : g.cmu_pot;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nint; k += gridDim.x * blockDim.x) {
-    int mu, nu;
-    if (kPacked) {
-      const int rc = g.st_pts[k];
-      mu = (rc >> 16) - 4;
-      nu = (rc & 0xffff) - 4;
-    } else {
-      mu = 1 + k / (g.nni - 2);
-      nu = 1 + k % (g.nni - 2);
-    }
-    const int ik = mu * g.nni + nu, ij = (mu + 4) * n8 + nu + 4;
-    const double *u = J.u;
-    double rhs, lhs;
-    if (J.kind == 1) {
-      rhs = (J.psa[ij] * J.psb[ij]) * g.g[ik];
-      lhs = (J.idel2 == 0.0) ? g.f3_mu[mu] : fma(J.idel2, g.e[ik], g.f3_mu[mu]);
-    } else {
-      rhs = J.rhs[ik];
-      lhs = J.lhs[ik];
-    }
-    const double *cm = cmu + mu * 8, *cn = g.cnu + nu * 8;
-    double cc = lhs * u[ij];
-    if (mu >= 4 && nu >= 4 && nu <= g.nni - 5) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int dm = (4 - q) * n8, dn = 4 - q;
-        cc = fma(cm[q], u[ij - dm], cc);
-        cc = fma(cm[4 + q], u[ij + dm], cc);
-        cc = fma(cn[q], u[ij - dn], cc);
-        cc = fma(cn[4 + q], u[ij + dn], cc);
-      }
-    } else {
-      // the stencil reaches the putin ghosts: read them as mirrored interior
-      // values
-      const int row = mu + 4, col = nu + 4;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int d = 4 - q;
-        cc = fma(cm[q], ghost_read(g, u, row - d, col, J.isym), cc);
-        cc = fma(cm[4 + q], u[ij + d * n8], cc);
-        cc = fma(cn[q], ghost_read(g, u, row, col - d, J.isym), cc);
-        cc = fma(cn[4 + q], ghost_read(g, u, row, col + d, J.isym), cc);
-      }
-    }
-    if (kPacked) {
-      J.rw[k] = make_float2(narrow_f64(rhs - cc), J.omegaf / narrow_f64(lhs));
-    } else {
-      J.r32[ik] = narrow_f64(rhs - cc);
-      if (need_w) J.w32[ik] = J.omegaf / narrow_f64(lhs);
-    }
-  }
-}
-
-
 // ----------------------------------------------------------------------
 // Elementwise kernels of the SCF path
 // ----------------------------------------------------------------------
@@ -2498,8 +2406,8 @@ static int cluster_sweep(x2g_ctx *ctx, const GridDev &g, const ColChoice &c, Job
 // wave (the remainder) goes first: its residual is the only one on the
 // critical path.  job(i): the table entry of job i.
 template <class JobOf>
-static int relax_on_chip(x2g_ctx *ctx, const GridDev &g, const ColChoice &col, int njobs, int nsweeps, JobOf job) {
-  const unsigned nblk = unsigned(grid_blocks((g.nni - 2) * (g.nmu - 5)));
+static int relax_on_chip(x2g_ctx *ctx, const GridDev &g, const ColChoice &col, int njobs, int nsweeps, bool fixed,
+                         JobOf job) {
   const bool overlap = ctx->residual_overlap != 0;
   const int first = njobs % col.wave ? njobs % col.wave : col.wave;
   cudaError_t err;
@@ -2508,7 +2416,7 @@ static int relax_on_chip(x2g_ctx *ctx, const GridDev &g, const ColChoice &col, i
     for (int i = 0; i < n; ++i) t.j[i] = job(i0 + i);
   };
   auto residual = [&](const JobTable &t, int n, cudaStream_t s) {
-    k_residual<false><<<dim3(nblk, unsigned(n)), kThreads, 0, s>>>(g, t, 0, col.sep ? 0 : 1);
+    launch_residual(g, t, n, fixed, false, !col.sep, s);
     ctx->launches += 1;
   };
   table(0, first, cur);
@@ -2535,10 +2443,11 @@ static int relax_on_chip(x2g_ctx *ctx, const GridDev &g, const ColChoice &col, i
 }
 
 // Mixed form in persistent bands: one launch batch (at most kParamJobs jobs).
-static int relax_bands(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, int nsweeps, int G, size_t smem) {
+static int relax_bands(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, int nsweeps, bool fixed, int G,
+                       size_t smem) {
   cudaError_t err;
   x2g_ctx::Pending pe{};
-  k_residual<true><<<dim3(grid_blocks((g.nni - 2) * (g.nmu - 5)), njobs), kThreads, 0, ctx->stream>>>(g, jt, 1, 1);
+  launch_residual(g, jt, njobs, fixed, true, true, ctx->stream);
   ctx->launches += 1;
   if (ctx->profiling) {
     int rc;
@@ -2637,6 +2546,8 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
   return X2G_OK;
 }
 
+constexpr long kFixedPoints = 1 << 17;  // fewest points of a call whose residuals are taken in fixed point
+
 // co-resident clusters of the cluster sweep and of its potentials' variant
 // for large batches on this grid on the context's device (0: that kernel
 // cannot run it)
@@ -2662,10 +2573,10 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
   // itself (22 of 331x481: 210 us, the plain kernel's two waves of 13 and 9
   // 233; 64 of 151x241 214 and 284); below that both take the same time, and
   // the plain kernel's results are the persistent-band sweep's bit for bit
-  bool sep = ctx->pot_clusters != 0;
-  for (int i = 0; i < njobs && sep; ++i) sep = (jobs[i].kind == 1 && !(jobs[i].lhs && jobs[i].rhs));
+  bool separable = true;
+  for (int i = 0; i < njobs && separable; ++i) separable = (jobs[i].kind == 1 && !(jobs[i].lhs && jobs[i].rhs));
   ColChoice col = choose_columns(ctx, grid->h, njobs, false);
-  if (sep && (ctx->pot_clusters == 1 || njobs > col.active)) {
+  if (separable && (ctx->pot_clusters == 1 || (ctx->pot_clusters == 2 && njobs > col.active))) {
     const ColChoice c = choose_columns(ctx, grid->h, njobs, true);
     if (c.plan) col = c;
   }
@@ -2678,6 +2589,10 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
     if (persistent_shape(ctx, g, want, &nj, &G1, &sm1) == X2G_OK && nj >= want) col = ColChoice();
     set_status(X2G_OK, "");
   }
+  // their stencil sums in fixed point, where there are tiles enough: 22 of
+  // 331x481 80 us (FMAs 149), 22 of 151x241 42 (54), one of 331x481 13 (14);
+  // one of 151x241 takes 9 (4).  The same for every sweep kernel and wave
+  const bool fixed = separable && long(njobs) * (g.nni - 2) * (g.nmu - 5) >= kFixedPoints;
   // per-job scratch: FP32 correction, residual and omega/lhs
   const size_t per_job =
       (size_t(g.next) * sizeof(float) + 2 * size_t(g.mxsize) * sizeof(float) + 256) / 256 * 256 + 256;
@@ -2698,7 +2613,7 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
     d.rw = reinterpret_cast<float2 *>(d.r32);  // persistent-band sweep: pairs over r32 and w32
     return d;
   };
-  if (col.plan) return relax_on_chip(ctx, g, col, njobs, nsweeps, job);
+  if (col.plan) return relax_on_chip(ctx, g, col, njobs, nsweeps, fixed, job);
   // the persistent-band sweep takes as many jobs per launch as give every
   // (job, run of tiles) its own co-resident block
   int per_launch = kParamJobs, G = 0;
@@ -2709,7 +2624,7 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
     const int nb = (njobs - b0 < per_launch) ? njobs - b0 : per_launch;
     JobTable jt{};
     for (int i = 0; i < nb; ++i) jt.j[i] = job(b0 + i);
-    if ((rc = relax_bands(ctx, g, jt, nb, nsweeps, G, smem))) return rc;
+    if ((rc = relax_bands(ctx, g, jt, nb, nsweeps, fixed, G, smem))) return rc;
   }
   // barrier error word: checked by the caller at its next synchronisation
   return X2G_OK;

@@ -51,6 +51,11 @@ struct AsymptArgs {
 };
 
 // ---- sweeps ----
+// mixed form: FP64 residuals of njobs jobs as FP32; packed: (r, omega / lhs)
+// pairs in st_pts order with the correction zeroed (persistent-band sweep),
+// otherwise plain nni x nmu arrays r32 and, with need_w, w32
+void launch_residual(const GridDev &g, const JobTable &jobs, int njobs, bool fixed, bool packed, bool need_w,
+                     cudaStream_t s);
 int cluster_occupancy(x2g_ctx *ctx, x2g_grid *grid, int *plain, int *pot);
 int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, int nsweeps, int precision);
 // FP64 sweep whose job table, right-hand-side buffers and barrier words live
