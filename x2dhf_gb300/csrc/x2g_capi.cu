@@ -420,6 +420,10 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
     wd.nblev = w.nblev;
     wd.delta = w.delta;
   }
+  std::vector<int2> march(h.march_pts.size());
+  for (size_t k = 0; k < march.size(); ++k) march[k] = make_int2(h.march_pts[k], h.march_mask[k]);
+  UPTO(march, d.march.pts);
+  UPTO(h.march_off, d.march.off);
   for (int k = 0; k <= HostGrid::kBandRuns; ++k) d.st_rows[k] = h.st_rows[k];
   UP(b32, borb_mu32);
   UP(p32, bpot_mu32);

@@ -127,6 +127,12 @@ struct HostGrid {
   int st_rows[kBandRuns + 1] = {};
   // bands of the on-chip FP32 sweep, by cluster size and threads per column
   std::vector<ColPlan> columns;
+  // SOR's points of ext rows 4..nmu-1 (4: the mu=1 axis) by row and side of
+  // the middle column, in list order: row r's left (right) points are entries
+  // [march_off[2(r-4)], march_off[2(r-4)+1]) (then up to march_off[2(r-4)+2])
+  // of march_pts (ext index) and march_mask (sor.mask, kMarchAxis... for axis
+  // points and the stride to what they read); a side ends with its axis point
+  std::vector<int> march_pts, march_mask, march_off;
   // the FP64 sweeps' wavefront schedules (build_wave_schedule): list-order
   // SOR over the "middle" list (sor, sormcsor.F90:20-132), and MCSOR as the
   // same sweep over the list colour after colour (mcsor, :143-386)
@@ -146,6 +152,14 @@ struct WaveDev {
   int nlev, nblev, delta;
 };
 
+// SOR's points by row and side (HostGrid::march_pts): (ext index, mask)
+struct MarchDev {
+  const int2 *pts;
+  const int *off;
+};
+constexpr unsigned kMarchAxisMu = 1u << 20, kMarchAxisUp = 1u << 21, kMarchAxisDown = 1u << 22;
+constexpr unsigned kMarchAxis = kMarchAxisMu | kMarchAxisUp | kMarchAxisDown;
+
 // ----------------------------------------------------------------------
 // Device view of a grid, passed by value to kernels.
 // ----------------------------------------------------------------------
@@ -162,6 +176,7 @@ struct GridDev {
   const int *st_pts, *st_off;
   int st_rows[17];
   WaveDev sor, mcsor;
+  MarchDev march;
   // FP32 copies of the coefficient tables for the mixed form
   const float *borb_mu32, *bpot_mu32, *d_nu32;
   const double *e_mu, *e_nu;
@@ -273,6 +288,7 @@ struct x2g_ctx {
   int band_blocks = 0;          // co-resident blocks for that size
   int band_sm_smem = 0;         // shared memory per SM
   int f64_blocks = -1;          // co-resident blocks of the cooperative FP64 sweep on this device
+  int march_smem = -1;          // shared memory that a block of the marching SOR sweep may have (0: it cannot run)
   int wave_ok = -1;             // the wavefront kernels can be co-resident, one block per SM
   int ortho_blocks = -1;        // co-resident blocks of the one-launch orthonormalisation
   int gram_blocks = -1;         // co-resident blocks of its Gram-matrix form

@@ -723,16 +723,11 @@ __device__ __forceinline__ bool wave_points1(const GridDev &g, const JobTable &j
   return true;
 }
 
-template <int kSplit>
-__global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev w, const __grid_constant__ JobTable jobs,
-                                                             int njobs, int nsweeps, BarrierDev bar, unsigned nblocks) {
-  extern __shared__ int s_off[];
-  const int nt = int(gridDim.x * blockDim.x), id = int(blockIdx.x * blockDim.x + threadIdx.x);
-  for (int k = threadIdx.x; k <= w.nlev; k += blockDim.x) s_off[k] = w.off[k];
-  for (int k = threadIdx.x; k <= w.nblev; k += blockDim.x) s_off[w.nlev + 1 + k] = w.boff[k];
-  // the tagged copy of every function, its ghost cells refreshed as putin
-  // does (in u too), and the (lhs, rhs) pairs: a potential's lhs = f3 +
-  // idel^2 e and rhs = psa psb g with the roundings of relaxPots.F90:81-95
+// Threads id of nt: the tagged copy of every function, its ghost cells
+// refreshed as putin does (in u too), and the (lhs, rhs) pairs: a potential's
+// lhs = f3 + idel^2 e and rhs = psa psb g with the roundings of
+// relaxPots.F90:81-95.
+__device__ __forceinline__ void wave_prologue(const GridDev &g, const JobTable &jobs, int njobs, int id, int nt) {
   for (int jb = 0; jb < njobs; ++jb) {
     const JobDev &J = jobs.j[jb];
     for (int k = id; k < g.next; k += nt) {
@@ -765,6 +760,16 @@ __global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev
       pairs[k] = lr;
     }
   }
+}
+
+template <int kSplit>
+__global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev w, const __grid_constant__ JobTable jobs,
+                                                             int njobs, int nsweeps, BarrierDev bar, unsigned nblocks) {
+  extern __shared__ int s_off[];
+  const int nt = int(gridDim.x * blockDim.x), id = int(blockIdx.x * blockDim.x + threadIdx.x);
+  for (int k = threadIdx.x; k <= w.nlev; k += blockDim.x) s_off[k] = w.off[k];
+  for (int k = threadIdx.x; k <= w.nblev; k += blockDim.x) s_off[w.nlev + 1 + k] = w.boff[k];
+  wave_prologue(g, jobs, njobs, id, nt);
   if (!grid_barrier(bar, nblocks)) return;
   WaveWalk<kSplit> walk;
   walk.off = s_off;
@@ -799,6 +804,234 @@ __global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev
       ok = wave_points1(g, jobs, it, nsweeps, bar);
     if (!ok) return;
     it = nx;
+  }
+}
+
+// ----------------------------------------------------------------------
+// List-order SOR of a few functions: the same dataflow on values in shared
+// memory.  A block owns four rows of one job (the mu=1 row included) for the
+// whole launch and keeps them, with four rows on each side, as (value, tag)
+// words in shared memory; warp s of its kMarchSweeps takes sweeps s, s +
+// kMarchSweeps, ..., four lanes for each of its eight runners: a row's columns
+// from the middle to one side, in list order, then the axis.  A runner goes on
+// as soon as its point's values are there, so the rows of a warp settle one
+// column apart.  The other warps fetch the neighbours' rows, a lane per row,
+// side and sweep, from the tagged copy in global memory.  A value of a row
+// outside the block's own is overwritten there only after its readers in this
+// block are through (see above), so the copies need no further order.
+//
+// What bounds it: the FP64 chain of a point (2240 cycles of the 4000 that a
+// step of one sweep takes) while a block has few runners at work, and the SM's
+// FP64 pipe when all of them are (ten warps of 24 operations a point, 19 cycles
+// each).  The way of a value through L2, most of a step's 5800 cycles when
+// every value takes it, is paid once per four rows.  SOR, 10 sweeps of one
+// orbital, wavefront / this: 331 x 481 2.26 / 1.52 ms, 151 x 181 0.93 / 0.68
+// ms, 91 x 121 0.62 / 0.46 ms.
+// ----------------------------------------------------------------------
+constexpr int kMarchRows = 4, kMarchSweeps = 10;
+constexpr int kMarchFetch = (8 * 2 * kMarchSweeps + 31) / 32;  // warps that fetch
+constexpr int kMarchThreads = 32 * (kMarchSweeps + kMarchFetch);
+
+__device__ __forceinline__ Tagged ld_near(unsigned at) {
+  unsigned long long lo, hi;
+  asm volatile("ld.volatile.shared.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(at) : "memory");
+  return Tagged{__longlong_as_double((long long)lo), int(unsigned(hi))};
+}
+__device__ __forceinline__ void st_near(unsigned at, double v, int tag) {
+  asm volatile("st.volatile.shared.v2.b64 [%0], {%1, %2};" ::"r"(at), "l"(__double_as_longlong(v)),
+               "l"((unsigned long long)(unsigned)tag)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kMarchThreads, 1)
+    k_march_f64(GridDev g, MarchDev w, const __grid_constant__ JobTable jobs, int njobs, int nsweeps, BarrierDev bar,
+                unsigned nblocks) {
+  extern __shared__ __align__(16) ulonglong2 near[];
+  const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
+  wave_prologue(g, jobs, njobs, int(blockIdx.x) * kMarchThreads + tid, int(gridDim.x) * kMarchThreads);
+  if (!grid_barrier(bar, nblocks)) return;
+  const int bands = int(gridDim.x) / njobs, jb = int(blockIdx.x) / bands;
+  const JobDev &J = jobs.j[jb];
+  const int n8 = g.n8, nmu = g.nmu;
+  const int r0 = 4 + (int(blockIdx.x) - jb * bands) * kMarchRows;
+  const unsigned base = unsigned(__cvta_generic_to_shared(near));
+  // shared address of ext index ij: rows r0 - 4 .. r0 + 7
+  const int first = (r0 - 4) * n8;
+  auto addr = [&](int ij) { return base + unsigned(ij - first) * 16u; };
+  for (int k = tid; k < (kMarchRows + 8) * n8; k += kMarchThreads) {
+    const int ij = min(first + k, g.next - 1);
+    const Tagged x = ld_tagged(J.tagged + ij);
+    st_near(base + unsigned(k) * 16u, x.v, x.tag);
+  }
+  __syncthreads();
+  WaveWait ww;
+  if (warp >= kMarchSweeps) {
+    // fetch: rows r0 - 4 .. r0 - 1 and r0 + 4 .. r0 + 7
+    const int id = tid - 32 * kMarchSweeps, h = id & 7, half = id >> 3 & 1, slot = id >> 4;
+    const int row = h < 4 ? r0 - 4 + h : r0 + kMarchRows + h - 4;
+    bool on = slot < kMarchSweeps && row >= 4 && row < nmu;
+    int s = slot, k = 0, n = 0, o = 0;
+    if (on) {
+      o = w.off[(row - 4) * 2 + half];
+      n = w.off[(row - 4) * 2 + half + 1] - o;
+    }
+    on = on && s < nsweeps && n > 0;
+    int ij = on ? __ldg(&w.pts[o].x) : 0;
+    while (__any_sync(0xffffffffu, on)) {
+      bool got = false;
+      if (on) {
+        const Tagged x = ld_tagged(J.tagged + ij);
+        got = x.tag > s;
+        if (got) {
+          st_near(addr(ij), x.v, x.tag);
+          if (++k == n) {
+            k = 0;
+            s += kMarchSweeps;
+            on = s < nsweeps;
+          }
+          ij = __ldg(&w.pts[o + k].x);
+        }
+      }
+      if (!__any_sync(0xffffffffu, got) && !__all_sync(0xffffffffu, ww.again(bar))) return;
+      if (__any_sync(0xffffffffu, got)) ww = WaveWait();
+    }
+    return;
+  }
+  const int role = lane & 3, row = r0 + (lane >> 3), half = lane >> 2 & 1;
+  double cf[4];
+  {
+    const double *c = role == 0 ? g.dmu2 : role == 1 ? g.dmu1 : role == 2 ? g.dni2 : g.dni1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) cf[q] = c[q];
+  }
+  const int st = role < 2 ? n8 : 1, bit = role < 2 ? 2 : 0;
+  const double omega = J.omega, omega1 = 1.0 - J.omega;
+  const double bmu = row < nmu ? (J.kind >= 1 ? g.bpot_mu : g.borb_mu)[row - 4] : 0.0;
+  int o = 0, n = 0;
+  if (row < nmu) {
+    o = w.off[(row - 4) * 2 + half];
+    n = w.off[(row - 4) * 2 + half + 1] - o;
+  }
+  const double2 *pairs = reinterpret_cast<const double2 *>(J.pairs) - 4 * g.nni - 4;  // by ext row * nni + ext col
+  for (int s = warp; s < nsweeps; s += kMarchSweeps) {
+    int k = 0;
+    bool on = n > 0;
+    int2 cur = on ? __ldg(w.pts + o) : make_int2(0, 0), nxt = cur;
+    if (n > 1) nxt = __ldg(w.pts + o + 1);
+    auto coef = [&](const int2 &e, double2 &lr, double &d) {
+      if (on && !(unsigned(e.y) & kMarchAxis)) {
+        const int col = e.x - row * n8;
+        lr = __ldcg(pairs + row * g.nni + col);
+        d = __ldg(g.d_nu + col - 4);
+      }
+    };
+    double2 lr = make_double2(1.0, 0.0), lr_n = lr;
+    double dnu = 0.0, dnu_n = 0.0;
+    coef(cur, lr, dnu);
+    double m[4], p[4], uc = 0.0;
+    unsigned miss = 0;
+    bool fresh = true;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) m[q] = p[q] = 0.0;
+    while (__any_sync(0xffffffffu, on)) {
+      const int ij = cur.x;
+      const unsigned mask = unsigned(cur.y), at = addr(ij);
+      const bool axis = (mask & kMarchAxis) != 0;
+      const int ast = axis ? ((mask & kMarchAxisMu) ? n8 : (mask & kMarchAxisUp) ? 1 : -1) : 0;
+      int other = 0;  // a value that is read by this point's value and does not read it back
+      if (fresh) {
+        coef(nxt, lr_n, dnu_n);
+        miss = !on ? 0u : axis ? (role == 0 ? 0x21fu : 0u) : 0x3ffu;
+        fresh = false;
+      }
+      if (axis) {
+        if ((mask & kMarchAxisMu) && ij - row * n8 <= 9) other = row * n8 + 4;
+        else if ((mask & kMarchAxisMu) && ij - row * n8 >= g.nni - 2) other = row * n8 + g.nni + 3;
+      } else if (role != 1) {
+        other = fifth_reader(g, mask, ij, role == 0 ? 0 : 1);
+      }
+      if (!other) miss &= ~0x200u;
+      if (axis) {
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+          if (miss & (1u << q)) {
+            const Tagged x = ld_near(at + unsigned((q + 1) * ast * 16));
+            if (x.tag > s) {
+              if (q < 4) m[q] = x.v;
+              else uc = x.v;
+              miss &= ~(1u << q);
+            }
+          }
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int e = 4 * (3 - q) + bit;
+          if (miss & (1u << q)) {
+            const Tagged x = ld_near(at - unsigned((4 - q) * st * 16));
+            if (x.tag >= s + int((mask >> e) & 1u)) {
+              m[q] = x.v;
+              miss &= ~(1u << q);
+            }
+          }
+          if (miss & (16u << q)) {
+            const Tagged y = ld_near(at + unsigned((4 - q) * st * 16));
+            if (y.tag >= s + int((mask >> (e + 1)) & 1u)) {
+              p[q] = y.v;
+              miss &= ~(16u << q);
+            }
+          }
+        }
+        if (miss & 256u) {
+          const Tagged c = ld_near(at);
+          if (c.tag >= s) {
+            uc = c.v;
+            miss &= ~256u;
+          }
+        }
+      }
+      if ((miss & 512u) && ld_near(addr(other)).tag >= s) miss &= ~512u;
+      const unsigned waits = __ballot_sync(0xffffffffu, miss != 0);
+      const bool ready = on && (waits >> (lane & 28) & 0xfu) == 0;
+      if (!__any_sync(0xffffffffu, ready)) {
+        if (!__all_sync(0xffffffffu, ww.again(bar))) return;
+        continue;
+      }
+      ww = WaveWait();
+      double v = 0.0;
+      if (__any_sync(0xffffffffu, ready && !axis)) {
+        // as wave_points4
+        const long long flip = (role & 1) ? (1ll << 63) : 0;
+        double a[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a[q] = A(m[q], __longlong_as_double(__double_as_longlong(p[q]) ^ flip));
+        double t = A(A(A(M(cf[0], a[0]), M(cf[1], a[1])), M(cf[2], a[2])), M(cf[3], a[3]));
+        t = M(role == 1 ? bmu : role == 3 ? dnu : 1.0, t);
+        const int b = lane & 28;
+        const double ddmi2 = __shfl_sync(0xffffffffu, t, b), bddmi1 = __shfl_sync(0xffffffffu, t, b + 1);
+        const double ddni2 = __shfl_sync(0xffffffffu, t, b + 2), dddni1 = __shfl_sync(0xffffffffu, t, b + 3);
+        const double cc = A(A(A(ddmi2, bddmi1), ddni2), dddni1);
+        v = A(D(M(omega, S(lr.y, cc)), lr.x), M(omega1, uc));
+      }
+      if (ready && axis && role == 0) {
+        v = 0.0;
+        if (J.isym == 1)
+          v = A(A(A(A(M(g.exeven[0], m[0]), M(g.exeven[1], m[1])), M(g.exeven[2], m[2])), M(g.exeven[3], m[3])),
+                M(g.exeven[4], uc));
+      }
+      if (ready) {
+        if (role == 0) {
+          st_near(at, v, s + 1);
+          wave_store(J, ij, v, s, nsweeps);
+        }
+        cur = nxt;
+        lr = lr_n;
+        dnu = dnu_n;
+        fresh = true;
+        on = ++k < n;
+        if (k + 1 < n) nxt = __ldg(w.pts + o + k + 1);
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -2479,6 +2712,24 @@ static int relax_bands(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, 
   return X2G_OK;
 }
 
+// whether a block of the marching SOR sweep can be resident with this much
+// shared memory (its cap is set to the device's opt-in maximum, once)
+static bool march_fits(x2g_ctx *ctx, size_t smem) {
+  if (ctx->march_smem < 0) {
+    int optin = 0, a = 0;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess ||
+        (optin -= 1024) < 0 ||  // the barrier's flag
+        cudaFuncSetAttribute((const void *)k_march_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, (const void *)k_march_f64, kMarchThreads, size_t(optin)) !=
+            cudaSuccess ||
+        a < 1)
+      optin = 0;
+    (void)cudaGetLastError();
+    ctx->march_smem = optin;
+  }
+  return smem <= size_t(ctx->march_smem);
+}
+
 // FP64 relaxation over the wavefront schedule w, in cooperative launches of
 // at most kParamJobs jobs and kWaveScratch bytes of scratch (the tagged copy
 // and the (lhs, rhs) pairs of a launch's jobs, used by the launches in turn;
@@ -2486,7 +2737,13 @@ static int relax_bands(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, 
 // 781 x 1201 job already has points enough in a step to fill the GPU).
 constexpr size_t kWaveScratch = size_t(256) << 20;
 static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2g_job *jobs, int njobs, int nsweeps,
-                      bool profile) {
+                      bool profile, const MarchDev *march = nullptr) {
+  const int bands = (g.nmu - 4 + kMarchRows - 1) / kMarchRows;
+  const size_t march_smem = size_t(kMarchRows + 8) * g.n8 * 16;
+  // SOR: the marching sweep while every band has its own SM (four orbitals of
+  // 91 x 121, 120 bands, 467 us, wavefront 641; four of 151 x 181 would take
+  // two launches of 690, wavefront 950)
+  if (march && (njobs * bands > ctx->num_sms || !march_fits(ctx, march_smem))) march = nullptr;
   const size_t tagged = (size_t(g.next) * 16 + 255) / 256 * 256, pairs = (size_t(g.mxsize) * 16 + 255) / 256 * 256;
   const int most =
       std::max(1, std::min(std::min(njobs, kParamJobs), int(std::min(kWaveScratch / (tagged + pairs), size_t(kParamJobs)))));
@@ -2533,6 +2790,16 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
     int nj = nb, ns = nsweeps;
     GridDev gd = g;
     WaveDev wd = w;
+    if (march) {
+      MarchDev md = *march;
+      nblocks = unsigned(nb * bands);
+      void *args[] = {&gd, &md, &jt, &nj, &ns, &bar, &nblocks};
+      err = cudaLaunchCooperativeKernel((const void *)k_march_f64, dim3(nblocks), dim3(kMarchThreads), args, march_smem,
+                                        ctx->stream);
+      if (err != cudaSuccess) return cuda_status(err, "cooperative SOR launch");
+      ctx->launches += 1;
+      continue;
+    }
     void *args[] = {&gd, &wd, &jt, &nj, &ns, &bar, &nblocks};
     err = cudaLaunchCooperativeKernel(per_sm < 85.0 ? (const void *)k_wave_f64<4> : (const void *)k_wave_f64<1>,
                                       dim3(nblocks), dim3(kWaveThreads), args, smem, ctx->stream);
@@ -2560,7 +2827,7 @@ int cluster_occupancy(x2g_ctx *ctx, x2g_grid *grid, int *plain, int *pot) {
 int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, int nsweeps, int precision) {
   if (njobs <= 0) return X2G_OK;
   if (nsweeps <= 0) return set_status(X2G_ERR_ARG, "nsweeps must be positive");
-  if (precision == X2G_SOR) return relax_wave(ctx, grid->d, grid->d.sor, jobs, njobs, nsweeps, false);
+  if (precision == X2G_SOR) return relax_wave(ctx, grid->d, grid->d.sor, jobs, njobs, nsweeps, false, &grid->d.march);
   // FP64 MCSOR: the same sweep over the colour-ordered list.  The barrier
   // sweep (k_mcsor_f64, 50 phases of three dependent levels) took 7.03 ms for
   // 22 potentials of 331 x 481, 1.80 ms for 5 and 0.52 ms for one 91 x 121

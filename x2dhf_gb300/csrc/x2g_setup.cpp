@@ -158,6 +158,34 @@ std::string build_wave_schedule(const HostGrid &g, const std::vector<int> &order
   return "";
 }
 
+// SOR's points by row and side, from the wavefront schedule (whose entries are
+// sorted by level, so every row and side is in list order).
+void build_march(HostGrid &g) {
+  const int rows = g.nmu - 4, n8 = g.n8, last = g.nni + 3, middle = (g.n8 - 1) / 2 - 1;  // last column of the first half
+  std::vector<std::vector<int>> pts(size_t(rows) * 2), mask(size_t(rows) * 2);
+  auto add = [&](int ij, int col, unsigned m) {
+    const size_t k = size_t(ij / n8 - 4) * 2 + (col > middle);
+    pts[k].push_back(ij);
+    mask[k].push_back(int(m));
+  };
+  for (size_t k = 0; k < g.sor.pts.size(); ++k) {
+    const int row = g.sor.pts[k] >> 16, col = g.sor.pts[k] & 0xffff;
+    add(row * n8 + col, col, unsigned(g.sor.mask[k]));
+  }
+  for (size_t k = 0; k < g.sor.bpts.size(); ++k) {
+    const int row = g.sor.bpts[k] >> 16, col = g.sor.bpts[k] & 0xffff;
+    add(row * n8 + col, col, col == 4 ? kMarchAxisUp : col == last ? kMarchAxisDown : kMarchAxisMu);
+  }
+  g.march_pts.clear();
+  g.march_mask.clear();
+  g.march_off.assign(1, 0);
+  for (size_t k = 0; k < pts.size(); ++k) {
+    g.march_pts.insert(g.march_pts.end(), pts[k].begin(), pts[k].end());
+    g.march_mask.insert(g.march_mask.end(), mask[k].begin(), mask[k].end());
+    g.march_off.push_back(int(g.march_pts.size()));
+  }
+}
+
 }  // namespace
 
 // Chunks of one segment appended to `chunks`: the segment's points (ext
@@ -646,6 +674,7 @@ static std::string build_schedule(HostGrid &g) {
     }
   std::string msg = build_wave_schedule(g, g.order, offs, g.sor);
   if (!msg.empty()) return msg;
+  build_march(g);
   std::vector<int> by_colour;
   by_colour.reserve(g.order.size());
   for (int c = 0; c < 5; ++c)
@@ -700,6 +729,9 @@ void copy_schedule(HostGrid &to, const HostGrid &from) {
   for (int k = 0; k <= HostGrid::kBandRuns; ++k) to.st_rows[k] = from.st_rows[k];
   to.columns = from.columns;
   to.sor = from.sor;
+  to.march_pts = from.march_pts;
+  to.march_mask = from.march_mask;
+  to.march_off = from.march_off;
   to.mcsor = from.mcsor;
 }
 constexpr size_t kScheduleCacheEntries = 8;
