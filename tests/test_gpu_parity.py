@@ -833,3 +833,36 @@ def test_fixed_point_residual_matches_fma_residual(ctx, nnu, nmu, field):
             assert torch.isfinite(y).all()
             assert bool(((x - y).abs() <= bound).all()), (on_chip, k, float(((x - y).abs() / (bound + 1e-300)).max()))
     g.close()
+
+
+@pytest.mark.parametrize("rhs_scale,lhs_scale", [(0.0, 1.0), (1e-290, 1.0), (1e250, 1.0), (1.0, 1e-160), (1.0, 1e160),
+                                                 (1e-158, 1e-122), (1e143, 1e120)])
+@pytest.mark.parametrize("njobs", [1, 5])
+def test_sor_quotients_over_the_exponent_range(ctx, rhs_scale, lhs_scale, njobs):
+    """The marching SOR sweep takes its quotients from stored reciprocals
+    where numerator and lhs are of moderate size and divides otherwise: bit
+    for bit the oracle's division on both sides of each limit, at zeros, and
+    with two (one job) and four (five jobs) rows per block."""
+    torch = pytest.importorskip("torch")
+    nnu, nmu = 91, 121
+    oc = Case(_grid_deck(nnu, nmu))
+    c, g = _grid(ctx, _grid_deck(nnu, nmu))
+    rng = np.random.default_rng(11)
+    omega, dev = oc.omega()[0], torch.device("cuda:0")
+    lhs = (oc.fock(1)[0] + oc.coeffs()[5]) * lhs_scale
+    kept, jobs, refs = [], [], []
+    for k in range(njobs):
+        u = oc.putin(1, rng.standard_normal(nnu * nmu) * rhs_scale / max(1e-300, 1e5 * lhs_scale))
+        rhs = rng.standard_normal(nnu * nmu) * rhs_scale * 10.0 ** rng.integers(-6, 7, nnu * nmu)
+        refs.append(oc.sweep(0, 1, 3, omega, u, lhs, rhs, oc.suppl(0), oc.suppl(2)))
+        kept.append([torch.tensor(x, device=dev) for x in (u, lhs, rhs)])
+        jobs.append(xg.Job(u=kept[-1][0].data_ptr(), lhs=kept[-1][1].data_ptr(), rhs=kept[-1][2].data_ptr(), omega=omega,
+                           isym=1, kind=0))
+    torch.cuda.synchronize()
+    xg.relax(ctx, g, jobs, 3, xg.SOR)
+    ctx.synchronize()
+    sl = np.s_[4:nmu + 4, 4:nnu + 4]
+    for k, (b, ref) in enumerate(zip(kept, refs)):
+        got, exp = (x.reshape(nmu + 8, nnu + 8)[sl] for x in (b[0].cpu().numpy(), ref))
+        assert np.array_equal(got, exp, equal_nan=True), k
+    g.close()

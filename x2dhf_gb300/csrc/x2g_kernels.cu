@@ -597,6 +597,26 @@ __device__ __forceinline__ int fifth_reader(const GridDev &g, unsigned mask, int
   return (mask & 0x20000u) ? ij - 5 : (mask & 0x40000u) ? ij + 5 : 0;
 }
 
+// a / b, rounded to nearest, from 1 / b = inv.x + inv.y to 106 bits: the
+// quotient from both parts is one of the two doubles around a / b, its
+// remainder is exact, and one correction by the rounded reciprocal gives the
+// rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990, theorem on the final
+// step): four operations in place of about ten.  inv.x = 0, and an a near an
+// end of the exponent range (or zero): the quotient itself.
+__device__ __forceinline__ double quotient(double a, double b, double2 inv) {
+  const int ex = (__double2hiint(a) >> 20) & 0x7ff;
+  if (unsigned(ex - 500) > 1000u || inv.x == 0.0) return D(a, b);
+  const double q = fma(a, inv.x, a * inv.y);
+  return fma(fma(-b, q, a), inv.x, q);
+}
+// 1 / b for quotient; 0 where b is not of moderate size
+__device__ __forceinline__ double2 inverse(double b) {
+  const int ex = (__double2hiint(b) >> 20) & 0x7ff;
+  if (unsigned(ex - 623) > 800u) return make_double2(0.0, 0.0);
+  const double r = D(1.0, b);
+  return make_double2(r, fma(-b, r, 1.0) * r);
+}
+
 // (lhs, rhs), b(mu) and d(nu) of an interior point
 struct WaveCoef {
   double2 lr;
@@ -726,7 +746,8 @@ __device__ __forceinline__ bool wave_points1(const GridDev &g, const JobTable &j
 // Threads id of nt: the tagged copy of every function, its ghost cells
 // refreshed as putin does (in u too), and the (lhs, rhs) pairs: a potential's
 // lhs = f3 + idel^2 e and rhs = psa psb g with the roundings of
-// relaxPots.F90:81-95.
+// relaxPots.F90:81-95.  kInverse: 1 / lhs after each pair.
+template <bool kInverse>
 __device__ __forceinline__ void wave_prologue(const GridDev &g, const JobTable &jobs, int njobs, int id, int nt) {
   for (int jb = 0; jb < njobs; ++jb) {
     const JobDev &J = jobs.j[jb];
@@ -757,7 +778,12 @@ __device__ __forceinline__ void wave_prologue(const GridDev &g, const JobTable &
       } else {
         lr = make_double2(J.lhs[k], J.rhs[k]);
       }
-      pairs[k] = lr;
+      if (kInverse) {
+        pairs[2 * k] = lr;
+        pairs[2 * k + 1] = inverse(lr.x);
+      } else {
+        pairs[k] = lr;
+      }
     }
   }
 }
@@ -769,7 +795,7 @@ __global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev
   const int nt = int(gridDim.x * blockDim.x), id = int(blockIdx.x * blockDim.x + threadIdx.x);
   for (int k = threadIdx.x; k <= w.nlev; k += blockDim.x) s_off[k] = w.off[k];
   for (int k = threadIdx.x; k <= w.nblev; k += blockDim.x) s_off[w.nlev + 1 + k] = w.boff[k];
-  wave_prologue(g, jobs, njobs, id, nt);
+  wave_prologue<false>(g, jobs, njobs, id, nt);
   if (!grid_barrier(bar, nblocks)) return;
   WaveWalk<kSplit> walk;
   walk.off = s_off;
@@ -809,28 +835,34 @@ __global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev
 
 // ----------------------------------------------------------------------
 // List-order SOR of a few functions: the same dataflow on values in shared
-// memory.  A block owns four rows of one job (the mu=1 row included) for the
+// memory.  A block owns kRows rows of one job (the mu=1 row included) for the
 // whole launch and keeps them, with four rows on each side, as (value, tag)
-// words in shared memory; warp s of its kMarchSweeps takes sweeps s, s +
-// kMarchSweeps, ..., four lanes for each of its eight runners: a row's columns
-// from the middle to one side, in list order, then the axis.  A runner goes on
+// words in shared memory.  A runner, four lanes, follows a row's columns in one
+// sweep from the middle to one side, in list order, then the axis; it goes on
 // as soon as its point's values are there, so the rows of a warp settle one
-// column apart.  The other warps fetch the neighbours' rows, a lane per row,
-// side and sweep, from the tagged copy in global memory.  A value of a row
-// outside the block's own is overwritten there only after its readers in this
-// block are through (see above), so the copies need no further order.
+// column apart.  A warp's eight runners are two sides of four rows in one sweep
+// or of two rows in two, and take every kMarchSweeps-th sweep.  The other warps
+// fetch the neighbours' rows, a lane per row, side and sweep, from the tagged
+// copy in global memory.  A value of a row outside the block's own is
+// overwritten there only after its readers in this block are through (see
+// above), so the copies need no further order.
 //
-// What bounds it: the FP64 chain of a point (2240 cycles of the 4000 that a
-// step of one sweep takes) while a block has few runners at work, and the SM's
-// FP64 pipe when all of them are (ten warps of 24 operations a point, 19 cycles
-// each).  The way of a value through L2, most of a step's 5800 cycles when
-// every value takes it, is paid once per four rows.  SOR, 10 sweeps of one
-// orbital, wavefront / this: 331 x 481 2.26 / 1.52 ms, 151 x 181 0.93 / 0.68
-// ms, 91 x 121 0.62 / 0.46 ms.
+// What bounds it: the FP64 chain of a point (2050 cycles) and one round of loads
+// while a block has few runners at work; more than four warps share an SM's
+// FP64 pipe (23 operations a point and warp of 19 cycles each), hence two rows
+// per block, half the warps on an SM, while there are SMs enough for that.  The
+// way of a value through L2, most of a step's 5800 cycles when every value
+// takes it, is paid once per block of rows.  All nine or ten values of a point
+// are loaded at once (one after the other, as each is found, took 1550 cycles).
+// SOR, 10 sweeps of one orbital, wavefront / this: 331 x 481 2.26 / 1.29 ms
+// (four rows), 151 x 181 0.93 / 0.48, 91 x 121 0.62 / 0.37 (two rows; four rows
+// 0.63 and 0.40).
 // ----------------------------------------------------------------------
-constexpr int kMarchRows = 4, kMarchSweeps = 10;
+constexpr int kMarchSweeps = 10;
 constexpr int kMarchFetch = (8 * 2 * kMarchSweeps + 31) / 32;  // warps that fetch
-constexpr int kMarchThreads = 32 * (kMarchSweeps + kMarchFetch);
+// threads of a block of kRows rows (4 or 2: a warp's eight runners are then
+// those of 4 / kRows sweeps)
+__host__ __device__ constexpr int march_threads(int rows) { return 32 * (kMarchSweeps * rows / 4 + kMarchFetch); }
 
 __device__ __forceinline__ Tagged ld_near(unsigned at) {
   unsigned long long lo, hi;
@@ -843,32 +875,34 @@ __device__ __forceinline__ void st_near(unsigned at, double v, int tag) {
                : "memory");
 }
 
-__global__ void __launch_bounds__(kMarchThreads, 1)
+template <int kRows>
+__global__ void __launch_bounds__(march_threads(kRows), 1)
     k_march_f64(GridDev g, MarchDev w, const __grid_constant__ JobTable jobs, int njobs, int nsweeps, BarrierDev bar,
                 unsigned nblocks) {
   extern __shared__ __align__(16) ulonglong2 near[];
+  constexpr int kThr = march_threads(kRows), kPer = 4 / kRows, kWarps = kMarchSweeps / kPer;
   const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
-  wave_prologue(g, jobs, njobs, int(blockIdx.x) * kMarchThreads + tid, int(gridDim.x) * kMarchThreads);
+  wave_prologue<true>(g, jobs, njobs, int(blockIdx.x) * kThr + tid, int(gridDim.x) * kThr);
   if (!grid_barrier(bar, nblocks)) return;
   const int bands = int(gridDim.x) / njobs, jb = int(blockIdx.x) / bands;
   const JobDev &J = jobs.j[jb];
   const int n8 = g.n8, nmu = g.nmu;
-  const int r0 = 4 + (int(blockIdx.x) - jb * bands) * kMarchRows;
+  const int r0 = 4 + (int(blockIdx.x) - jb * bands) * kRows;
   const unsigned base = unsigned(__cvta_generic_to_shared(near));
-  // shared address of ext index ij: rows r0 - 4 .. r0 + 7
+  // shared address of ext index ij: rows r0 - 4 .. r0 + kRows + 3
   const int first = (r0 - 4) * n8;
   auto addr = [&](int ij) { return base + unsigned(ij - first) * 16u; };
-  for (int k = tid; k < (kMarchRows + 8) * n8; k += kMarchThreads) {
+  for (int k = tid; k < (kRows + 8) * n8; k += kThr) {
     const int ij = min(first + k, g.next - 1);
     const Tagged x = ld_tagged(J.tagged + ij);
     st_near(base + unsigned(k) * 16u, x.v, x.tag);
   }
   __syncthreads();
   WaveWait ww;
-  if (warp >= kMarchSweeps) {
-    // fetch: rows r0 - 4 .. r0 - 1 and r0 + 4 .. r0 + 7
-    const int id = tid - 32 * kMarchSweeps, h = id & 7, half = id >> 3 & 1, slot = id >> 4;
-    const int row = h < 4 ? r0 - 4 + h : r0 + kMarchRows + h - 4;
+  if (warp >= kWarps) {
+    // fetch: the four rows on each side
+    const int id = tid - 32 * kWarps, h = id & 7, half = id >> 3 & 1, slot = id >> 4;
+    const int row = h < 4 ? r0 - 4 + h : r0 + kRows + h - 4;
     bool on = slot < kMarchSweeps && row >= 4 && row < nmu;
     int s = slot, k = 0, n = 0, o = 0;
     if (on) {
@@ -897,7 +931,7 @@ __global__ void __launch_bounds__(kMarchThreads, 1)
     }
     return;
   }
-  const int role = lane & 3, row = r0 + (lane >> 3), half = lane >> 2 & 1;
+  const int role = lane & 3, half = lane >> 2 & 1, row = r0 + (lane >> 3) % kRows;
   double cf[4];
   {
     const double *c = role == 0 ? g.dmu2 : role == 1 ? g.dmu1 : role == 2 ? g.dni2 : g.dni1;
@@ -912,88 +946,71 @@ __global__ void __launch_bounds__(kMarchThreads, 1)
     o = w.off[(row - 4) * 2 + half];
     n = w.off[(row - 4) * 2 + half + 1] - o;
   }
-  const double2 *pairs = reinterpret_cast<const double2 *>(J.pairs) - 4 * g.nni - 4;  // by ext row * nni + ext col
-  for (int s = warp; s < nsweeps; s += kMarchSweeps) {
+  const double2 *pairs = reinterpret_cast<const double2 *>(J.pairs) - 2 * (4 * g.nni + 4);  // by ext row * nni + ext col
+  for (int s = warp * kPer + (lane >> 3) / kRows; __any_sync(0xffffffffu, s < nsweeps); s += kMarchSweeps) {
     int k = 0;
-    bool on = n > 0;
-    int2 cur = on ? __ldg(w.pts + o) : make_int2(0, 0), nxt = cur;
-    if (n > 1) nxt = __ldg(w.pts + o + 1);
-    auto coef = [&](const int2 &e, double2 &lr, double &d) {
+    bool on = n > 0 && s < nsweeps;
+    // (a runner without a row looks at a point of the first one)
+    int2 cur = on ? __ldg(w.pts + o) : make_int2(r0 * n8 + 8, 0), nxt = cur, nxt2 = cur;
+    if (n > 1) nxt = __ldg(w.pts + o + 1);  // entries three ahead, coefficients one
+    if (n > 2) nxt2 = __ldg(w.pts + o + 2);
+    auto coef = [&](const int2 &e, double2 &lr, double2 &inv, double &d) {
       if (on && !(unsigned(e.y) & kMarchAxis)) {
         const int col = e.x - row * n8;
-        lr = __ldcg(pairs + row * g.nni + col);
+        lr = __ldcg(pairs + 2 * (row * g.nni + col));
+        inv = __ldcg(pairs + 2 * (row * g.nni + col) + 1);
         d = __ldg(g.d_nu + col - 4);
       }
     };
-    double2 lr = make_double2(1.0, 0.0), lr_n = lr;
+    double2 lr = make_double2(1.0, 0.0), lr_n = lr, inv = make_double2(1.0, 0.0), inv_n = inv;
     double dnu = 0.0, dnu_n = 0.0;
-    coef(cur, lr, dnu);
-    double m[4], p[4], uc = 0.0;
-    unsigned miss = 0;
+    coef(cur, lr, inv, dnu);
     bool fresh = true;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) m[q] = p[q] = 0.0;
     while (__any_sync(0xffffffffu, on)) {
       const int ij = cur.x;
       const unsigned mask = unsigned(cur.y), at = addr(ij);
       const bool axis = (mask & kMarchAxis) != 0;
-      const int ast = axis ? ((mask & kMarchAxisMu) ? n8 : (mask & kMarchAxisUp) ? 1 : -1) : 0;
-      int other = 0;  // a value that is read by this point's value and does not read it back
       if (fresh) {
-        coef(nxt, lr_n, dnu_n);
-        miss = !on ? 0u : axis ? (role == 0 ? 0x21fu : 0u) : 0x3ffu;
+        coef(nxt, lr_n, inv_n, dnu_n);
         fresh = false;
       }
+      // a point's neighbours and its old value, or the five values of an
+      // extrapolation; other: a value that is read by this point's and does
+      // not read it back
+      const int ast = (mask & kMarchAxisMu) ? n8 : (mask & kMarchAxisUp) ? 1 : -1;
+      int other = ij;
       if (axis) {
         if ((mask & kMarchAxisMu) && ij - row * n8 <= 9) other = row * n8 + 4;
         else if ((mask & kMarchAxisMu) && ij - row * n8 >= g.nni - 2) other = row * n8 + g.nni + 3;
       } else if (role != 1) {
-        other = fifth_reader(g, mask, ij, role == 0 ? 0 : 1);
+        const int f = fifth_reader(g, mask, ij, role == 0 ? 0 : 1);
+        other = f ? f : ij;
       }
-      if (!other) miss &= ~0x200u;
-      if (axis) {
+      Tagged x[4], y[4];
 #pragma unroll
-        for (int q = 0; q < 5; ++q)
-          if (miss & (1u << q)) {
-            const Tagged x = ld_near(at + unsigned((q + 1) * ast * 16));
-            if (x.tag > s) {
-              if (q < 4) m[q] = x.v;
-              else uc = x.v;
-              miss &= ~(1u << q);
-            }
-          }
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int e = 4 * (3 - q) + bit;
-          if (miss & (1u << q)) {
-            const Tagged x = ld_near(at - unsigned((4 - q) * st * 16));
-            if (x.tag >= s + int((mask >> e) & 1u)) {
-              m[q] = x.v;
-              miss &= ~(1u << q);
-            }
-          }
-          if (miss & (16u << q)) {
-            const Tagged y = ld_near(at + unsigned((4 - q) * st * 16));
-            if (y.tag >= s + int((mask >> (e + 1)) & 1u)) {
-              p[q] = y.v;
-              miss &= ~(16u << q);
-            }
-          }
-        }
-        if (miss & 256u) {
-          const Tagged c = ld_near(at);
-          if (c.tag >= s) {
-            uc = c.v;
-            miss &= ~256u;
-          }
-        }
+      for (int q = 0; q < 4; ++q) {
+        x[q] = ld_near(axis ? at + unsigned((q + 1) * ast * 16) : at - unsigned((4 - q) * st * 16));
+        y[q] = ld_near(axis ? at : at + unsigned((4 - q) * st * 16));
       }
-      if ((miss & 512u) && ld_near(addr(other)).tag >= s) miss &= ~512u;
-      const unsigned waits = __ballot_sync(0xffffffffu, miss != 0);
+      const Tagged c = ld_near(axis ? at + unsigned(5 * ast * 16) : at), z = ld_near(addr(other));
+      bool ok = z.tag >= s;
+      double m[4], p[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int e = 4 * (3 - q) + bit;
+        m[q] = x[q].v;
+        p[q] = y[q].v;
+        ok = ok && x[q].tag >= s + (axis ? 1 : int(mask >> e & 1u));
+        ok = ok && (axis || y[q].tag >= s + int(mask >> (e + 1) & 1u));
+      }
+      const double uc = c.v;
+      ok = ok && c.tag >= s + (axis ? 1 : 0);
+      if (axis && role != 0) ok = true;
+      const unsigned waits = __ballot_sync(0xffffffffu, !ok);
       const bool ready = on && (waits >> (lane & 28) & 0xfu) == 0;
       if (!__any_sync(0xffffffffu, ready)) {
         if (!__all_sync(0xffffffffu, ww.again(bar))) return;
+        if (ww.spins > 4) __nanosleep(ww.spins > 16 ? 200 : 40);
         continue;
       }
       ww = WaveWait();
@@ -1010,7 +1027,10 @@ __global__ void __launch_bounds__(kMarchThreads, 1)
         const double ddmi2 = __shfl_sync(0xffffffffu, t, b), bddmi1 = __shfl_sync(0xffffffffu, t, b + 1);
         const double ddni2 = __shfl_sync(0xffffffffu, t, b + 2), dddni1 = __shfl_sync(0xffffffffu, t, b + 3);
         const double cc = A(A(A(ddmi2, bddmi1), ddni2), dddni1);
-        v = A(D(M(omega, S(lr.y, cc)), lr.x), M(omega1, uc));
+        // omega (rhs - cc) and omega1 times the old value, on two lanes at once
+        const double o = M(role == 1 ? omega1 : omega, role == 1 ? uc : S(lr.y, cc));
+        const double old = __shfl_sync(0xffffffffu, o, b + 1);
+        v = A(quotient(o, lr.x, inv), old);  // (of role 0)
       }
       if (ready && axis && role == 0) {
         v = 0.0;
@@ -1025,10 +1045,12 @@ __global__ void __launch_bounds__(kMarchThreads, 1)
         }
         cur = nxt;
         lr = lr_n;
+        inv = inv_n;
         dnu = dnu_n;
         fresh = true;
         on = ++k < n;
-        if (k + 1 < n) nxt = __ldg(w.pts + o + k + 1);
+        nxt = nxt2;
+        if (k + 2 < n) nxt2 = __ldg(w.pts + o + k + 2);
       }
       __syncwarp();
     }
@@ -2712,20 +2734,21 @@ static int relax_bands(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, 
   return X2G_OK;
 }
 
-// whether a block of the marching SOR sweep can be resident with this much
+// whether blocks of the marching SOR sweep can be resident with this much
 // shared memory (its cap is set to the device's opt-in maximum, once)
 static bool march_fits(x2g_ctx *ctx, size_t smem) {
   if (ctx->march_smem < 0) {
-    int optin = 0, a = 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess ||
-        (optin -= 1024) < 0 ||  // the barrier's flag
-        cudaFuncSetAttribute((const void *)k_march_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, (const void *)k_march_f64, kMarchThreads, size_t(optin)) !=
-            cudaSuccess ||
-        a < 1)
-      optin = 0;
+    int optin = 0;
+    bool ok = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
+              (optin -= 1024) > 0;  // the barrier's flag
+    auto fits = [&](const void *fn, int threads) {
+      int a = 0;
+      return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) == cudaSuccess &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fn, threads, size_t(optin)) == cudaSuccess && a >= 1;
+    };
+    ok = ok && fits((const void *)k_march_f64<2>, march_threads(2)) && fits((const void *)k_march_f64<4>, march_threads(4));
     (void)cudaGetLastError();
-    ctx->march_smem = optin;
+    ctx->march_smem = ok ? optin : 0;
   }
   return smem <= size_t(ctx->march_smem);
 }
@@ -2738,13 +2761,15 @@ static bool march_fits(x2g_ctx *ctx, size_t smem) {
 constexpr size_t kWaveScratch = size_t(256) << 20;
 static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2g_job *jobs, int njobs, int nsweeps,
                       bool profile, const MarchDev *march = nullptr) {
-  const int bands = (g.nmu - 4 + kMarchRows - 1) / kMarchRows;
-  const size_t march_smem = size_t(kMarchRows + 8) * g.n8 * 16;
-  // SOR: the marching sweep while every band has its own SM (four orbitals of
-  // 91 x 121, 120 bands, 467 us, wavefront 641; four of 151 x 181 would take
-  // two launches of 690, wavefront 950)
-  if (march && (njobs * bands > ctx->num_sms || !march_fits(ctx, march_smem))) march = nullptr;
-  const size_t tagged = (size_t(g.next) * 16 + 255) / 256 * 256, pairs = (size_t(g.mxsize) * 16 + 255) / 256 * 256;
+  // SOR: the marching sweep while every block of rows has its own SM (four
+  // orbitals of 91 x 121, 120 blocks of four rows, 373 us, wavefront 641; two
+  // and three of 151 x 181 578 and 585; four would take two launches, wavefront
+  // 950)
+  int rows = 0;
+  for (int r = 4; r >= 2 && march; r /= 2)
+    if (njobs * ((g.nmu - 4 + r - 1) / r) <= ctx->num_sms && march_fits(ctx, size_t(r + 8) * g.n8 * 16)) rows = r;
+  if (!rows) march = nullptr;
+  const size_t tagged = (size_t(g.next) * 16 + 255) / 256 * 256, pairs = (size_t(g.mxsize) * (march ? 32 : 16) + 255) / 256 * 256;
   const int most =
       std::max(1, std::min(std::min(njobs, kParamJobs), int(std::min(kWaveScratch / (tagged + pairs), size_t(kParamJobs)))));
   char *scratch = static_cast<char *>(ctx_workspace(ctx, (tagged + pairs) * size_t(most)));
@@ -2792,10 +2817,11 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
     WaveDev wd = w;
     if (march) {
       MarchDev md = *march;
-      nblocks = unsigned(nb * bands);
+      nblocks = unsigned(nb * ((g.nmu - 4 + rows - 1) / rows));
       void *args[] = {&gd, &md, &jt, &nj, &ns, &bar, &nblocks};
-      err = cudaLaunchCooperativeKernel((const void *)k_march_f64, dim3(nblocks), dim3(kMarchThreads), args, march_smem,
-                                        ctx->stream);
+      err = cudaLaunchCooperativeKernel(rows == 2 ? (const void *)k_march_f64<2> : (const void *)k_march_f64<4>,
+                                        dim3(nblocks), dim3(unsigned(march_threads(rows))), args,
+                                        size_t(rows + 8) * g.n8 * 16, ctx->stream);
       if (err != cudaSuccess) return cuda_status(err, "cooperative SOR launch");
       ctx->launches += 1;
       continue;
