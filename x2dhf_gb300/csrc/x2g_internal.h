@@ -259,6 +259,8 @@ struct x2g_ctx {
   // reusable device workspace
   void *work = nullptr;
   size_t work_bytes = 0;
+  void *host_arrays = nullptr;  // device copies of a host call's arrays
+  size_t host_arrays_bytes = 0;
   void *red = nullptr;  // reduction partials
   size_t red_bytes = 0;
   double *host_red = nullptr;  // pinned host buffer for small readbacks
