@@ -28,13 +28,14 @@
 // counted on the receiver's barrier: a cluster barrier per phase took 440
 // cycles, 665 with plain stores into the neighbours' memory to drain.
 //
-// What bounds it: instruction issue, about 85 instructions per slot of 32
-// points at 0.45 per cycle and SM quarter (17 loads and stores, 20 packed
-// operations of two roundings each), and a fifth of a phase at its barrier;
-// where a launch is small, the latency of a phase (0.9 us at three slots).
-// Against the sweep with a list of points per warp and a cluster barrier per
-// colour and level (10 sweeps, us): one orbital of 151 x 241 58 (106), of 331 x
-// 481 97 (132), six 101 (132), 22 potentials of 331 x 481 210 (two waves, 382).
+// What bounds it: instruction issue (per slot of 32 points 17 loads and stores
+// and 20 packed operations of two roundings each, 12 for potentials), at 0.45
+// per cycle and SM quarter, and a fifth of a phase at its barrier; where a launch
+// is small, the latency of a phase (0.9 us at three slots).  Against the sweep
+// with a list of points per warp and a cluster barrier per colour and level (10
+// sweeps, us): one orbital of 151 x 241 58 (106), of 331 x 481 97 (132), six 101
+// (132), 22 potentials of 331 x 481 173 (two waves, 382; 210 with relax_f32's
+// order of operations).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -114,6 +115,8 @@ __device__ __forceinline__ bool wait_halo(unsigned bar, unsigned parity) {
 }
 
 struct ColThread {
+  float wl[4], wr[4];  // kSep: nu weights of the neighbours at distance 4, 3, 2, 1
+  float cs;            // kSep: the seam partner's weight
   float d, lq, omega, omega1;
   int lane, src;        // this lane and the column seam's partner lane (itself: no partner)
   int warp, seam_warp;  // equal: this warp holds the column seam
@@ -146,6 +149,12 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
   return d;
 }
 
+__device__ __forceinline__ float rcp_fast(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // the new value of a point with residual r from its column's rows v[0..8]
 // (-4..4), its row's columns h[0..3] (-4..-1) and h[4..7] (1..4), b of its row
 // and t: omega / lhs, or the lhs row term (kSep); the operations and roundings
@@ -153,6 +162,28 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
 template <bool kSep>
 __device__ __forceinline__ float col_value(const ColPlan &p, const ColThread &T, const float *v, const float *h, float b,
                                            float t, float r) {
+  if (kSep) {
+    // a neighbour and its mirror image, weighted by dmu2 +- b dmu1 along mu
+    // and by dni2 +- d dni1 (fixed for the column) along nu, in one instruction
+    const unsigned long long *m1 = reinterpret_cast<const unsigned long long *>(p.m1);
+    const unsigned long long *m2 = reinterpret_cast<const unsigned long long *>(p.m2);
+    unsigned long long cc = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned long long wm = fma2(pack2(b, b), m1[q], m2[q]);
+      cc = q == 0 ? mul2(wm, pack2(v[q], v[8 - q])) : fma2(wm, pack2(v[q], v[8 - q]), cc);
+      cc = fma2(pack2(T.wl[q], T.wr[q]), pack2(h[q], h[7 - q]), cc);
+    }
+    const float2 sum = unpack2(cc);
+    const float w = T.omega * rcp_fast(t - T.lq);
+    float out = __fmaf_rn(T.omega1, v[4], w * (r - (sum.x + sum.y)));
+    if (T.warp == T.seam_warp) {
+      // the partner column's change since the old value used above, weighted
+      // (0 without a partner)
+      out = __fmaf_rn(-w * T.cs, __shfl_sync(0xffffffffu, out - v[4], T.src), out);
+    }
+    return out;
+  }
   const unsigned long long *c2 = reinterpret_cast<const unsigned long long *>(p.c2);
   const unsigned long long *c1 = reinterpret_cast<const unsigned long long *>(p.c1);
   unsigned long long s2 = 0, s1 = 0;
@@ -164,7 +195,7 @@ __device__ __forceinline__ float col_value(const ColPlan &p, const ColThread &T,
     s1 = q == 0 ? mul2(c1[q], dif) : fma2(c1[q], dif, s1);
   }
   const float2 d2 = unpack2(s2), d1 = unpack2(s1);
-  const float w = kSep ? __fdividef(T.omega, t - T.lq) : t;
+  const float w = t;
   const float mu = __fmaf_rn(b, d1.x, d2.x);
   float out = __fmaf_rn(T.omega1, v[4], w * (r - __fmaf_rn(T.d, d1.y, mu + d2.y)));
   if (T.warp == T.seam_warp) {
@@ -305,10 +336,18 @@ __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
   T.omega1 = J.omega1f;
   T.d = in ? g.d_nu32[nu] : 0.0f;
   T.lq = (kSep && in) ? narrow_f64(J.idel2 * g.e_nu[nu]) : 0.0f;
+  if (kSep) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      T.wl[q] = __fmaf_rn(T.d, g.dni1f[q], g.dni2f[q]);
+      T.wr[q] = __fmaf_rn(-T.d, g.dni1f[q], g.dni2f[q]);
+    }
+  }
   // column seam: 1-based columns nnix + 2 and nnix + 3 read the new values of
   // nnix and nnix - 1, two and four columns to their left
   T.lane = lane;
   T.src = lane - (free ? 0 : (col == nnix + 1) ? 2 : (col == nnix + 2) ? 4 : 0);
+  if (kSep) T.cs = T.src == lane ? 0.0f : T.src + 2 == lane ? T.wl[2] : T.wl[0];
   T.warp = warp;
   T.seam_warp = free ? -1 : (nnix - 7 + p.shift) / 32 + group * p.warps;
   // arm both parities of a side for the values of the first two phases

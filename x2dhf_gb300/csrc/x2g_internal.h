@@ -60,9 +60,10 @@ constexpr int kMaxCluster = 16;
 struct ColPlan {
   int size, groups, maxrows, slots, pitch, warps, shift;
   // set for the launch: the rows the kernel's arrays hold, the FP32 stencil
-  // weights as (mu, nu) pairs, (-1, -1)
+  // weights as (mu, nu) pairs, (-1, -1), and those along mu as (dmu1, -dmu1)
+  // and (dmu2, dmu2)
   int rows;
-  float2 c2[4], c1[4], neg;
+  float2 c2[4], c1[4], neg, m1[4], m2[4];
   int row0[kMaxCluster + 1], cut[kMaxCluster];
 };
 

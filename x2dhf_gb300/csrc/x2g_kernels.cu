@@ -2640,6 +2640,8 @@ static int cluster_sweep(x2g_ctx *ctx, const GridDev &g, const ColChoice &c, Job
   for (int k = 0; k < 4; ++k) {
     plan.c2[k] = make_float2(g.dmu2f[k], g.dni2f[k]);
     plan.c1[k] = make_float2(g.dmu1f[k], g.dni1f[k]);
+    plan.m1[k] = make_float2(g.dmu1f[k], -g.dmu1f[k]);
+    plan.m2[k] = make_float2(g.dmu2f[k], g.dmu2f[k]);
   }
   plan.neg = make_float2(-1.0f, -1.0f);
   int *err_word = reinterpret_cast<int *>(ctx->bar + 2);
@@ -2863,9 +2865,9 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
   const GridDev &g = grid->d;
   // potentials built from orbitals have a separable lhs: batches of them
   // beyond the plain kernel's clusters take the kernel that forms omega / lhs
-  // itself (22 of 331x481: 210 us, the plain kernel's two waves of 13 and 9
-  // 233; 64 of 151x241 214 and 284); below that both take the same time, and
-  // the plain kernel's results are the persistent-band sweep's bit for bit
+  // itself (22 of 331x481: 173 us, the plain kernel's two waves of 13 and 9
+  // 233; 64 of 151x241 191 and 284); below that the plain kernel's results are
+  // the persistent-band sweep's bit for bit
   bool separable = true;
   for (int i = 0; i < njobs && separable; ++i) separable = (jobs[i].kind == 1 && !(jobs[i].lhs && jobs[i].rhs));
   ColChoice col = choose_columns(ctx, grid->h, njobs, false);
