@@ -866,3 +866,49 @@ def test_sor_quotients_over_the_exponent_range(ctx, rhs_scale, lhs_scale, njobs)
         got, exp = (x.reshape(nmu + 8, nnu + 8)[sl] for x in (b[0].cpu().numpy(), ref))
         assert np.array_equal(got, exp, equal_nan=True), k
     g.close()
+
+
+@pytest.mark.parametrize("form,nnu,nmu,njobs", [("fp64", 151, 241, 24), ("sor", 61, 61, 80)])
+@pytest.mark.parametrize("values", ["random", "equal", "ends", "specials"])
+def test_wide_wavefront_bitexact(ctx, form, nnu, nmu, njobs, values):
+    """Wide steps form part of the stencil's products on the integer pipes:
+    bit for bit the oracle's FP64 results for values of every magnitude, pairs
+    that cancel or differ in the last bits, zeros of both signs, values at the
+    ends of the exponent range, infinities and NaNs.  (SOR's steps are never
+    that wide: its one-lane form, on the same values.)"""
+    torch = pytest.importorskip("torch")
+    oc = Case(_grid_deck(nnu, nmu))
+    c, g = _grid(ctx, _grid_deck(nnu, nmu))
+    rng = np.random.default_rng(5)
+    omega, dev, n = oc.omega()[0], torch.device("cuda:0"), nnu * nmu
+    lhs = oc.fock(1)[0] + oc.coeffs()[5]
+    kept, jobs, refs = [], [], []
+    for k in range(4):
+        if values == "random":
+            v = rng.standard_normal(n) * 10.0 ** rng.integers(-30, 31, n)
+        elif values == "equal":
+            v = rng.choice([-1.0, 1.0], n) * (1.0 + rng.integers(-3, 4, n) * 2.0 ** -52) * rng.choice([0.0, 1.0], n)
+        elif values == "ends":
+            v = rng.standard_normal(n) * 10.0 ** rng.choice([-308, -300, -225, -215, 0, 150, 190, 200, 210], n)
+        else:
+            v = rng.standard_normal(n)
+            v[rng.integers(0, n, 3)] = np.inf
+            v[rng.integers(0, n, 3)] = np.nan
+            v[rng.integers(0, n, n // 4)] = -0.0
+        u = oc.putin(1 if k % 2 == 0 else -1, v)
+        rhs = rng.standard_normal(n)
+        refs.append(oc.sweep(0 if form == "sor" else 1, 1 if k % 2 == 0 else -1, 2, omega, u, lhs, rhs, oc.suppl(0),
+                             oc.suppl(2)))
+        kept.append([u, torch.tensor(lhs, device=dev), torch.tensor(rhs, device=dev)])
+    us = [torch.tensor(kept[k % 4][0], device=dev) for k in range(njobs)]
+    for k, u in enumerate(us):
+        jobs.append(xg.Job(u=u.data_ptr(), lhs=kept[k % 4][1].data_ptr(), rhs=kept[k % 4][2].data_ptr(), omega=omega,
+                           isym=1 if k % 2 == 0 else -1, kind=0))
+    torch.cuda.synchronize()
+    xg.relax(ctx, g, jobs, 2, xg.SOR if form == "sor" else xg.FP64)
+    ctx.synchronize()
+    sl = np.s_[4:nmu + 4, 4:nnu + 4]
+    for k, u in enumerate(us):
+        got, exp = (x.reshape(nmu + 8, nnu + 8)[sl] for x in (u.cpu().numpy(), refs[k % 4]))
+        assert np.array_equal(got, exp, equal_nan=True), k
+    g.close()

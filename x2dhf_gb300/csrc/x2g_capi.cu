@@ -319,6 +319,9 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
   std::memcpy(d.dni2, h.dni2, sizeof d.dni2);
   std::memcpy(d.exeven, h.exeven, sizeof d.exeven);
   for (int k = 0; k < 4; ++k) {
+    const bool ok[4] = {pair_coef(h.dmu2[k], d.pmu2[k]), pair_coef(h.dmu1[k], d.pmu1[k]), pair_coef(h.dni2[k], d.pnu2[k]),
+                        pair_coef(h.dni1[k], d.pnu1[k])};
+    d.pairs = (k == 0 || d.pairs) && ok[0] && ok[1] && ok[2] && ok[3];
     d.dmu1f[k] = float(h.dmu1[k]);
     d.dmu2f[k] = float(h.dmu2[k]);
     d.dni1f[k] = float(h.dni1[k]);

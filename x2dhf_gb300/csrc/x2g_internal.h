@@ -9,6 +9,8 @@
 
 #include "../../include/x2dhf_gpu.h"
 
+#include "x2g_pairs.cuh"
+
 namespace x2g {
 
 constexpr double kPrecis = 2.220446049250313080847263336181640625e-16;  // epsilon(1d0), initVariables.F90:397
@@ -168,6 +170,8 @@ struct GridDev {
   int nni, nmu, n8, m8, next, mxsize, ntiles, nlev, mpole;
   double r2;
   double dmu1[4], dmu2[4], dni1[4], dni2[4], exeven[5], diag;
+  PairCoef pmu2[4], pmu1[4], pnu2[4], pnu1[4];  // dmu2, dmu1, dni2, dni1 as factors of pair_products
+  bool pairs;                                   // all of them are of moderate size
   const double *borb_mu, *bpot_mu, *f3_mu, *d_nu;
   const double *e, *f0, *f1, *f2, *f4, *g, *wgt1, *wgt2, *leg;
   const double *wf;  // wgt2 f4: the weight of the orbital inner products (Gram-matrix orthonormalisation)

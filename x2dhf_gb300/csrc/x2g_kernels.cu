@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "x2g_columns.cuh"
+#include "x2g_pairs.cuh"
 
 namespace x2g {
 
@@ -618,12 +619,15 @@ __device__ __forceinline__ double2 inverse(double b) {
 }
 
 // (lhs, rhs), b(mu) and d(nu) of an interior point
+template <bool kInverse>
 struct WaveCoef {
-  double2 lr;
+  double2 lr, inv;
   double b, d;
   __device__ __forceinline__ WaveCoef(const GridDev &g, const JobDev &J, const WaveItem &it) {
     const int mu = it.row() - 4, nu = it.col() - 4;
-    lr = __ldcg(reinterpret_cast<const double2 *>(J.pairs) + mu * g.nni + nu);
+    const double2 *at = reinterpret_cast<const double2 *>(J.pairs) + (kInverse ? 2 : 1) * (mu * g.nni + nu);
+    lr = __ldcg(at);
+    inv = kInverse ? __ldcg(at + 1) : make_double2(0.0, 0.0);
     b = __ldg((J.kind >= 1 ? g.bpot_mu : g.borb_mu) + mu);
     d = __ldg(g.d_nu + nu);
   }
@@ -639,7 +643,7 @@ __device__ __forceinline__ bool wave_points4(const GridDev &g, const JobTable &j
   double m[4], p[4], uc = 0.0;
   unsigned miss = on ? 0x3ffu : 0u;  // values still to come: 8 neighbours, the centre, a fifth reader
   const int ij = it.row() * g.n8 + it.col();
-  const WaveCoef co(g, J, it);
+  const WaveCoef<false> co(g, J, it);
   const int fifth = (role == 1) ? 0 : fifth_reader(g, it.mask, ij, role == 0 ? 0 : 1);
   if (!fifth) miss &= ~0x200u;
   WaveWait ww;
@@ -696,14 +700,20 @@ __device__ __forceinline__ bool wave_points4(const GridDev &g, const JobTable &j
   return true;
 }
 
+// kWide: a step holds so many points that the FP64 pipe is the bound.  The
+// products of the sums and differences of the neighbours at distance 4 and 3
+// then go to the integer pipes (pair_products), 16 of the 53 FP64 operations
+// of a point besides its quotient, and the quotient comes from a stored
+// reciprocal.  Three or four distances there make the integer side the bound.
 // interior points, one lane each
+template <bool kWide>
 __device__ __forceinline__ bool wave_points1(const GridDev &g, const JobTable &jobs, const WaveItem &it, int nsweeps,
                                              const BarrierDev &bar) {
   const JobDev &J = jobs.j[it.jb];
   const bool on = it.s >= 0;
   double n[16], uc = 0.0;
   const int ij = it.row() * g.n8 + it.col();
-  const WaveCoef co(g, J, it);
+  const WaveCoef<kWide> co(g, J, it);
   const int f0 = fifth_reader(g, it.mask, ij, 0), f1 = fifth_reader(g, it.mask, ij, 1);
   bool got = !on;
   WaveWait ww;
@@ -728,17 +738,25 @@ __device__ __forceinline__ bool wave_points1(const GridDev &g, const JobTable &j
     if (!__all_sync(0xffffffffu, ww.again(bar))) return false;
   }
   if (on) {
-    const double ddmi2 = A(A(A(M(g.dmu2[0], A(n[14], n[15])), M(g.dmu2[1], A(n[10], n[11]))),
-                             M(g.dmu2[2], A(n[6], n[7]))), M(g.dmu2[3], A(n[2], n[3])));
-    const double ddmi1 = A(A(A(M(g.dmu1[0], S(n[14], n[15])), M(g.dmu1[1], S(n[10], n[11]))),
-                             M(g.dmu1[2], S(n[6], n[7]))), M(g.dmu1[3], S(n[2], n[3])));
-    const double ddni2 = A(A(A(M(g.dni2[0], A(n[12], n[13])), M(g.dni2[1], A(n[8], n[9]))),
-                             M(g.dni2[2], A(n[4], n[5]))), M(g.dni2[3], A(n[0], n[1])));
-    const double ddni1 = A(A(A(M(g.dni1[0], S(n[12], n[13])), M(g.dni1[1], S(n[8], n[9]))),
-                             M(g.dni1[2], S(n[4], n[5]))), M(g.dni1[3], S(n[0], n[1])));
+    double m2[4], m1[4], n2[4], n1[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const double xm = n[14 - 4 * q], ym = n[15 - 4 * q], xn = n[12 - 4 * q], yn = n[13 - 4 * q];
+      if (!kWide || q >= 2 || !pair_products(xm, ym, g.pmu2[q], g.pmu1[q], m2[q], m1[q])) {
+        m2[q] = M(g.dmu2[q], A(xm, ym));
+        m1[q] = M(g.dmu1[q], S(xm, ym));
+      }
+      if (!kWide || q >= 2 || !pair_products(xn, yn, g.pnu2[q], g.pnu1[q], n2[q], n1[q])) {
+        n2[q] = M(g.dni2[q], A(xn, yn));
+        n1[q] = M(g.dni1[q], S(xn, yn));
+      }
+    }
+    const double ddmi2 = A(A(A(m2[0], m2[1]), m2[2]), m2[3]), ddmi1 = A(A(A(m1[0], m1[1]), m1[2]), m1[3]);
+    const double ddni2 = A(A(A(n2[0], n2[1]), n2[2]), n2[3]), ddni1 = A(A(A(n1[0], n1[1]), n1[2]), n1[3]);
     const double omega = J.omega, omega1 = 1.0 - J.omega;
     const double cc = A(A(A(ddmi2, M(co.b, ddmi1)), ddni2), M(co.d, ddni1));
-    wave_store(J, ij, A(D(M(omega, S(co.lr.y, cc)), co.lr.x), M(omega1, uc)), it.s, nsweeps);
+    const double num = M(omega, S(co.lr.y, cc));
+    wave_store(J, ij, A(kWide ? quotient(num, co.lr.x, co.inv) : D(num, co.lr.x), M(omega1, uc)), it.s, nsweeps);
   }
   return true;
 }
@@ -788,14 +806,14 @@ __device__ __forceinline__ void wave_prologue(const GridDev &g, const JobTable &
   }
 }
 
-template <int kSplit>
+template <int kSplit, bool kWide>
 __global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev w, const __grid_constant__ JobTable jobs,
                                                              int njobs, int nsweeps, BarrierDev bar, unsigned nblocks) {
   extern __shared__ int s_off[];
   const int nt = int(gridDim.x * blockDim.x), id = int(blockIdx.x * blockDim.x + threadIdx.x);
   for (int k = threadIdx.x; k <= w.nlev; k += blockDim.x) s_off[k] = w.off[k];
   for (int k = threadIdx.x; k <= w.nblev; k += blockDim.x) s_off[w.nlev + 1 + k] = w.boff[k];
-  wave_prologue<false>(g, jobs, njobs, id, nt);
+  wave_prologue<kWide>(g, jobs, njobs, id, nt);
   if (!grid_barrier(bar, nblocks)) return;
   WaveWalk<kSplit> walk;
   walk.off = s_off;
@@ -827,7 +845,7 @@ __global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev
     else if (kSplit == 4)
       ok = wave_points4(g, jobs, it, nsweeps, bar, cf);
     else
-      ok = wave_points1(g, jobs, it, nsweeps, bar);
+      ok = wave_points1<kWide>(g, jobs, it, nsweeps, bar);
     if (!ok) return;
     it = nx;
   }
@@ -2771,7 +2789,7 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
   for (int r = 4; r >= 2 && march; r /= 2)
     if (njobs * ((g.nmu - 4 + r - 1) / r) <= ctx->num_sms && march_fits(ctx, size_t(r + 8) * g.n8 * 16)) rows = r;
   if (!rows) march = nullptr;
-  const size_t tagged = (size_t(g.next) * 16 + 255) / 256 * 256, pairs = (size_t(g.mxsize) * (march ? 32 : 16) + 255) / 256 * 256;
+  const size_t tagged = (size_t(g.next) * 16 + 255) / 256 * 256, pairs = (size_t(g.mxsize) * 32 + 255) / 256 * 256;
   const int most =
       std::max(1, std::min(std::min(njobs, kParamJobs), int(std::min(kWaveScratch / (tagged + pairs), size_t(kParamJobs)))));
   char *scratch = static_cast<char *>(ctx_workspace(ctx, (tagged + pairs) * size_t(most)));
@@ -2780,11 +2798,15 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
   if (smem > kWaveSmem) return set_status(X2G_ERR_ARG, "grid too large for the wavefront's level table");
   if (ctx->wave_ok < 0) {
     int a = 0, b = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, (const void *)k_wave_f64<4>, kWaveThreads, kWaveSmem);
+    int w = 0;
+    cudaError_t e =
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, (const void *)k_wave_f64<4, false>, kWaveThreads, kWaveSmem);
     if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void *)k_wave_f64<1>, kWaveThreads, kWaveSmem);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void *)k_wave_f64<1, false>, kWaveThreads, kWaveSmem);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&w, (const void *)k_wave_f64<1, true>, kWaveThreads, kWaveSmem);
     if (e != cudaSuccess) return cuda_status(e, "occupancy query");
-    ctx->wave_ok = (a >= 1 && b >= 1) ? 1 : 0;
+    ctx->wave_ok = (a >= 1 && b >= 1 && w >= 1) ? 1 : 0;
   }
   if (!ctx->wave_ok) return set_status(X2G_ERR_CUDA, "cooperative FP64 sweep cannot be resident");
   for (int b0 = 0; b0 < njobs; b0 += most) {
@@ -2802,7 +2824,10 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
     // four lanes per point while the average step is narrow: MCSOR, 10
     // sweeps, four lanes / one lane: 289 / 329 us at 58 points a step and SM
     // (151 x 241, 2 jobs), 369 / 368 us at 85 (91 x 121, 10 jobs), 507 / 389
-    // us at 145 (151 x 241, 5 jobs)
+    // us at 145 (151 x 241, 5 jobs).  One lane, FP64 pipe
+    // alone / its wide form: 785 / 842 us at 386 (331 x 481, 3 jobs), 896 / 901
+    // at 515 (4), 1256 / 1250 at 694 (151 x 241, 24), 1034 / 982 at 644 (331 x
+    // 481, 5), 4290 / 3850 at 2833 (22)
     const double steps = double(nsweeps - 1) * w.delta + std::max(w.nlev, w.nblev);
     const double per_sm = double(nb) * nsweeps * double(g.nni - 2) * double(g.nmu - 5) / steps / ctx->num_sms;
     x2g_ctx::Pending pe{};
@@ -2829,7 +2854,9 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
       continue;
     }
     void *args[] = {&gd, &wd, &jt, &nj, &ns, &bar, &nblocks};
-    err = cudaLaunchCooperativeKernel(per_sm < 85.0 ? (const void *)k_wave_f64<4> : (const void *)k_wave_f64<1>,
+    err = cudaLaunchCooperativeKernel(per_sm < 85.0               ? (const void *)k_wave_f64<4, false>
+                                      : per_sm < 600.0 || !g.pairs ? (const void *)k_wave_f64<1, false>
+                                                                   : (const void *)k_wave_f64<1, true>,
                                       dim3(nblocks), dim3(kWaveThreads), args, smem, ctx->stream);
     if (err != cudaSuccess) return cuda_status(err, "cooperative FP64 sweep launch");
     ctx->launches += 1;
