@@ -912,3 +912,11 @@ def test_wide_wavefront_bitexact(ctx, form, nnu, nmu, njobs, values):
         got, exp = (x.reshape(nmu + 8, nnu + 8)[sl] for x in (u.cpu().numpy(), refs[k % 4]))
         assert np.array_equal(got, exp, equal_nan=True), k
     g.close()
+
+
+# blocks of four rows with two lanes a point (long rows, all sweeps at work) and of eight rows, a last block with one
+# row, more sweeps than a block has under way at once
+@pytest.mark.parametrize("nnu,nmu,njobs,nsweeps", [(181, 31, 12, 10), (181, 31, 30, 12), (31, 61, 18, 3)])
+@pytest.mark.parametrize("isym", [1, -1])
+def test_marching_sor_bitexact(ctx, nnu, nmu, njobs, nsweeps, isym):
+    test_wavefront_sweeps_bitexact(ctx, nnu, nmu, njobs, nsweeps, "sor", isym)

@@ -855,32 +855,35 @@ __global__ void __launch_bounds__(kWaveThreads, 1) k_wave_f64(GridDev g, WaveDev
 // List-order SOR of a few functions: the same dataflow on values in shared
 // memory.  A block owns kRows rows of one job (the mu=1 row included) for the
 // whole launch and keeps them, with four rows on each side, as (value, tag)
-// words in shared memory.  A runner, four lanes, follows a row's columns in one
-// sweep from the middle to one side, in list order, then the axis; it goes on
-// as soon as its point's values are there, so the rows of a warp settle one
-// column apart.  A warp's eight runners are two sides of four rows in one sweep
-// or of two rows in two, and take every kMarchSweeps-th sweep.  The other warps
-// fetch the neighbours' rows, a lane per row, side and sweep, from the tagged
-// copy in global memory.  A value of a row outside the block's own is
-// overwritten there only after its readers in this block are through (see
-// above), so the copies need no further order.
+// words in shared memory.  A runner, kLanes lanes, follows a row's columns in
+// one sweep from the middle to one side, in list order, then the axis; it goes
+// on as soon as its point's values are there, so the rows of a warp settle one
+// column apart.  A warp's runners are both sides of all rows, in march_per
+// sweeps, and take every kMarchSweeps-th sweep.  The other warps fetch the
+// neighbours' rows, a lane per row, side and sweep, from the tagged copy in
+// global memory.  A value of a row outside the block's own is overwritten there
+// only after its readers in this block are through (see above), so the copies
+// need no further order.
 //
-// What bounds it: the FP64 chain of a point (2050 cycles) and one round of loads
-// while a block has few runners at work; more than four warps share an SM's
-// FP64 pipe (23 operations a point and warp of 19 cycles each), hence two rows
-// per block, half the warps on an SM, while there are SMs enough for that.  The
-// way of a value through L2, most of a step's 5800 cycles when every value
-// takes it, is paid once per block of rows.  All nine or ten values of a point
-// are loaded at once (one after the other, as each is found, took 1550 cycles).
-// SOR, 10 sweeps of one orbital, wavefront / this: 331 x 481 2.26 / 1.29 ms
-// (four rows), 151 x 181 0.93 / 0.48, 91 x 121 0.62 / 0.37 (two rows; four rows
-// 0.63 and 0.40).
+// What bounds it: the FP64 chain of a point (2050 cycles with four lanes) and
+// one round of loads while a block has few runners at work; more than four
+// warps share an SM's FP64 pipe (19 cycles an operation and warp; 23 operations
+// for 8 points with four lanes, 33 for 16 with two), hence few rows per block,
+// fewer warps on an SM, while there are SMs enough for that, and two lanes where
+// the pipe is the bound.  The way of a value through L2, most of a step's 5800
+// cycles when every value takes it, is paid once per block of rows.  All nine or
+// ten values of a point are loaded at once (one after the other, as each is
+// found, took 1550 cycles).  SOR, 10 sweeps of one orbital, wavefront / this:
+// 331 x 481 2.26 / 1.14 ms (four rows, two lanes), 151 x 181 0.93 / 0.48, 91 x
+// 121 0.62 / 0.36 (two rows, four lanes; four rows 0.63 and 0.40).
 // ----------------------------------------------------------------------
 constexpr int kMarchSweeps = 10;
 constexpr int kMarchFetch = (8 * 2 * kMarchSweeps + 31) / 32;  // warps that fetch
-// threads of a block of kRows rows (4 or 2: a warp's eight runners are then
-// those of 4 / kRows sweeps)
-__host__ __device__ constexpr int march_threads(int rows) { return 32 * (kMarchSweeps * rows / 4 + kMarchFetch); }
+// sweeps that a warp's runners are of, and threads of a block
+__host__ __device__ constexpr int march_per(int rows, int lanes) { return 16 / lanes / rows; }
+__host__ __device__ constexpr int march_threads(int rows, int lanes) {
+  return 32 * (kMarchSweeps / march_per(rows, lanes) + kMarchFetch);
+}
 
 __device__ __forceinline__ Tagged ld_near(unsigned at) {
   unsigned long long lo, hi;
@@ -893,12 +896,12 @@ __device__ __forceinline__ void st_near(unsigned at, double v, int tag) {
                : "memory");
 }
 
-template <int kRows>
-__global__ void __launch_bounds__(march_threads(kRows), 1)
+template <int kRows, int kLanes>
+__global__ void __launch_bounds__(march_threads(kRows, kLanes), 1)
     k_march_f64(GridDev g, MarchDev w, const __grid_constant__ JobTable jobs, int njobs, int nsweeps, BarrierDev bar,
                 unsigned nblocks) {
   extern __shared__ __align__(16) ulonglong2 near[];
-  constexpr int kThr = march_threads(kRows), kPer = 4 / kRows, kWarps = kMarchSweeps / kPer;
+  constexpr int kThr = march_threads(kRows, kLanes), kPer = march_per(kRows, kLanes), kWarps = kMarchSweeps / kPer;
   const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
   wave_prologue<true>(g, jobs, njobs, int(blockIdx.x) * kThr + tid, int(gridDim.x) * kThr);
   if (!grid_barrier(bar, nblocks)) return;
@@ -949,14 +952,18 @@ __global__ void __launch_bounds__(march_threads(kRows), 1)
     }
     return;
   }
-  const int role = lane & 3, half = lane >> 2 & 1, row = r0 + (lane >> 3) % kRows;
-  double cf[4];
-  {
-    const double *c = role == 0 ? g.dmu2 : role == 1 ? g.dmu1 : role == 2 ? g.dni2 : g.dni1;
+  const int role = lane % kLanes, runner = lane / kLanes, half = runner & 1, row = r0 + (runner >> 1) % kRows;
+  const bool along_nu = role >= kLanes / 2;
+  // four lanes: second and first derivative along mu, then along nu; two: both
+  // along mu, along nu (cf2 and cf1)
+  double cf2[4], cf1[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) cf[q] = c[q];
+  for (int q = 0; q < 4; ++q) {
+    cf2[q] = along_nu ? g.dni2[q] : g.dmu2[q];
+    cf1[q] = along_nu ? g.dni1[q] : g.dmu1[q];
+    if (kLanes == 4 && (role & 1)) cf2[q] = cf1[q];
   }
-  const int st = role < 2 ? n8 : 1, bit = role < 2 ? 2 : 0;
+  const int st = along_nu ? 1 : n8, bit = along_nu ? 0 : 2;
   const double omega = J.omega, omega1 = 1.0 - J.omega;
   const double bmu = row < nmu ? (J.kind >= 1 ? g.bpot_mu : g.borb_mu)[row - 4] : 0.0;
   int o = 0, n = 0;
@@ -965,7 +972,7 @@ __global__ void __launch_bounds__(march_threads(kRows), 1)
     n = w.off[(row - 4) * 2 + half + 1] - o;
   }
   const double2 *pairs = reinterpret_cast<const double2 *>(J.pairs) - 2 * (4 * g.nni + 4);  // by ext row * nni + ext col
-  for (int s = warp * kPer + (lane >> 3) / kRows; __any_sync(0xffffffffu, s < nsweeps); s += kMarchSweeps) {
+  for (int s = warp * kPer + (runner >> 1) / kRows; __any_sync(0xffffffffu, s < nsweeps); s += kMarchSweeps) {
     int k = 0;
     bool on = n > 0 && s < nsweeps;
     // (a runner without a row looks at a point of the first one)
@@ -1000,8 +1007,8 @@ __global__ void __launch_bounds__(march_threads(kRows), 1)
       if (axis) {
         if ((mask & kMarchAxisMu) && ij - row * n8 <= 9) other = row * n8 + 4;
         else if ((mask & kMarchAxisMu) && ij - row * n8 >= g.nni - 2) other = row * n8 + g.nni + 3;
-      } else if (role != 1) {
-        const int f = fifth_reader(g, mask, ij, role == 0 ? 0 : 1);
+      } else {
+        const int f = fifth_reader(g, mask, ij, along_nu ? 1 : 0);
         other = f ? f : ij;
       }
       Tagged x[4], y[4];
@@ -1025,7 +1032,7 @@ __global__ void __launch_bounds__(march_threads(kRows), 1)
       ok = ok && c.tag >= s + (axis ? 1 : 0);
       if (axis && role != 0) ok = true;
       const unsigned waits = __ballot_sync(0xffffffffu, !ok);
-      const bool ready = on && (waits >> (lane & 28) & 0xfu) == 0;
+      const bool ready = on && (waits >> (lane & ~(kLanes - 1)) & ((1u << kLanes) - 1)) == 0;
       if (!__any_sync(0xffffffffu, ready)) {
         if (!__all_sync(0xffffffffu, ww.again(bar))) return;
         if (ww.spins > 4) __nanosleep(ww.spins > 16 ? 200 : 40);
@@ -1034,16 +1041,33 @@ __global__ void __launch_bounds__(march_threads(kRows), 1)
       ww = WaveWait();
       double v = 0.0;
       if (__any_sync(0xffffffffu, ready && !axis)) {
-        // as wave_points4
-        const long long flip = (role & 1) ? (1ll << 63) : 0;
-        double a[4];
+        const int b = lane & ~(kLanes - 1);
+        double ddmi2, bddmi1, ddni2, dddni1;
+        if (kLanes == 4) {
+          // as wave_points4
+          const long long flip = (role & 1) ? (1ll << 63) : 0;
+          double a[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) a[q] = A(m[q], __longlong_as_double(__double_as_longlong(p[q]) ^ flip));
-        double t = A(A(A(M(cf[0], a[0]), M(cf[1], a[1])), M(cf[2], a[2])), M(cf[3], a[3]));
-        t = M(role == 1 ? bmu : role == 3 ? dnu : 1.0, t);
-        const int b = lane & 28;
-        const double ddmi2 = __shfl_sync(0xffffffffu, t, b), bddmi1 = __shfl_sync(0xffffffffu, t, b + 1);
-        const double ddni2 = __shfl_sync(0xffffffffu, t, b + 2), dddni1 = __shfl_sync(0xffffffffu, t, b + 3);
+          for (int q = 0; q < 4; ++q) a[q] = A(m[q], __longlong_as_double(__double_as_longlong(p[q]) ^ flip));
+          double t = A(A(A(M(cf2[0], a[0]), M(cf2[1], a[1])), M(cf2[2], a[2])), M(cf2[3], a[3]));
+          t = M(role == 1 ? bmu : role == 3 ? dnu : 1.0, t);
+          ddmi2 = __shfl_sync(0xffffffffu, t, b);
+          bddmi1 = __shfl_sync(0xffffffffu, t, b + 1);
+          ddni2 = __shfl_sync(0xffffffffu, t, b + 2);
+          dddni1 = __shfl_sync(0xffffffffu, t, b + 3);
+        } else {
+          double t2 = M(cf2[0], A(m[0], p[0])), t1 = M(cf1[0], S(m[0], p[0]));
+#pragma unroll
+          for (int q = 1; q < 4; ++q) {
+            t2 = A(t2, M(cf2[q], A(m[q], p[q])));
+            t1 = A(t1, M(cf1[q], S(m[q], p[q])));
+          }
+          t1 = M(along_nu ? dnu : bmu, t1);
+          ddmi2 = __shfl_sync(0xffffffffu, t2, b);
+          bddmi1 = __shfl_sync(0xffffffffu, t1, b);
+          ddni2 = __shfl_sync(0xffffffffu, t2, b + 1);
+          dddni1 = __shfl_sync(0xffffffffu, t1, b + 1);
+        }
         const double cc = A(A(A(ddmi2, bddmi1), ddni2), dddni1);
         // omega (rhs - cc) and omega1 times the old value, on two lanes at once
         const double o = M(role == 1 ? omega1 : omega, role == 1 ? uc : S(lr.y, cc));
@@ -2754,6 +2778,20 @@ static int relax_bands(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, 
   return X2G_OK;
 }
 
+struct MarchKernel {
+  const void *fn;
+  int threads;
+};
+// two lanes a point where all of a block's sweeps are at work on a row at once
+// (they follow each other 8 columns apart): 331 x 481, four rows, 1.14 ms (four
+// lanes 1.28); 151 x 181, two functions 585 us (558); 91 x 121, four 427 (365)
+static MarchKernel march_kernel(int rows, int nsweeps, int nni) {
+  if (rows == 2) return {(const void *)k_march_f64<2, 4>, march_threads(2, 4)};
+  if (rows == 8) return {(const void *)k_march_f64<8, 2>, march_threads(8, 2)};
+  if (std::min(nsweeps, nni / 16) < kMarchSweeps) return {(const void *)k_march_f64<4, 4>, march_threads(4, 4)};
+  return {(const void *)k_march_f64<4, 2>, march_threads(4, 2)};
+}
+
 // whether blocks of the marching SOR sweep can be resident with this much
 // shared memory (its cap is set to the device's opt-in maximum, once)
 static bool march_fits(x2g_ctx *ctx, size_t smem) {
@@ -2766,7 +2804,11 @@ static bool march_fits(x2g_ctx *ctx, size_t smem) {
       return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) == cudaSuccess &&
              cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fn, threads, size_t(optin)) == cudaSuccess && a >= 1;
     };
-    ok = ok && fits((const void *)k_march_f64<2>, march_threads(2)) && fits((const void *)k_march_f64<4>, march_threads(4));
+    for (int rows = 2; rows <= 8; rows *= 2)
+      for (int sweeps : {1, kMarchSweeps}) {
+        const MarchKernel k = march_kernel(rows, sweeps, 16 * kMarchSweeps);
+        ok = ok && fits(k.fn, k.threads);
+      }
     (void)cudaGetLastError();
     ctx->march_smem = ok ? optin : 0;
   }
@@ -2781,12 +2823,14 @@ static bool march_fits(x2g_ctx *ctx, size_t smem) {
 constexpr size_t kWaveScratch = size_t(256) << 20;
 static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2g_job *jobs, int njobs, int nsweeps,
                       bool profile, const MarchDev *march = nullptr) {
-  // SOR: the marching sweep while every block of rows has its own SM (four
-  // orbitals of 91 x 121, 120 blocks of four rows, 373 us, wavefront 641; two
-  // and three of 151 x 181 578 and 585; four would take two launches, wavefront
-  // 950)
+  // SOR: the marching sweep with the fewest rows a block (2, 4, 8) that give
+  // every block its own SM, else the wavefront.  10 sweeps, us, this /
+  // wavefront: two functions of 331 x 481 (eight rows) 1704 / 2462, four and
+  // six of 151 x 181 (eight) 765 / 952 and 769 / 1032, four and eight of 91 x
+  // 121 (four, eight) 365 / 641 and 483 / 681; beyond that the wavefront is
+  // bound by the FP64 pipe, which this uses worse
   int rows = 0;
-  for (int r = 4; r >= 2 && march; r /= 2)
+  for (int r = 8; r >= 2 && march; r /= 2)
     if (njobs * ((g.nmu - 4 + r - 1) / r) <= ctx->num_sms && march_fits(ctx, size_t(r + 8) * g.n8 * 16)) rows = r;
   if (!rows) march = nullptr;
   const size_t tagged = (size_t(g.next) * 16 + 255) / 256 * 256, pairs = (size_t(g.mxsize) * 32 + 255) / 256 * 256;
@@ -2846,8 +2890,8 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
       MarchDev md = *march;
       nblocks = unsigned(nb * ((g.nmu - 4 + rows - 1) / rows));
       void *args[] = {&gd, &md, &jt, &nj, &ns, &bar, &nblocks};
-      err = cudaLaunchCooperativeKernel(rows == 2 ? (const void *)k_march_f64<2> : (const void *)k_march_f64<4>,
-                                        dim3(nblocks), dim3(unsigned(march_threads(rows))), args,
+      const MarchKernel k = march_kernel(rows, ns, g.nni);
+      err = cudaLaunchCooperativeKernel(k.fn, dim3(nblocks), dim3(unsigned(k.threads)), args,
                                         size_t(rows + 8) * g.n8 * 16, ctx->stream);
       if (err != cudaSuccess) return cuda_status(err, "cooperative SOR launch");
       ctx->launches += 1;
