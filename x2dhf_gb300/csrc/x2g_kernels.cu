@@ -1678,22 +1678,53 @@ inline int red_blocks(const GridDev &g) {
 }
 constexpr int kMaxK = 16;
 
-template <int K>
-__device__ void block_sum_store(double (&v)[K], double *partials) {
-  __shared__ double sh[kThreads / 32][K];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// The sums over a warp of P values each (a power of two up to 16): lane q 32 /
+// P returns that of v[q].  At every halving of the tree the two lanes of a pair
+// also share the values left, so P values take P - 1 + log2(32 / P) additions
+// and not 5 P; each value's tree and its roundings are those of a shuffle tree
+// by itself (additions only swap their operands).
+template <int P>
+__device__ __forceinline__ double warp_sums(double (&x)[P]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
 #pragma unroll
-  for (int q = 0; q < K; ++q) {
-    double x = v[q];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[w][q] = x;
+  for (int n = P; n > 1; n /= 2, o /= 2) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < n / 2; ++j) {
+      const double keep = up ? x[j + n / 2] : x[j], send = up ? x[j] : x[j + n / 2];
+      x[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
   }
+  double s = x[0];
+#pragma unroll
+  for (; o > 0; o /= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// The block's sums of K values, value q < n of block b to base[b bstride + q
+// qstride].  FP64 additions bound the reductions (the trees of 16 values took
+// 80 a warp, 19 cycles each of the SM's pipe).
+template <int K>
+__device__ void block_sum_store(double (&v)[K], double *base, int bstride, int qstride, int n = K) {
+  constexpr int P = K == 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
+  __shared__ double sh[kThreads / 32][P];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double x[P];
+#pragma unroll
+  for (int q = 0; q < P; ++q) x[q] = q < K ? v[q] : 0.0;
+  const double sum = warp_sums<P>(x);
+  if (lane % (32 / P) == 0) sh[w][lane / (32 / P)] = sum;
   __syncthreads();
-  if (threadIdx.x < K) {
+  if (threadIdx.x < n) {
     double s = 0.0;
     for (int i = 0; i < kThreads / 32; ++i) s += sh[i][threadIdx.x];
-    partials[blockIdx.x * K + threadIdx.x] = s;
+    base[size_t(blockIdx.x) * bstride + size_t(threadIdx.x) * qstride] = s;
   }
+}
+template <int K>
+__device__ void block_sum_store(double (&v)[K], double *partials) {
+  block_sum_store<K>(v, partials, K, 1);
 }
 
 // Every block stores its K partial sums; the block that finishes last (an
@@ -1701,32 +1732,10 @@ __device__ void block_sum_store(double (&v)[K], double *partials) {
 // block order -- the same order on every run -- and
 // writes out[0..nout).  Returns true in that block.  No block waits for
 // another.
-// Sum of partial q of nblocks blocks' stores (K per block), in block order:
-// thread t adds blocks t, t + blockDim, ..., then a warp tree, then the warp
-// totals in warp order.  Every thread of the block gets the total.
-__device__ double sum_partials(const double *partials, int K, int q, int nblocks) {
-  __shared__ double sh[kThreads / 32];
-  __shared__ double tot;
-  double s = 0.0;
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) s += __ldcg(partials + size_t(b) * K + q);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int i = 0; i < kThreads / 32; ++i) t += sh[i];
-    tot = t;
-  }
-  __syncthreads();
-  const double r = tot;
-  __syncthreads();
-  return r;
-}
-
-// sum_partials of nq <= kMaxK slots at once, slot q of block b at
-// base[b * bstride + q * qstride]: the same sums in the same order, with one
-// pass over the partials and two block barriers for all of them; out[] in
-// shared memory, valid in every thread on return
+// The sums over the blocks of nq <= kMaxK slots, slot q of block b at base[b *
+// bstride + q * qstride]: thread t adds blocks t, t + blockDim, ..., then a
+// warp tree, then the warp totals in warp order.  out[] in shared memory, valid
+// in every thread on return
 __device__ void sum_partials_multi(const double *base, int bstride, int qstride, int nq, int nblocks, double *out) {
   __shared__ double sh[kThreads / 32][kMaxK];
   double s[kMaxK];
@@ -1737,12 +1746,17 @@ __device__ void sum_partials_multi(const double *base, int bstride, int qstride,
     for (int q = 0; q < kMaxK; ++q)
       if (q < nq) s[q] += __ldcg(base + size_t(b) * bstride + size_t(q) * qstride);
   }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (nq <= 3) {
 #pragma unroll
-  for (int q = 0; q < kMaxK; ++q) {
-    if (q >= nq) break;
-    double x = s[q];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][q] = x;
+    for (int q = 0; q < 3; ++q) {
+      double x[1] = {s[q]};
+      if (q < nq) x[0] = warp_sums<1>(x);
+      if (q < nq && lane == 0) sh[w][q] = x[0];
+    }
+  } else {
+    const double sum = warp_sums<kMaxK>(s);
+    if (lane % (32 / kMaxK) == 0) sh[w][lane / (32 / kMaxK)] = sum;
   }
   __syncthreads();
   if (threadIdx.x < nq) {
@@ -1763,11 +1777,12 @@ __device__ bool block_sum_finish(double (&v)[K], double *partials, double *out, 
   __syncthreads();
   if (!s_last) return false;
   __threadfence();
-  for (int q = 0; q < nout; ++q) {
-    const double t = sum_partials(partials, K, q, int(gridDim.x));
-    if (threadIdx.x == 0) out[q] = t;
+  __shared__ double s_out[kMaxK];
+  sum_partials_multi(partials, K, 1, nout, int(gridDim.x), s_out);
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < nout; ++q) out[q] = s_out[q];
+    *ticket = 0u;
   }
-  if (threadIdx.x == 0) *ticket = 0u;
   return true;
 }
 
@@ -1954,13 +1969,8 @@ __global__ void __launch_bounds__(kThreads) k_orthonormalise(GridDev g, const __
         v[j] += w2 * M(M(p, p), f4);
       }
     }
-#pragma unroll
-    for (int j = 0; j < kGroup; ++j) {
-      if (a + j >= n) break;
-      double w[1] = {v[j]};
-      block_sum_store<1>(w, partials + size_t(a + j) * nb);
-      __syncthreads();
-    }
+    block_sum_store<kGroup>(v, partials + size_t(a) * nb, 1, nb, min(kGroup, n - a));
+    __syncthreads();
   }
   __threadfence();
   if (!grid_barrier(bar, unsigned(nb))) return;
