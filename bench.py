@@ -483,24 +483,24 @@ def run_gpu(args):
             "peak_kind": peak_kind,
             "bytes_per_point_update": BYTES_PER_PT[1],
             "note": ("achieved = 16 algorithmic B per point-update / launch time; the correction lives in shared "
-                     "memory during the sweeps, so DRAM traffic is far below it and the launch is bound by the "
-                     "colour-phase latency (cluster barrier + shared-memory pipe), not by HBM" if on_chip else
+                     "memory during the sweeps, so DRAM traffic is far below it and the launch is bound by "
+                     "instruction issue and the latency of a colour phase, not by HBM" if on_chip else
                      "achieved = 16 algorithmic B per point-update / launch time; the correction stays in shared "
                      "memory for the whole launch, so DRAM traffic stays far below the algorithmic bytes and the "
                      "launch is bound by phase latency (neighbour wait, halo round trip, level chain), not by HBM"),
             "sweep_ms_total": msmx, "sweep_launches": nmx, "point_updates": ptsmx,
             "point_updates_per_launch": pts_per_launch,
-            # SM-side utilisation of the on-chip sweep (ncu --set full, one launch of 16 potentials on
-            # this grid; profiles/mixed_cluster_pot_sweep_poisson_b16_331x481.md): the kernel's bound
-            "sm_side_ncu": ({"l1_shared_throughput_frac": 0.524, "issue_active_frac": 0.439,
-                             "lsu_instruction_frac": 0.342, "fma_pipe_frac": 0.194,
-                             "barrier_stalls_per_issue": 7.63} if on_chip else None),
+            # SM-side utilisation of the on-chip sweep (ncu, one launch of 22 potentials on this grid;
+            # profiles/columns_sweep_n2_22_potentials.md): the kernel's bound
+            "sm_side_ncu": ({"l1_shared_throughput_frac": 0.530, "issue_active_frac": 0.38,
+                             "lsu_instruction_frac": 0.437, "fma_pipe_frac": 0.136,
+                             "barrier_stalls_per_issue": 1.53} if on_chip else None),
             "clusters_co_resident": {"plain": occ[0], "potentials_variant": occ[1],
                                      "potentials_variant_mode": args.potential_clusters},
             "colouring": args.colouring,
             "residual_overlap": args.residual_overlap,
             "orthonormalise": args.orthonormalise,
-            "fp64_kernel": {"kernel": "k_mcsor_f64", "achieved_gbs": sweep_gbs_64,
+            "fp64_kernel": {"kernel": "k_wave_f64", "achieved_gbs": sweep_gbs_64,
                             "frac_hbm": (sweep_gbs_64 / hbm) if sweep_gbs_64 else None,
                             "achieved_tflops": pts64 * FLOPS_PER_PT / (ms64 / 1e3) / 1e12 if ms64 > 0 else None,
                             "bound": "fp64 ALU (1.19 TFLOP/s measured on this GB300)",

@@ -113,11 +113,13 @@ int x2g_grid_table(x2g_grid *grid, int which, double *host_out);
 int x2g_host_table(int nnu, int nmu, double r, double rinf, double z1, double z2, int which, double *out);
 int x2g_host_schedule(int nnu, int nmu, int *npoints, int *ntiles, int *nlevels, int *order, int *tile,
                       int *colour, int *level);
-/* Cluster plan of the on-chip FP32 sweep of the mixed form (no CUDA call):
- * CTAs per relaxation job (0 = grid too large, persistent-band kernel used),
- * rows of the largest band, shared memory per CTA, band starts row0[C+1]. */
+/* Plan of whole schedule tiles for one cluster per relaxation job (no CUDA
+ * call): CTAs (0 = the grid needs more than one cluster), rows of the largest
+ * band, shared memory per CTA, band starts row0[C+1].  The on-chip sweep of the
+ * mixed form cuts the grid by columns and rows of its own and picks the cluster
+ * size per batch; this plan and its chunk lists serve inspection and tests. */
 int x2g_host_cluster_plan(int nnu, int nmu, int *csize, int *maxrows, long *smem, int *row0);
-/* Chunk lists of the on-chip sweep (host only): chunks of up to 4 points of
+/* Chunk lists of that plan (host only): chunks of up to 4 points of
  * one row at stride 5, packed (band row << 19) | (ext col << 2) | (count-1),
  * and the offsets of each CTA's 5 colours x (levels + 2) segments (level 0
  * off the shared band edges, level 0 near them, level-0 seam points, levels

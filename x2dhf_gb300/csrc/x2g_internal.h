@@ -96,8 +96,9 @@ struct HostGrid {
   std::vector<int> pts;  // ext indices grouped [tile][colour][level]
   std::vector<int> off;  // (ntiles*5*nlev + 1) offsets into pts
   std::vector<int> pts_rc;  // same points as (ext row << 16) | ext col
-  // cluster plan of the on-chip FP32 sweep: cl_size CTAs per job, CTA k
-  // owns tiles [cl_tile0[k], cl_tile0[k+1]) = ext rows [cl_row0[k], cl_row0[k+1])
+  // plan of whole tiles for one cluster per job (host only, for inspection;
+  // the on-chip sweep's are in columns): cl_size CTAs per job, CTA k owns
+  // tiles [cl_tile0[k], cl_tile0[k+1]) = ext rows [cl_row0[k], cl_row0[k+1])
   int cl_size = 0, cl_maxrows = 0, cl_maxchunks = 0, cl_wa = 1, cl_wb = 1, cl_ws = 1;
   // warps per role of the potentials' variant (two CTAs per SM, at most kPotWarpsRef)
   int cl_pa = 1, cl_pb = 1, cl_ps = 1;
