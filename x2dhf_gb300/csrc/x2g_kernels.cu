@@ -405,7 +405,9 @@ __global__ void __launch_bounds__(kThreads) k_mcsor_f64(GridDev g, const __grid_
 // after the other.
 // ----------------------------------------------------------------------
 constexpr int kWaveThreads = 512;
-constexpr size_t kWaveSmem = 47 * 1024;  // level offsets held in shared memory, within the default cap
+// level offsets held in shared memory: a usual grid's within the default cap,
+// the most that a launch may ask for
+constexpr size_t kWaveSmem = 47 * 1024, kWaveSmemMost = 200 * 1024;
 constexpr unsigned kTagFixed = 0x7fffffffu;  // values no sweep changes
 
 struct Tagged {
@@ -2849,12 +2851,16 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
   char *scratch = static_cast<char *>(ctx_workspace(ctx, (tagged + pairs) * size_t(most)));
   if (!scratch) return set_status(X2G_ERR_ALLOC, "workspace allocation failed");
   const size_t smem = size_t(w.nlev + w.nblev + 2) * sizeof(int);
-  if (smem > kWaveSmem) return set_status(X2G_ERR_ARG, "grid too large for the wavefront's level table");
+  if (smem > kWaveSmemMost) return set_status(X2G_ERR_ARG, "grid too large for the wavefront's level table");
   if (ctx->wave_ok < 0) {
     int a = 0, b = 0;
     int w = 0;
-    cudaError_t e =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, (const void *)k_wave_f64<4, false>, kWaveThreads, kWaveSmem);
+    cudaError_t e = cudaSuccess;
+    for (const void *fn : {(const void *)k_wave_f64<4, false>, (const void *)k_wave_f64<1, false>,
+                           (const void *)k_wave_f64<1, true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kWaveSmemMost));
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, (const void *)k_wave_f64<4, false>, kWaveThreads, kWaveSmem);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void *)k_wave_f64<1, false>, kWaveThreads, kWaveSmem);
     if (e == cudaSuccess)
