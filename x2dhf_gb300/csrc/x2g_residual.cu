@@ -223,6 +223,7 @@ __global__ void __launch_bounds__(kThreadsRes, kBlocksRes)
   const int nuc = in ? nu : nni - 2;
   const unsigned at_ext = 8u * unsigned((mu1 + 4) * n8 + nuc + 4), at_int = 8u * unsigned(mu1 * nni + nuc);
   double rest[kRowsPerWarp];
+  float w32[kRowsPerWarp];  // kPacked: omega / lhs
   {
     const double idel2 = J.idel2;
     const bool plain = __double2hiint(idel2) == 0;
@@ -236,13 +237,10 @@ __global__ void __launch_bounds__(kThreadsRes, kBlocksRes)
       if (rows > 0) {
         if (!plain) lhs = fma(idel2, at(g.e, k), lhs);
         rest[q] = fma(-lhs, at(u, e), (at(psa, e) * at(psb, e)) * at(g.g, k));
-        if (need_w && in && q < rows) {
-          const float w = J.omegaf / narrow_f64(lhs);
-          if (kPacked)
-            J.rw[__ldg(g.st_place + (mu1 + q - 1) * (nni - 2) + nu - 1)].y = w;
-          else
-            J.w32[(mu1 + q) * nni + nu] = w;
-        }
+        if (kPacked)
+          w32[q] = J.omegaf / narrow_f64(lhs);
+        else if (need_w && in && q < rows)
+          J.w32[(mu1 + q) * nni + nu] = J.omegaf / narrow_f64(lhs);
       }
     }
   }
@@ -319,7 +317,7 @@ __global__ void __launch_bounds__(kThreadsRes, kBlocksRes)
     }
     if (in && q < rows) {
       if (kPacked)
-        J.rw[__ldg(g.st_place + (mu1 + q - 1) * (nni - 2) + nu - 1)].x = r;
+        J.rw[__ldg(g.st_place + (mu1 + q - 1) * (nni - 2) + nu - 1)] = make_float2(r, w32[q]);
       else
         J.r32[(mu1 + q) * nni + nu] = r;
     }
