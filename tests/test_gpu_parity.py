@@ -920,3 +920,37 @@ def test_wide_wavefront_bitexact(ctx, form, nnu, nmu, njobs, values):
 @pytest.mark.parametrize("isym", [1, -1])
 def test_marching_sor_bitexact(ctx, nnu, nmu, njobs, nsweeps, isym):
     test_wavefront_sweeps_bitexact(ctx, nnu, nmu, njobs, nsweeps, "sor", isym)
+
+
+@pytest.mark.parametrize("njobs,nsweeps", [(7, 2), (9, 1)])
+def test_large_band_blocks_match_single_jobs(ctx, njobs, nsweeps):
+    """Seven jobs of 781x1201 fit one launch of the persistent-band sweep only
+    in blocks of 1024 threads (nine: seven of those and a last launch of two in
+    shorter bands): the bands' heights do not enter the results, so each job
+    equals the same job relaxed alone bit for bit."""
+    torch = pytest.importorskip("torch")
+    nnu, nmu = 781, 1201
+    g = xg.Grid(ctx, nnu, nmu, 2.0, 25.0, 1.0, 1.0)
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(7)
+    u0 = []
+    for _ in range(njobs):
+        u = torch.zeros(nmu + 8, nnu + 8, dtype=torch.float64, device=dev)
+        u[4:nmu + 4, 4:nnu + 4] = torch.randn(nmu, nnu, generator=gen, dtype=torch.float64, device=dev)
+        u0.append(u)
+    lhs = -1e4 * (1.0 + torch.rand(nmu * nnu, generator=gen, dtype=torch.float64, device=dev))
+    rhs = torch.randn(nmu * nnu, generator=gen, dtype=torch.float64, device=dev)
+
+    def jobs(us):
+        return [xg.Job(u=u.data_ptr(), lhs=lhs.data_ptr(), rhs=rhs.data_ptr(), omega=1.9, isym=1 if k % 2 == 0 else -1, kind=0)
+                for k, u in enumerate(us)]
+
+    together, alone = [u.clone() for u in u0], [u.clone() for u in u0]
+    torch.cuda.synchronize()
+    xg.relax(ctx, g, jobs(together), nsweeps, xg.MIXED)
+    for j in jobs(alone):
+        xg.relax(ctx, g, [j], nsweeps, xg.MIXED)
+    ctx.synchronize()
+    for k, (x, y, u) in enumerate(zip(together, alone, u0)):
+        assert torch.equal(x, y) and not torch.equal(x, u), k
+    g.close()

@@ -1163,7 +1163,8 @@ __host__ __device__ inline size_t band_smem_bytes(const GridDev &g, int G) {
 // and a halo piece that reaches into an own row covers only ghost columns
 // (zero throughout).  The kernel ends with u += e and the FP64 axis values
 // of u on the band's rows, so the correction never returns to global memory.
-__global__ void __launch_bounds__(kBandThreads) k_mcsor_f32p(GridDev g, const __grid_constant__ JobTable jobs,
+template <int kMost>
+__global__ void __launch_bounds__(kMost) k_mcsor_f32p(GridDev g, const __grid_constant__ JobTable jobs,
                                                                int nsweeps, int G, BarrierDev bar,
                                                                unsigned *phase) {
   extern __shared__ __align__(16) float sband[];
@@ -2598,20 +2599,31 @@ static ColChoice choose_columns(x2g_ctx *ctx, const HostGrid &h, int njobs, bool
   return best;
 }
 
+static const void *band_kernel(int threads) {
+  return threads == kBandThreads ? (const void *)k_mcsor_f32p<kBandThreads> : (const void *)k_mcsor_f32p<2 * kBandThreads>;
+}
+
 // Launch shape of the persistent-band sweep: the most jobs per launch (at
 // most `most`) and the shortest tile runs G for which every (job, run) gets
-// its own co-resident block at two 512-thread blocks per SM (the band's
-// shared memory must fit twice per SM).  The function's shared memory cap
-// is raised once to the device's opt-in maximum, as for the cluster kernel.
-static int persistent_shape(x2g_ctx *ctx, const GridDev &g, int most, int *nj, int *G, size_t *smem) {
+// its own co-resident block, at two 512-thread blocks per SM (the band's
+// shared memory must fit twice) or, where that holds more jobs, one block of
+// 1024: its band is twice as high with the same halos.  A launch takes 285 us
+// and 30 per job of 781 x 1201 (10 sweeps), so fewer launches are faster: seven
+// jobs 544 us in one launch of the large blocks, 758 in two of the small ones;
+// six 468 (480 in large ones).  The functions' shared memory cap is raised once
+// to the device's opt-in maximum, as for the cluster kernel.
+static int persistent_shape(x2g_ctx *ctx, const GridDev &g, int most, int *nj, int *G, size_t *smem,
+                            int *threads = nullptr) {
   if (!ctx->band_attr) {
     // the cap counts dynamic bytes only: the opt-in maximum less the
     // kernel's static shared memory (the neighbour wait's flag)
     int optin = 0;
     cudaFuncAttributes fa{};
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa, (const void *)k_mcsor_f32p) != cudaSuccess ||
-        cudaFuncSetAttribute((const void *)k_mcsor_f32p, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncGetAttributes(&fa, band_kernel(kBandThreads)) != cudaSuccess ||
+        cudaFuncSetAttribute(band_kernel(kBandThreads), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             optin - int(fa.sharedSizeBytes)) != cudaSuccess ||
+        cudaFuncSetAttribute(band_kernel(2 * kBandThreads), cudaFuncAttributeMaxDynamicSharedMemorySize,
                              optin - int(fa.sharedSizeBytes)) != cudaSuccess) {
       (void)cudaGetLastError();
       return set_status(X2G_ERR_CUDA, "persistent sweep attributes could not be set");
@@ -2623,32 +2635,28 @@ static int persistent_shape(x2g_ctx *ctx, const GridDev &g, int most, int *nj, i
     ctx->band_sm_smem = per_sm;
   }
   for (int n = most; n >= 1; --n)
-    for (int r = 1; r <= HostGrid::kBandRuns; ++r) {
-      const size_t sm = band_smem_bytes(g, r);
-      if (sm > size_t(ctx->band_attr)) break;
-      // two blocks per SM (1024 threads) hide more latency than one block
-      // with twice the band
-      int bpsm = int(size_t(ctx->band_sm_smem) / (sm + 1024));
-      if (bpsm < 2) break;
-      bpsm = 2;
-      const int items = n * ((g.ntiles + r - 1) / r);
-      if (bpsm >= 1 && items <= bpsm * ctx->num_sms) {
+    for (int bpsm = 2; bpsm >= 1; --bpsm)
+      for (int r = 1; r <= HostGrid::kBandRuns; ++r) {
+        const size_t sm = band_smem_bytes(g, r);
+        if (sm > size_t(ctx->band_attr) || int(size_t(ctx->band_sm_smem) / (sm + 1024)) < bpsm) break;
+        const int items = n * ((g.ntiles + r - 1) / r), nt = kBandThreads * (bpsm == 1 ? 2 : 1);
+        if (items > bpsm * ctx->num_sms) continue;
         // confirm with the occupancy calculator (once per shared size)
-        if (ctx->band_key != long(sm)) {
+        const long key = long(sm) * 2 + bpsm - 1;
+        if (ctx->band_key != key) {
           int per = 0;
-          cudaError_t err =
-              cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)k_mcsor_f32p, kBandThreads, sm);
+          cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, band_kernel(nt), nt, sm);
           if (err != cudaSuccess) return cuda_status(err, "occupancy query");
-          ctx->band_key = long(sm);
+          ctx->band_key = key;
           ctx->band_blocks = per * ctx->num_sms;
         }
         if (items > ctx->band_blocks) continue;
         *nj = n;
         *G = r;
         *smem = sm;
+        if (threads) *threads = nt;
         return X2G_OK;
       }
-    }
   return set_status(X2G_ERR_ARG, "grid too large for the persistent FP32 sweep");
 }
 
@@ -2755,7 +2763,7 @@ static int relax_on_chip(x2g_ctx *ctx, const GridDev &g, const ColChoice &col, i
 
 // Mixed form in persistent bands: one launch batch (at most kParamJobs jobs).
 static int relax_bands(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, int nsweeps, bool fixed, int G,
-                       size_t smem) {
+                       size_t smem, int threads) {
   cudaError_t err;
   x2g_ctx::Pending pe{};
   launch_residual(g, jt, njobs, fixed, true, true, ctx->stream);
@@ -2779,7 +2787,7 @@ static int relax_bands(x2g_ctx *ctx, const GridDev &g, JobTable &jt, int njobs, 
   int ns = nsweeps;
   GridDev gd = g;
   void *args[] = {&gd, &jt, &ns, &G, &bar, &phase};
-  err = cudaLaunchCooperativeKernel((const void *)k_mcsor_f32p, dim3(nb), dim3(kBandThreads), args, smem, ctx->stream);
+  err = cudaLaunchCooperativeKernel(band_kernel(threads), dim3(nb), dim3(unsigned(threads)), args, smem, ctx->stream);
   if (err != cudaSuccess) return cuda_status(err, "cooperative MCSOR launch");
   ctx->launches += 1;
   if (ctx->profiling) {
@@ -2998,15 +3006,19 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
   if (col.plan) return relax_on_chip(ctx, g, col, njobs, nsweeps, fixed, job);
   // the persistent-band sweep takes as many jobs per launch as give every
   // (job, run of tiles) its own co-resident block
-  int per_launch = kParamJobs, G = 0;
+  int per_launch = kParamJobs, G = 0, threads = kBandThreads;
   size_t smem = 0;
-  int rc = persistent_shape(ctx, g, njobs < kParamJobs ? njobs : kParamJobs, &per_launch, &G, &smem);
+  int rc = persistent_shape(ctx, g, njobs < kParamJobs ? njobs : kParamJobs, &per_launch, &G, &smem, &threads);
   if (rc) return rc;
   for (int b0 = 0; b0 < njobs; b0 += per_launch) {
-    const int nb = (njobs - b0 < per_launch) ? njobs - b0 : per_launch;
+    int nb = (njobs - b0 < per_launch) ? njobs - b0 : per_launch;
+    // a short last launch in shorter bands, so that it fills the SMs too (33 jobs
+    // of 781 x 1201 in launches of six: 2728 us, 2745 with the last three in runs
+    // of six tiles)
+    if (nb < per_launch && (rc = persistent_shape(ctx, g, nb, &nb, &G, &smem, &threads))) return rc;
     JobTable jt{};
     for (int i = 0; i < nb; ++i) jt.j[i] = job(b0 + i);
-    if ((rc = relax_bands(ctx, g, jt, nb, nsweeps, fixed, G, smem))) return rc;
+    if ((rc = relax_bands(ctx, g, jt, nb, nsweeps, fixed, G, smem, threads))) return rc;
   }
   // barrier error word: checked by the caller at its next synchronisation
   return X2G_OK;
