@@ -887,14 +887,20 @@ __host__ __device__ constexpr int march_threads(int rows, int lanes) {
   return 32 * (kMarchSweeps / march_per(rows, lanes) + kMarchFetch);
 }
 
+// one 128-bit access: a reader must never see a tag without its value (a vector
+// of two 64-bit ones may be taken apart)
 __device__ __forceinline__ Tagged ld_near(unsigned at) {
   unsigned long long lo, hi;
-  asm volatile("ld.volatile.shared.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(at) : "memory");
+  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.cta.shared.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+               : "=l"(lo), "=l"(hi)
+               : "r"(at)
+               : "memory");
   return Tagged{__longlong_as_double((long long)lo), int(unsigned(hi))};
 }
 __device__ __forceinline__ void st_near(unsigned at, double v, int tag) {
-  asm volatile("st.volatile.shared.v2.b64 [%0], {%1, %2};" ::"r"(at), "l"(__double_as_longlong(v)),
-               "l"((unsigned long long)(unsigned)tag)
+  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%0, %1};\n\tst.relaxed.cta.shared.b128 [%2], q;\n\t}" ::"l"(
+                   __double_as_longlong(v)),
+               "l"((unsigned long long)(unsigned)tag), "r"(at)
                : "memory");
 }
 
