@@ -138,11 +138,12 @@ int x2g_host_free_chunks(int nnu, int nmu, int *nchunks, int *noff, int *chunks,
 int x2g_host_band_schedule(int nnu, int nmu, int *npoints, int *ntiles, int *nlevels, int *pts, int *off, int *rows,
                            int *tile_row0, int *tile_row1);
 /* Longest time one block of a persistent sweep waits for the others (its
- * grid barrier or its neighbours' phase counts) before the launch gives up:
- * the block records X2G_ERR_TIMEOUT in the context's error word and every
- * block returns, so a stalled launch never hangs the GPU.  The error word
- * stays set, and later launches on the context leave at their first wait,
- * until x2g_synchronize (or the call's own readback) reports it and clears
+ * grid barrier, its neighbours' phase counts or halo values, or a value of the
+ * FP64 sweeps without barriers) before the launch gives up: the block records
+ * X2G_ERR_TIMEOUT in the context's error word and every block returns, so a
+ * stalled launch never hangs the GPU.  The error word stays set, and later
+ * launches on the context leave at their first wait (the mixed form's cluster
+ * sweep before its first sweep, with the functions as they were), until x2g_synchronize (or the call's own readback) reports it and clears
  * it.  Default 2 s; 0 makes any wait that is not met at once fail (for
  * testing the error path).  Applies to launches queued after the call.  The
  * reference has no device waits (its threads join, src/c/mcsor_pthread.c:87). */

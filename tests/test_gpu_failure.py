@@ -111,3 +111,87 @@ def test_wait_limit_argument_checked():
     assert ei.value.code == 1
     ctx.set_wait_limit(2.0)
     ctx.close()
+
+
+@pytest.mark.parametrize("clusters", [True, False], ids=["potentials", "plain"])
+def test_on_chip_sweep_timeout_is_reported_and_context_recovers(ne, clusters):
+    """The on-chip sweep's waits for its neighbours' halo values: the same
+    contract; a launch that finds the error word set leaves u alone, and so
+    does a cluster in which a wait ran out."""
+    torch, c = ne[0], ne[1]
+    ctx = xg.Context(0)
+    ctx.set_potential_clusters(clusters)
+    g = xg.Grid(ctx, c.nnu, c.nmu, c.r, c.rinf, c.z1, c.z2)
+    assert min(g.cluster_occupancy()) > 0
+    keep, bufs, jobs = _batch(ne)
+    xg.relax(ctx, g, jobs, 10, xg.MIXED)
+    ctx.synchronize()
+    ref = [b.cpu().numpy() for b in bufs]
+    start = [s[4] for s in ne[3]]
+    k1 = _batch(ne)
+    ctx.set_wait_limit(0.0)
+    xg.relax(ctx, g, k1[2], 10, xg.MIXED)
+    k2 = _batch(ne)
+    ctx.set_wait_limit(2.0)
+    xg.relax(ctx, g, k2[2], 10, xg.MIXED)
+    with pytest.raises(xg.X2GError) as ei:
+        ctx.synchronize()
+    assert ei.value.code == 4, str(ei.value)
+    for k, (x, y, s, r) in enumerate(zip(k1[1], k2[1], start, ref)):
+        x, y = x.cpu().numpy(), y.cpu().numpy()
+        assert np.array_equal(y, s), k
+        assert np.array_equal(x, s) or np.array_equal(x, r), k
+    assert any(np.array_equal(x.cpu().numpy(), s) for x, s in zip(k1[1], start))
+    keep, bufs, jobs = _batch(ne)
+    xg.relax(ctx, g, jobs, 10, xg.MIXED)
+    ctx.synchronize()
+    for k, (b, r) in enumerate(zip(bufs, ref)):
+        assert np.array_equal(b.cpu().numpy(), r), k
+    g.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("njobs", [1, 12], ids=["marching", "wavefront"])
+def test_value_waits_of_the_fp64_sweeps_run_out(njobs):
+    """List-order SOR hands values on without barriers.  A sweep of 331 x 481
+    takes about a millisecond and its outer rows' first values half of that,
+    so with a limit of 0.1 ms the grid barrier at the start is met and the
+    waits for values run out: the middle of the grid is relaxed, the outer
+    rows are not."""
+    torch = pytest.importorskip("torch")
+    nnu, nmu = 331, 481
+    dev = torch.device("cuda:0")
+    gen = torch.Generator().manual_seed(njobs)
+    ctx = xg.Context(0)
+    g = xg.Grid(ctx, nnu, nmu, 2.0, 25.0, 1.0, 1.0)
+    lhs = (-1e4 * (1.0 + torch.rand(nmu * nnu, generator=gen, dtype=torch.float64))).to(dev)
+    rhs = torch.randn(nmu * nnu, generator=gen, dtype=torch.float64).to(dev)
+    u0 = torch.zeros(nmu + 8, nnu + 8, dtype=torch.float64)
+    u0[4:nmu + 4, 4:nnu + 4] = torch.randn(nmu, nnu, generator=gen, dtype=torch.float64)
+
+    def relax(limit):
+        us = [u0.to(dev) for _ in range(njobs)]
+        jobs = [xg.Job(u=u.data_ptr(), lhs=lhs.data_ptr(), rhs=rhs.data_ptr(), omega=1.8, isym=1, kind=0) for u in us]
+        torch.cuda.synchronize()
+        ctx.set_wait_limit(limit)
+        xg.relax(ctx, g, jobs, 1, xg.SOR)
+        ctx.set_wait_limit(2.0)
+        return us
+
+    ref = relax(2.0)
+    ctx.synchronize()
+    cut = relax(1e-4)
+    with pytest.raises(xg.X2GError) as ei:
+        ctx.synchronize()
+    assert ei.value.code == 4, str(ei.value)
+    inner, middle = np.s_[5:nmu, 5:nnu + 3], np.s_[nmu // 2:nmu // 2 + 8, nnu // 2:nnu // 2 + 8]
+    for k, x in enumerate(cut):
+        x = x.cpu()
+        assert torch.equal(x[middle], ref[k].cpu()[middle]), k
+        assert not torch.equal(x[inner], ref[k].cpu()[inner]), k
+    again = relax(2.0)
+    ctx.synchronize()
+    for x, r in zip(again, ref):
+        assert torch.equal(x, r)
+    g.close()
+    ctx.close()

@@ -45,10 +45,6 @@
 
 namespace x2g {
 
-// most polls of one wait for a neighbour's halo values (each suspends for a
-// while by itself; a phase needs a few): then the error word is set, the
-// thread goes on and waits no more, and the call reports the timeout
-constexpr int kColPolls = 1 << 16;
 constexpr int kColGuard = 32;  // words before and after the band that idle lanes may read
 
 // Rows the arrays of a CTA hold after the band's first: every thread goes
@@ -85,6 +81,9 @@ ColKernel column_kernel_broad(int slots, bool sep);  // broad
 namespace {
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return unsigned(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void st_cta(unsigned addr, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ unsigned in_cta(unsigned addr, int rank) {
   unsigned a;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
@@ -95,9 +94,13 @@ __device__ __forceinline__ void push_halo(unsigned addr, float v, unsigned bar) 
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(addr), "f"(v), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ void expect_bytes(unsigned bar, unsigned bytes) {
-  asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes)
-               : "memory");
+// (negative: nothing)
+__device__ __forceinline__ void expect_bytes(unsigned bar, int bytes) {
+  asm volatile(
+      "{\n\t.reg .b64 t;\n\t.reg .pred p;\n\tsetp.ge.s32 p, %1, 0;\n\t"
+      "@p mbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(bar),
+      "r"(bytes)
+      : "memory");
 }
 __device__ __forceinline__ bool poll_bar(unsigned bar, unsigned parity) {
   unsigned ok;
@@ -107,10 +110,29 @@ __device__ __forceinline__ bool poll_bar(unsigned bar, unsigned parity) {
                : "memory");
   return ok != 0;
 }
-// false: it ran out
-__device__ __forceinline__ bool wait_halo(unsigned bar, unsigned parity) {
-  for (int k = 0; k < kColPolls; ++k)
+// the same without suspending
+__device__ __forceinline__ bool test_bar(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok)
+               : "r"(bar), "r"(parity)
+               : "memory");
+  return ok != 0;
+}
+// a wait for a neighbour's halo values, a few polls as a rule; false: it ran
+// out (now recorded), or another one did
+__device__ __forceinline__ bool wait_halo(unsigned bar, unsigned parity, const BarrierDev &b) {
+  if (test_bar(bar, parity)) return true;
+  unsigned long long t0 = 0;
+  for (unsigned k = 1; b.limit_ns != 0; ++k) {
     if (poll_bar(bar, parity)) return true;
+    if ((k & 15u) != 0) continue;
+    if (*(volatile int *)b.err) return false;
+    const unsigned long long now = globaltimer();
+    if (t0 == 0) t0 = now;
+    if (now - t0 >= b.limit_ns) break;
+  }
+  atomicCAS(b.err, 0, X2G_ERR_TIMEOUT);
   return false;
 }
 
@@ -224,7 +246,7 @@ __device__ __forceinline__ float col_value(const ColPlan &p, const ColThread &T,
 template <int kM, bool kSep, int kPitch, int kGroups, int kMinBlocks>
 __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
     k_columns(GridDev g, const __grid_constant__ ColPlan p, const __grid_constant__ JobTable jobs, int nsweeps,
-              int free, int *err) {
+              int free, BarrierDev limit) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const int C = p.size, rank = int(cl.block_rank());
@@ -245,6 +267,7 @@ __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
   float2 *const BL = reinterpret_cast<float2 *>(W + (kSep ? 0 : p.rows * kPitch));
   const int w_off = int(W - E);
   const bool in = col >= 5 && col <= nni + 2;  // the thread has a column
+  const int err0 = tid == 0 ? *(volatile int *)limit.err : 0;
   const int nu = in ? col - 4 : 1;
   for (int k = tid; k < ne; k += nt) smem[k] = 0.0f;
   for (int k = tid; k < p.rows; k += nt) {
@@ -298,9 +321,12 @@ __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
     }
   }
   // halo barriers: [side][phase parity], side 0 the values from the CTA before
-  // and the bytes that each colour's phase receives, [side][colour]
+  // and the bytes that each colour's phase receives, [side][colour]; failed: a
+  // wait has run out, of this block (or, before it began, elsewhere); skip: one
+  // of the cluster's blocks, which write it once they are through
   const unsigned bar0 = smem_addr(BL + p.rows);
   int *const s_bytes = reinterpret_cast<int *>(BL + p.rows) + 8;
+  volatile int *const failed = s_bytes + 10, *const skip = s_bytes + 11;
   const bool has_up = rank > 0, has_dn = rank < C - 1;
   // this thread's column at band row 0 in the neighbours' arrays
   const unsigned own = smem_addr(E + col);
@@ -308,6 +334,10 @@ __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
   const unsigned dn = has_dn ? in_cta(own, rank + 1) - unsigned(n * kPitch * 4) : 0u;
   const unsigned up_bar = has_up ? in_cta(bar0, rank - 1) + 16u : 0u;  // its side 1
   const unsigned dn_bar = has_dn ? in_cta(bar0, rank + 1) : 0u;
+  if (tid == 0) {
+    *failed = err0;
+    *skip = 0;
+  }
   if (tid < 4)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8u * tid) : "memory");
 #pragma unroll 1
@@ -327,8 +357,8 @@ __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
     const int na_ = __syncthreads_count(in && group == 0 && has_up && above > 0);
     const int nb_ = __syncthreads_count(in && group == 0 && has_dn && below > 0);
     if (tid == 0) {
-      s_bytes[c] = 4 * na_;
-      s_bytes[5 + c] = 4 * nb_;
+      s_bytes[c] = has_up ? 4 * na_ : -1;
+      s_bytes[5 + c] = has_dn ? 4 * nb_ : -1;
     }
   }
   ColThread T;
@@ -350,9 +380,11 @@ __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
   if (kSep) T.cs = T.src == lane ? 0.0f : T.src + 2 == lane ? T.wl[2] : T.wl[0];
   T.warp = warp;
   T.seam_warp = free ? -1 : (nnix - 7 + p.shift) / 32 + group * p.warps;
-  // arm both parities of a side for the values of the first two phases
+  // arm both parities of a side for the values of the first two phases.  After
+  // a failed wait (-1) the barrier's last turn may still be open, and one more
+  // arrival than it has room for faults; nothing waits for it any more
   auto arm = [&](int side, int c, int parity) {
-    if (side == 0 ? has_up : has_dn) expect_bytes(bar0 + unsigned(16 * side + 8 * parity), unsigned(s_bytes[5 * side + c]));
+    expect_bytes(bar0 + unsigned(16 * side + 8 * parity), *(volatile int *)(s_bytes + 5 * side + c));
   };
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
@@ -363,6 +395,10 @@ __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
   const bool push_up = has_up && group == 0, push_dn = has_dn && g1 == n;
   bool wait_up = push_up, wait_dn = push_dn;
   for (int s = 0; s < nsweeps; ++s) {
+    // only this block's waits write the flag, and none comes between the barrier
+    // before this and the next one, so its threads agree; it stays until the
+    // whole cluster is through
+    if (*failed) break;
     if (s > 0) {
       // axis of e for the band's rows; the mu=1 row is band row -1 of the
       // first CTA
@@ -381,10 +417,12 @@ __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
         // the neighbours' values of phase - 1
         const int use = (phase - 1) >> 1, parity = (phase - 1) & 1;
         bool ok = true;
-        if (wait_up) ok = wait_halo(bar0 + 8u * parity, use & 1);
-        if (wait_dn) ok = wait_halo(bar0 + 16u + 8u * parity, use & 1) && ok;
-        if (!ok) {
-          atomicCAS(err, 0, X2G_ERR_TIMEOUT);
+        if (wait_up) ok = wait_halo(bar0 + 8u * parity, use & 1, limit);
+        if (ok && wait_dn) ok = wait_halo(bar0 + 16u + 8u * parity, use & 1, limit);
+        if (!ok) {  // to the end of this sweep with the values that are there
+          *failed = 1;
+#pragma unroll 1
+          for (int k = 0; k < 10; ++k) *(volatile int *)(s_bytes + k) = -1;
           wait_up = wait_dn = false;
         }
       }
@@ -443,8 +481,17 @@ __global__ void __launch_bounds__(kPitch * kGroups, kMinBlocks)
       if (phase > 0 && tid < 2) arm(tid, (c + 1) % 5, (phase - 1) & 1);
     }
   }
+  if (tid < C && *failed) st_cta(in_cta(smem_addr(s_bytes + 11), tid), 1);
   cluster_arrive();
   cluster_wait();  // no CTA leaves while a neighbour may still write its halo
+  if (*skip) {
+    // u stays as it was.  Values pushed before the cluster's barrier and not
+    // waited for may be on their way into this CTA's memory for a microsecond:
+    // it is kept for a hundred
+    const unsigned long long t0 = globaltimer();
+    for (int k = 0; k < 1024 && globaltimer() - t0 < 100000; ++k) __nanosleep(1000);
+    return;
+  }
   // u += e on the band, then the FP64 axis of u for its rows (the mu=1 row
   // and the corners by the first CTA)
   double *const u = J.u;

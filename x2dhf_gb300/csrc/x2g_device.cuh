@@ -5,6 +5,12 @@
 
 namespace x2g {
 
+__device__ __forceinline__ unsigned long long globaltimer() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
 // double -> float with round to nearest even, on the integer pipes (GB300
 // issues conversion instructions on its narrow FP64 pipe); values beyond the
 // float range become infinities, values below its normal range signed zero

@@ -32,12 +32,6 @@ __device__ __forceinline__ T ldcg(const T *p) {
   return __ldcg(p);
 }
 
-__device__ __forceinline__ unsigned long long globaltimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 // Whether a wait that started at t0 has run out: checked every 256 spins,
 // or at every spin when the limit is 0 (a wait not met at once fails).
 __device__ __forceinline__ bool wait_expired(const BarrierDev &b, unsigned spins, unsigned long long t0) {
@@ -2712,8 +2706,8 @@ static int cluster_sweep(x2g_ctx *ctx, const GridDev &g, const ColChoice &c, Job
     plan.m2[k] = make_float2(g.dmu2f[k], g.dmu2f[k]);
   }
   plan.neg = make_float2(-1.0f, -1.0f);
-  int *err_word = reinterpret_cast<int *>(ctx->bar + 2);
-  void *args[] = {&gd, &plan, &jt, &nsweeps, &free, &err_word};
+  BarrierDev limit{ctx->bar, ctx->bar + 1, reinterpret_cast<int *>(ctx->bar + 2), ctx->wait_limit_ns};
+  void *args[] = {&gd, &plan, &jt, &nsweeps, &free, &limit};
   cudaError_t err = cudaLaunchKernelExC(&cfg, c.fn, args);
   if (err != cudaSuccess) return cuda_status(err, "cluster MCSOR launch");
   ctx->launches += 1;
