@@ -2936,7 +2936,7 @@ static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2
   return X2G_OK;
 }
 
-constexpr long kFixedPoints = 1 << 17;  // fewest points of a call whose residuals are taken in fixed point
+constexpr long kFixedPoints = 1 << 16;  // fewest points of a function whose residual alone is taken in fixed point
 
 // co-resident clusters of the cluster sweep and of its potentials' variant
 // for large batches on this grid on the context's device (0: that kernel
@@ -2979,10 +2979,14 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
     if (persistent_shape(ctx, g, want, &nj, &G1, &sm1) == X2G_OK && nj >= want) col = ColChoice();
     set_status(X2G_OK, "");
   }
-  // their stencil sums in fixed point, where there are tiles enough: 22 of
-  // 331x481 80 us (FMAs 149), 22 of 151x241 42 (54), one of 331x481 13 (14);
-  // one of 151x241 takes 9 (4).  The same for every sweep kernel and wave
-  const bool fixed = separable && long(njobs) * (g.nni - 2) * (g.nmu - 5) >= kFixedPoints;
+  // their stencil sums in fixed point with the potentials' kernel, and on grids
+  // that no on-chip kernel holds, where a function alone has tiles enough (22 of
+  // 331x481 80 us, FMAs 149; 22 of 151x241 42 and 54; one of 331x481 13 and 14).
+  // The kernel and the grid decide, not the number of jobs, so that a function's
+  // result does not depend on its batch, and the plain kernel's results (mode 0,
+  // SCFs in the reference's order) stay the persistent-band sweep's
+  const bool fixed = separable && ctx->pot_clusters != 0 &&
+                     (col.sep || (column_shapes(ctx, grid->h).empty() && long(g.nni - 2) * (g.nmu - 5) >= kFixedPoints));
   // per-job scratch: FP32 correction, residual and omega/lhs
   const size_t per_job =
       (size_t(g.next) * sizeof(float) + 2 * size_t(g.mxsize) * sizeof(float) + 256) / 256 * 256 + 256;
