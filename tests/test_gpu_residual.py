@@ -1,4 +1,8 @@
-"""FP64 residuals of the mixed form."""
+"""FP64 residuals of the mixed form, each point against its own terms.
+
+After one sweep the correction of a point that no other point of the first
+colour reaches is omega / lhs times its residual: u's change shows the residual
+to the last bits that u holds."""
 import numpy as np
 import pytest
 
@@ -14,6 +18,24 @@ def ctx():
     c = xg.Context(0)
     yield c
     c.close()
+
+
+def _first_points(nnu, nmu):
+    """Ext indices of the points that are relaxed before any of their neighbours."""
+    order, pts, tile, colour, level = xg.host_schedule(nnu, nmu)
+    return pts[(colour == 0) & (level == 0)]
+
+
+def _fields(nnu, nmu, rng):
+    row, col = np.arange(nmu)[:, None], np.arange(nnu)[None, :]
+    rand = lambda: rng.standard_normal((nmu, nnu))  # noqa: E731
+    spikes = rand() * (rng.random((nmu, nnu)) < 0.01)
+    return {"smooth": np.exp(-0.01 * row) * np.cos(0.01 * col), "random": rand(), "spikes": spikes,
+            # one value in a hundred far above the others: the ends of many stencils
+            "arms": spikes + 2.0 ** -14 * rand(),
+            "steep": np.exp(-0.43 * (row % 100)) * (1.0 + 0.1 * rand()),
+            "steeper": rand() * np.exp(-0.95 * (row % 50) - 0.5 * (col % 50)),
+            "axis": np.sin(np.pi * col / (nnu - 1)) ** 2 * np.exp(-0.02 * row)}
 
 
 def _extended(v, isym):
@@ -62,6 +84,56 @@ class Operator:
         psa = start.copy()
         psa[self.row, self.col] = (self.apply(u, idel)[0] / LD(self.g[self.ik])).astype(np.float64)
         return psa
+
+
+# potentials on chip (both row pitches), and a grid that takes the persistent-band sweep
+@pytest.mark.parametrize("nnu,nmu", [(91, 121), (361, 91), (811, 121)])
+@pytest.mark.parametrize("mode", [True, False], ids=["fixed", "fma"])
+def test_residual_of_every_point_in_terms_of_its_own(ctx, nnu, nmu, mode):
+    """18 roundings to 53 bits of sums that the absolute terms bound, an FP32
+    rounding of the residual, of omega / lhs (from two rounded terms and a fast
+    reciprocal, 2^-21) and of their product, and u's own last bit.  (A sum in
+    units of values a tile away, as a point left to it wrongly has, is off by
+    up to 2^-42 of its terms.)"""
+    torch = pytest.importorskip("torch")
+    g = xg.Grid(ctx, nnu, nmu, 2.0, 25.0, 1.0, 1.0)
+    dev, rng, omega = torch.device("cuda:0"), np.random.default_rng(nnu), 1.8
+    op = Operator(g, nnu, nmu, _first_points(nnu, nmu))
+    row, col = op.row, op.col
+    one = torch.ones((nmu + 8) * (nnu + 8), dtype=torch.float64, device=dev)
+    cases, jobs = [], []
+    for name, v in _fields(nnu, nmu, rng).items():
+        for idel, isym in ((0, 1), (1, -1), (2, 1)):
+            u = _extended(v, isym)
+            # near its solution, so that the residual is what the rounding leaves
+            psa = op.source(u, idel, np.zeros_like(u))
+            bare = u.copy()
+            bare[0:4], bare[4:nmu + 4, 0:4], bare[4:nmu + 4, nnu + 4:] = 0.0, 0.0, 0.0  # ghosts are not the caller's
+            du, dpsa = (torch.tensor(x.ravel(), device=dev) for x in (bare, psa))
+            cases.append((name, idel, u, psa, du, dpsa))
+            jobs.append(xg.Job(u=du.data_ptr(), psa=dpsa.data_ptr(), psb=one.data_ptr(), omega=omega, isym=isym, idel=idel,
+                               kind=1))
+    ctx.set_potential_clusters(mode)
+    torch.cuda.synchronize()
+    try:
+        xg.relax(ctx, g, jobs, 1, xg.MIXED)
+        ctx.synchronize()
+    finally:
+        ctx.set_potential_clusters("auto")
+    eps = LD(2.0) ** -53
+    for name, idel, u, psa, du, _ in cases:
+        lhs = LD(op.lhs(idel))
+        au, terms, parts = op.apply(u, idel)
+        rhs = LD(psa[row, col]) * LD(op.g[op.ik])
+        r, terms = rhs - au, terms + abs(rhs)
+        # and the weights: formed here and there from steps that differ in their last bit, with four roundings
+        off = 18 * eps * terms + 8 * eps * parts
+        want = omega * r / lhs
+        got = LD(du.cpu().numpy().reshape(u.shape)[row, col]) - LD(u[row, col])
+        bound = abs(omega / lhs) * off + LD(2.0) ** -20 * abs(want) + eps * (abs(LD(u[row, col])) + abs(want))
+        worst = float((abs(got - want) / (bound + LD(1e-300))).max())
+        assert worst <= 1, (name, idel, worst)
+    g.close()
 
 
 @pytest.mark.parametrize("nnu,nmu", [(151, 241), (331, 481)])

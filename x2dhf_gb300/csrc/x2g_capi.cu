@@ -344,9 +344,10 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
       cnu[nu * 8 + q] = h.dni2[q] + h.d_nu[nu] * h.dni1[q];
       cnu[nu * 8 + 4 + q] = h.dni2[q] - h.d_nu[nu] * h.dni1[q];
     }
-  // no weight above 2^57 and no point's weights above 2^60 together
+  // the potentials' weights as whole numbers: none above 2^57, no point's above
+  // 2^60 together
   double most = 0.0, mu_sum = 0.0, nu_sum = 0.0;
-  for (const auto *v : {&cmo, &cmp, &cnu})
+  for (const auto *v : {&cmp, &cnu})
     for (size_t k = 8; k < v->size() - 8; k += 8) {  // the axes have no points
       double sum = 0.0;
       for (size_t q = k; q < k + 8; ++q) {
@@ -357,6 +358,7 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
       to = std::max(to, sum);
     }
   d.wscale = std::min(57 - (std::ilogb(most) + 1), 60 - (std::ilogb(mu_sum + nu_sum) + 1));
+  d.near = std::ilogb(h.diag) - (57 - d.wscale) + 4;
   auto fixed = [&](const std::vector<double> &v) {
     std::vector<int2> w(v.size());
     for (size_t k = 8; k < v.size() - 8; ++k) {
@@ -439,8 +441,7 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
   UP(cmo, cmu_orb);
   UP(cmp, cmu_pot);
   UP(cnu, cnu);
-  const std::vector<int2> fixed_mo = fixed(cmo), fixed_mp = fixed(cmp), fixed_nu = fixed(cnu);
-  UP(fixed_mo, wmu_orb);
+  const std::vector<int2> fixed_mp = fixed(cmp), fixed_nu = fixed(cnu);
   UP(fixed_mp, wmu_pot);
   UP(fixed_nu, wnu);
   UP(place, st_place);

@@ -193,8 +193,12 @@ struct GridDev {
   const double *cmu_orb, *cmu_pot, *cnu;
   // the same as fixed-point numbers w 2^wscale = .x 2^29 + .y with |.x| <=
   // 2^28, |.y| <= 2^28, and the place of interior point (mu, nu) in st_pts
-  const int2 *wmu_orb, *wmu_pot, *wnu;
+  // (potentials)
+  const int2 *wmu_pot, *wnu;
   int wscale;
+  // a value of u whose exponent is at most this far below its tile's largest
+  // makes lhs u at least 2^-4 of the largest weight times that value
+  int near;
   const int *st_place;
   // per-grid moment tables (built on the device at grid creation):
   // exm[(idel * 8 + q) * mxsize + k] = wgt2 f4 P_{q+1}^idel(cos th) (r2 r)^(q+1)

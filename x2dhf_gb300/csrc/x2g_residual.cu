@@ -8,23 +8,57 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// Mixed form residual r = rhs - A u in FP64 over the interior, stored as
-// FP32 with omega / lhs; the stencil uses the grid's separable weights (one
-// FMA per neighbour) and reads the ghost cells as mirrored interior values,
-// so u needs no ghost refresh first.  kPacked: the points are taken in
-// st_pts order and stored as (r, w) pairs in that order (persistent-band
-// sweep);
-// otherwise r32 / w32 are plain nni x nmu arrays (cluster sweep; need_w 0:
-// the potentials' cluster sweep forms omega / lhs itself, only r32 is
-// stored).
+// r = rhs - A u of an interior point in FP64, and its lhs; the stencil uses the
+// grid's separable weights (one FMA per neighbour) and reads the ghost cells as
+// mirrored interior values, so u needs no ghost refresh first
+__device__ __forceinline__ double residual_at(const GridDev &g, const JobDev &J, int mu, int nu, double &lhs) {
+  const int n8 = g.n8, ik = mu * g.nni + nu, ij = (mu + 4) * n8 + nu + 4;
+  const double *u = J.u;
+  double rhs;
+  if (J.kind == 1) {
+    rhs = (J.psa[ij] * J.psb[ij]) * g.g[ik];
+    lhs = (J.idel2 == 0.0) ? g.f3_mu[mu] : fma(J.idel2, g.e[ik], g.f3_mu[mu]);
+  } else {
+    rhs = J.rhs[ik];
+    lhs = J.lhs[ik];
+  }
+  const double *cm = (J.kind == 0 ? g.cmu_orb : g.cmu_pot) + mu * 8, *cn = g.cnu + nu * 8;
+  double cc = lhs * u[ij];
+  if (mu >= 4 && nu >= 4 && nu <= g.nni - 5) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int dm = (4 - q) * n8, dn = 4 - q;
+      cc = fma(cm[q], u[ij - dm], cc);
+      cc = fma(cm[4 + q], u[ij + dm], cc);
+      cc = fma(cn[q], u[ij - dn], cc);
+      cc = fma(cn[4 + q], u[ij + dn], cc);
+    }
+  } else {
+    // the stencil reaches the putin ghosts
+    const int row = mu + 4, col = nu + 4;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int d = 4 - q;
+      cc = fma(cm[q], ghost_read(g, u, row - d, col, J.isym), cc);
+      cc = fma(cm[4 + q], u[ij + d * n8], cc);
+      cc = fma(cn[q], ghost_read(g, u, row, col - d, J.isym), cc);
+      cc = fma(cn[4 + q], ghost_read(g, u, row, col + d, J.isym), cc);
+    }
+  }
+  return rhs - cc;
+}
+
+// Mixed form residual over the interior, stored as FP32 with omega / lhs.
+// kPacked: the points are taken in st_pts order and stored as (r, w) pairs in
+// that order (persistent-band sweep); otherwise r32 / w32 are plain nni x nmu
+// arrays (cluster sweep; need_w 0: the potentials' cluster sweep forms omega /
+// lhs itself, only r32 is stored).
 template <bool kPacked>
 __global__ void k_residual(GridDev g, const __grid_constant__ JobTable jobs, int zero_e, int need_w) {
   const JobDev &J = jobs.j[blockIdx.y];
   const int nint = (g.nni - 2) * (g.nmu - 5);
-  const int n8 = g.n8;
   if (zero_e)
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < g.next; k += gridDim.x * blockDim.x) J.e32[k] = 0.0f;
-  const double *cmu = (J.kind == 0) ? g.cmu_orb : g.cmu_pot;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nint; k += gridDim.x * blockDim.x) {
     int mu, nu;
     if (kPacked) {
@@ -35,44 +69,13 @@ __global__ void k_residual(GridDev g, const __grid_constant__ JobTable jobs, int
       mu = 1 + k / (g.nni - 2);
       nu = 1 + k % (g.nni - 2);
     }
-    const int ik = mu * g.nni + nu, ij = (mu + 4) * n8 + nu + 4;
-    const double *u = J.u;
-    double rhs, lhs;
-    if (J.kind == 1) {
-      rhs = (J.psa[ij] * J.psb[ij]) * g.g[ik];
-      lhs = (J.idel2 == 0.0) ? g.f3_mu[mu] : fma(J.idel2, g.e[ik], g.f3_mu[mu]);
-    } else {
-      rhs = J.rhs[ik];
-      lhs = J.lhs[ik];
-    }
-    const double *cm = cmu + mu * 8, *cn = g.cnu + nu * 8;
-    double cc = lhs * u[ij];
-    if (mu >= 4 && nu >= 4 && nu <= g.nni - 5) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int dm = (4 - q) * n8, dn = 4 - q;
-        cc = fma(cm[q], u[ij - dm], cc);
-        cc = fma(cm[4 + q], u[ij + dm], cc);
-        cc = fma(cn[q], u[ij - dn], cc);
-        cc = fma(cn[4 + q], u[ij + dn], cc);
-      }
-    } else {
-      // the stencil reaches the putin ghosts: read them as mirrored interior
-      // values
-      const int row = mu + 4, col = nu + 4;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int d = 4 - q;
-        cc = fma(cm[q], ghost_read(g, u, row - d, col, J.isym), cc);
-        cc = fma(cm[4 + q], u[ij + d * n8], cc);
-        cc = fma(cn[q], ghost_read(g, u, row, col - d, J.isym), cc);
-        cc = fma(cn[4 + q], ghost_read(g, u, row, col + d, J.isym), cc);
-      }
-    }
+    double lhs;
+    const double r = residual_at(g, J, mu, nu, lhs);
     if (kPacked) {
-      J.rw[k] = make_float2(narrow_f64(rhs - cc), J.omegaf / narrow_f64(lhs));
+      J.rw[k] = make_float2(narrow_f64(r), J.omegaf / narrow_f64(lhs));
     } else {
-      J.r32[ik] = narrow_f64(rhs - cc);
+      const int ik = mu * g.nni + nu;
+      J.r32[ik] = narrow_f64(r);
       if (need_w) J.w32[ik] = J.omegaf / narrow_f64(lhs);
     }
   }
@@ -93,16 +96,23 @@ __global__ void k_residual(GridDev g, const __grid_constant__ JobTable jobs, int
 // nearest: truncated values shift the sums by a constant sign, and SCFs then
 // stall at their noise floor.
 //
-// A point's sum is as accurate as FMAs if its stencil reaches a value within
-// 2^-5 of the tile's largest: the point and the four at the ends of its arms
-// are looked at, and points without one (about one row of 32 in 25 of the
-// potentials of N2), tiles at the ends of the exponent range and values that do
-// not fit the units are summed by FMAs.
+// All of this is in units of the tile's largest value and of the grid's largest
+// weight, W (about 2^-58 of their product in all), where the FMAs round to 53
+// bits of what a point's own terms come to.  So a point keeps the sum where its
+// term lhs u alone is within 2^-4 of W times the tile's largest value (|lhs| is
+// never below the diagonal's, so that u's exponent tells): there the error is no
+// larger than the FMAs', root mean square and worst, in terms of the point's
+// largest product (smooth potentials 4.7e-17 and 2e-16 against 1.8e-16 and
+// 9e-16, points at the limit 9e-17 against 1.8e-16).  The others, values that do
+// not fit the units, and tiles at the ends of the exponent range are collected
+// and summed by FMAs, 32 at a time, the same as k_residual's bits (smooth
+// potentials of sigma pairs: none; of pi pairs, small near the axis, 4 % of the
+// points of 331 x 481 and 15 % of 151 x 241, that lie in 20 and 44 % of a warp's
+// rows).
 //
-// What bounds it: instruction issue, about 300 a point of which 96 are the
-// products (two instructions each); the FP64 pipe is 40 % busy with the four
-// operations left.  8 rows per warp share the column's weights and its values;
-// 22 potentials of 331 x 481: 80 us, with FMAs 149.
+// What bounds it: its warps wait for the tile and the orbitals, then for the
+// products, about 300 instructions a point of which 96 are the products (two
+// each); 8 rows per warp share the column's weights and its values.
 constexpr int kTile = 32;           // columns and rows of a block's tile
 constexpr int kSpan = kTile + 8;    // with the stencil's four on each side
 constexpr int kRowsPerWarp = 8;
@@ -110,7 +120,6 @@ constexpr int kThreadsRes = kTile / kRowsPerWarp * 32;
 constexpr int kBlocksRes = 5;
 constexpr int kWarpSpan = kSpan / (kThreadsRes / 32);        // rows of the tile that a warp loads
 constexpr int kValues = kWarpSpan + (kWarpSpan + 3) / 4;  // values that a thread loads
-constexpr int kNear = 5;  // a value whose exponent is at most this far below the tile's largest is near it
 
 // x 2^(1081 - top), rounded, as .x 2^29 + .y with |.x| <= 2^30, |.y| <= 2^28;
 // top: the largest exponent field of the tile; flip: sign bit to change
@@ -158,19 +167,9 @@ struct Acc {
   }
 };
 
-// the stencil's neighbours at a point, by FMAs
-__device__ __noinline__ double stencil64(const GridDev &g, const double *u, const double *cm, const double *cn, int row,
-                                         int col, int isym) {
-  double cc = 0.0;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int d = 4 - q;
-    cc = fma(cm[q], ghost_read(g, u, row - d, col, isym), cc);
-    cc = fma(cm[4 + q], u[(row + d) * g.n8 + col], cc);
-    cc = fma(cn[q], ghost_read(g, u, row, col - d, isym), cc);
-    cc = fma(cn[4 + q], ghost_read(g, u, row, col + d, isym), cc);
-  }
-  return cc;
+__device__ __noinline__ float residual_fma(const GridDev &g, const JobDev &J, int mu, int nu) {
+  double lhs;
+  return narrow_f64(residual_at(g, J, mu, nu, lhs));
 }
 
 // x at a byte offset: one 32-bit offset serves arrays of one layout
@@ -185,8 +184,9 @@ __global__ void __launch_bounds__(kThreadsRes, kBlocksRes)
   const JobDev &J = jobs.j[blockIdx.y];
   __shared__ int2 tile[kSpan * kSpan];
   __shared__ int4 s_wmu[kTile * 4];
-  __shared__ unsigned s_near[kSpan], s_ends[kSpan];
+  __shared__ unsigned s_near[kSpan];
   __shared__ int s_top[kThreadsRes / 32];
+  __shared__ unsigned char s_rest[kThreadsRes / 32][kRowsPerWarp * 32];  // a warp's points that are left to FMAs
   const int tid = int(threadIdx.x), lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int down = int(blockIdx.x) / across;
   const int mu0 = down * kTile + 1, nu0 = (int(blockIdx.x) - down * across) * kTile + 1;
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kThreadsRes, kBlocksRes)
   // out of reach of the fixed point's exponents: infinities, NaNs and tiles
   // at the ends of the range go point by point
   const bool far = top < 256 || top > 1792;
-  const int low = far ? 0x7fffffff : (top - kNear) << 20;
+  const int low = far ? 0x7fffffff : (top - g.near) << 20;
   unsigned near = 0, edge = 0;
 #pragma unroll
   for (int q = 0; q < kValues; ++q) {
@@ -273,17 +273,11 @@ __global__ void __launch_bounds__(kThreadsRes, kBlocksRes)
     else
       edge = (lane >> 2) == q - kWarpSpan ? w >> 8 * (lane & 3) & 0xffu : edge;
   }
-  // lane i's row of the tile: near values in columns 4..35, and in 0..31 or 8..39
-  if (lane < kWarpSpan) {
-    s_near[warp * kWarpSpan + lane] = __funnelshift_r(near, edge, 4);
-    s_ends[warp * kWarpSpan + lane] = near | __funnelshift_r(near, edge, 8);
-  }
+  // lane i's row of the tile: near values in columns 4..35
+  if (lane < kWarpSpan) s_near[warp * kWarpSpan + lane] = __funnelshift_r(near, edge, 4);
   __syncthreads();
   if (rows <= 0) return;
-  // lane q's row of points: whether the point, or one four rows or columns from
-  // it, is near the tile's largest (otherwise its values have too few bits)
-  const int first = warp * kRowsPerWarp + (lane & (kRowsPerWarp - 1));
-  const unsigned fit = s_near[first] | s_near[first + 4] | s_near[first + 8] | s_ends[first + 4];
+  int left = 0;
   int2 wn[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) wn[q] = at(g.wnu, unsigned(nuc * 64 + q * 8));
@@ -308,19 +302,29 @@ __global__ void __launch_bounds__(kThreadsRes, kBlocksRes)
     }
     const long long sum = s.a + ((s.b + (1ll << 28)) >> 29);
     float r = from_units(to_units(rest[q], unit) - sum, unit);
-    // what does not fit the tile's units is large
+    if (zero) r = narrow_f64(rest[q]);
+    // rest beyond the tile's units
     const bool large = ((unsigned(__double2hiint(rest[q])) >> 20) & 0x7ffu) > unsigned(unit + 8);
-    if (!(__shfl_sync(0xffffffffu, fit, q) >> lane & 1u) || large) {
-      const int mu = mu1 + min(q, rows - 1);
-      r = narrow_f64(zero ? rest[q]
-                          : rest[q] - stencil64(g, u, g.cmu_pot + mu * 8, g.cnu + nuc * 8, mu + 4, nuc + 4, isym));
+    const bool keep = zero || ((s_near[warp * kRowsPerWarp + q + 4] >> lane & 1u) != 0 && !large), on = in && q < rows;
+    const unsigned others = __ballot_sync(0xffffffffu, on && !keep);
+    if (others >> lane & 1u) s_rest[warp][left + __popc(others & ((1u << lane) - 1))] = (unsigned char)(q * 32 + lane);
+    left += __popc(others);
+    if (kPacked) {
+      float2 *const to = J.rw + __ldg(g.st_place + (mu1 + min(q, rows - 1) - 1) * (nni - 2) + nuc - 1);
+      if (on && keep) *to = make_float2(r, w32[q]);
+      if (on && !keep) to->y = w32[q];
+    } else if (on && keep) {
+      J.r32[(mu1 + q) * nni + nu] = r;
     }
-    if (in && q < rows) {
-      if (kPacked)
-        J.rw[__ldg(g.st_place + (mu1 + q - 1) * (nni - 2) + nu - 1)] = make_float2(r, w32[q]);
-      else
-        J.r32[(mu1 + q) * nni + nu] = r;
-    }
+  }
+  __syncwarp();
+  for (int k = lane; k < left; k += 32) {
+    const int id = s_rest[warp][k], mu = mu1 + id / 32, at_nu = nu0 + id % 32;
+    const float r = residual_fma(g, J, mu, at_nu);
+    if (kPacked)
+      J.rw[__ldg(g.st_place + (mu - 1) * (nni - 2) + at_nu - 1)].x = r;
+    else
+      J.r32[mu * nni + at_nu] = r;
   }
 }
 
