@@ -119,7 +119,17 @@ int x2g_host_schedule(int nnu, int nmu, int *npoints, int *ntiles, int *nlevels,
  * mixed form cuts the grid by columns and rows of its own and picks the cluster
  * size per batch; this plan and its chunk lists serve inspection and tests. */
 int x2g_host_cluster_plan(int nnu, int nmu, int *csize, int *maxrows, long *smem, int *row0);
-/* Chunk lists of that plan (host only): chunks of up to 4 points of
+/* Band plan of the on-chip sweep for clusters of csize CTAs with `groups`
+ * threads per column (no CUDA call; X2G_ERR_SCHEDULE: the grid has none): the
+ * most points of one colour in a thread's rows, rows of the largest band, band
+ * starts row0[csize + 1] (ext rows from 5) and the row cut[k] of band k where
+ * the second thread's rows begin; and the kernel that runs it for other
+ * functions (potentials 0) or potentials built from orbitals (1; 2: two CTAs
+ * per SM): its slots (0: none does), the rows its arrays hold and its shared
+ * memory per CTA.  No reference counterpart. */
+int x2g_host_column_plan(int nnu, int nmu, int csize, int groups, int potentials, int *slots, int *maxrows, int *row0,
+                         int *cut, int *kernel_slots, int *kernel_rows, long *smem);
+/* Chunk lists of x2g_host_cluster_plan's plan (host only): chunks of up to 4 points of
  * one row at stride 5, packed (band row << 19) | (ext col << 2) | (count-1),
  * and the offsets of each CTA's 5 colours x (levels + 2) segments (level 0
  * off the shared band edges, level 0 near them, level-0 seam points, levels

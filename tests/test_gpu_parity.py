@@ -954,3 +954,14 @@ def test_large_band_blocks_match_single_jobs(ctx, njobs, nsweeps):
     for k, (x, y, u) in enumerate(zip(together, alone, u0)):
         assert torch.equal(x, y) and not torch.equal(x, u), k
     g.close()
+
+
+# grids of few columns and many rows (more points of a colour per thread, three row pitches) and of many columns and few
+# rows (25 warps)
+@pytest.mark.parametrize("nnu,nmu", [(241, 901), (271, 811), (151, 1201), (121, 1831), (91, 2431), (541, 31), (781, 31)])
+def test_tall_and_flat_grids_run_on_chip(ctx, nnu, nmu):
+    torch = pytest.importorskip("torch")
+    g = xg.Grid(ctx, nnu, nmu, 2.0, 25.0, 1.0, 1.0)
+    assert min(g.cluster_occupancy()) > 0
+    g.close()
+    test_column_sweep_matches_band_sweep(ctx, nnu, nmu, 2, 3)

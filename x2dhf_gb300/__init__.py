@@ -76,7 +76,7 @@ EXPORTS = [
     "tpoolStop4mcsor_", "tpoolStop4pots_", "x2g_host_table", "x2g_host_schedule", "x2g_profile",
     "x2g_relax_noalloc", "x2g_host_cluster_plan", "x2g_set_mixed_on_chip", "x2g_set_potential_clusters", "x2g_cluster_occupancy",
     "x2g_set_mixed_colouring", "x2g_set_residual_overlap", "x2g_set_gram_orthonormalise",
-    "x2g_host_cluster_chunks", "x2g_host_free_chunks", "x2g_host_band_schedule",
+    "x2g_host_column_plan", "x2g_host_cluster_chunks", "x2g_host_free_chunks", "x2g_host_band_schedule",
     "x2g_convert_selftest", "x2g_set_wait_limit", "x2g_host_sor_schedule",
 ]
 
@@ -135,6 +135,7 @@ def lib():
     L.x2g_profile.argtypes = [P, I, I, dp, dp, C.POINTER(C.c_long)]
     L.x2g_host_cluster_plan.argtypes = [I, I, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_long),
                                         C.POINTER(C.c_int)]
+    L.x2g_host_column_plan.argtypes = [I] * 5 + [C.POINTER(C.c_int)] * 6 + [C.POINTER(C.c_long)]
     L.x2g_set_mixed_on_chip.argtypes = [P, I]
     L.x2g_set_potential_clusters.argtypes = [P, I]
     L.x2g_set_mixed_colouring.argtypes = [P, I]
@@ -392,6 +393,20 @@ def host_cluster_chunks(nnu, nmu, colouring="reference"):
     _check(f(nnu, nmu, C.byref(nc), C.byref(no), ch.ctypes.data_as(C.POINTER(C.c_int)),
              off.ctypes.data_as(C.POINTER(C.c_int))))
     return ch.view(np.uint32), off
+
+
+def host_column_plan(nnu, nmu, csize, groups, potentials=0):
+    """Band plan of the on-chip sweep for clusters of csize CTAs and `groups`
+    threads per column, and the kernel that runs it (no GPU needed); None if
+    the grid has no such plan."""
+    L = lib()
+    s, m, ks, kr = (C.c_int() for _ in range(4))
+    row0, cut, smem = (C.c_int * (csize + 1))(), (C.c_int * csize)(), C.c_long()
+    if L.x2g_host_column_plan(nnu, nmu, csize, groups, potentials, C.byref(s), C.byref(m), row0, cut, C.byref(ks),
+                              C.byref(kr), C.byref(smem)):
+        return None
+    return dict(slots=s.value, maxrows=m.value, row0=list(row0), cut=list(cut), kernel_slots=ks.value,
+                kernel_rows=kr.value, smem=smem.value)
 
 
 def host_cluster_plan(nnu, nmu):

@@ -68,7 +68,7 @@ inline size_t column_smem(int rows, int pitch, bool sep, int threads) {
 // The instantiations, by the most points of a colour in a column (null: none
 // holds that many).  kPitch...: their row pitch and most threads of a group;
 // pair: two CTAs per SM.
-constexpr int kPitchNarrow = 352, kPitchWide = 512, kPitchBroad = 544;
+constexpr int kPitchThin = 160, kPitchSlim = 256, kPitchNarrow = 352, kPitchWide = 512, kPitchBroad = 544, kPitchFlat = 800;
 struct ColKernel {
   const void *fn;
   int slots;
@@ -77,6 +77,39 @@ ColKernel column_kernel_split(int slots, bool sep);  // narrow, two threads per 
 ColKernel column_kernel_pair(int slots, bool sep);   // narrow, two CTAs per SM (sep only)
 ColKernel column_kernel_wide(int slots, bool sep);   // wide
 ColKernel column_kernel_broad(int slots, bool sep);  // broad
+ColKernel column_kernel_slim(int slots, bool sep);   // tall grids of few columns, two threads per column
+ColKernel column_kernel_thin(int slots, bool sep);   // the same, of fewer still
+ColKernel column_kernel_flat(int slots, bool sep);   // many columns, few rows
+// The instantiation for a plan whose columns need a pitch of `need` (pair: two
+// CTAs per SM), and its pitch.
+inline ColKernel column_kernel(const ColPlan &p, bool sep, bool pair, int need, int &pitch) {
+  pitch = kPitchNarrow;
+  if (pair) return p.groups == 1 && need <= pitch ? column_kernel_pair(p.slots, sep) : ColKernel{nullptr, 0};
+  if (need <= kPitchNarrow) {
+    if (p.groups != 2) return {nullptr, 0};
+    // five slots reach 800 rows; beyond, the largest cluster takes more of them
+    // (one orbital of 151 x 811 89 us, in the persistent bands 238; 241 x 901 114
+    // and 253, 271 x 811 126 and 251)
+    if (p.slots <= 5) return column_kernel_split(p.slots, sep);
+    if (p.size != kMaxCluster) return {nullptr, 0};
+    if (need <= kPitchThin && p.slots > 10) {
+      pitch = kPitchThin;
+      return column_kernel_thin(p.slots, sep);
+    }
+    if (need <= kPitchSlim) {
+      pitch = kPitchSlim;
+      return column_kernel_slim(p.slots, sep);
+    }
+    return column_kernel_split(p.slots, sep);
+  }
+  if (p.groups != 1) return {nullptr, 0};
+  // 541 x 31: 93 us, in the persistent bands 252
+  pitch = need <= kPitchWide ? kPitchWide : need <= kPitchBroad ? kPitchBroad : kPitchFlat;
+  if (need > pitch) return {nullptr, 0};
+  return pitch == kPitchWide    ? column_kernel_wide(p.slots, sep)
+         : pitch == kPitchBroad ? column_kernel_broad(p.slots, sep)
+                                : column_kernel_flat(p.slots, sep);
+}
 
 namespace {
 

@@ -12,6 +12,8 @@ ColKernel column_kernel_split(int slots, bool sep) {
   if (!sep && slots <= 4) return {(const void *)k_columns<4, false, 352, 2, 1>, 4};
   if (sep && slots <= 5) return {(const void *)k_columns<5, true, 352, 2, 1>, 5};
   if (!sep && slots <= 5) return {(const void *)k_columns<5, false, 352, 2, 1>, 5};
+  if (sep && slots <= 6) return {(const void *)k_columns<6, true, 352, 2, 1>, 6};
+  if (!sep && slots <= 6) return {(const void *)k_columns<6, false, 352, 2, 1>, 6};
   return {nullptr, slots};
 }
 

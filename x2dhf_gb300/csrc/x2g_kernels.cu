@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "x2g_columns.cuh"
+#include "x2g_columns_plan.h"
 #include "x2g_pairs.cuh"
 
 namespace x2g {
@@ -2545,15 +2546,9 @@ static const std::vector<x2g_ctx::ColumnShape> &column_shapes(x2g_ctx *ctx, cons
   for (size_t i = 0; i < h.columns.size(); ++i)
     for (int kind = 0; kind < 3; ++kind) {
       const ColPlan &p = h.columns[i];
-      const int need = std::max(p.pitch, p.warps * 32);
-      const int pitch = need <= kPitchNarrow ? kPitchNarrow : need <= kPitchWide ? kPitchWide : kPitchBroad;
-      // up to 11 warps in a row: two threads per column, or two CTAs per SM
-      if (need > pitch || p.groups != (pitch == kPitchNarrow && kind != 2 ? 2 : 1)) continue;
-      if (kind == 2 && pitch != kPitchNarrow) continue;
-      const ColKernel k = kind == 2               ? column_kernel_pair(p.slots, true)
-                          : pitch == kPitchNarrow ? column_kernel_split(p.slots, kind == 1)
-                          : pitch == kPitchWide   ? column_kernel_wide(p.slots, kind == 1)
-                                                  : column_kernel_broad(p.slots, kind == 1);
+      int pitch = 0;
+      const ColKernel k = column_kernel(p, kind > 0, kind == 2, std::max(p.pitch, p.warps * 32), pitch);
+      if (!k.fn) continue;
       x2g_ctx::ColumnShape c{int(i), k.fn, kind > 0, column_rows(p, k.slots), 0, 0};
       c.smem = column_smem(c.rows, pitch, c.sep, p.warps * p.groups * 32);
       c.active = cluster_active(ctx, c.fn, p.size, p.warps * p.groups * 32, c.smem);
@@ -3431,3 +3426,23 @@ void launch_moments(x2g_ctx *ctx, const GridDev &g, const MomentItem *items, int
 
 
 }  // namespace x2g
+
+extern "C" int x2g_host_column_plan(int nnu, int nmu, int csize, int groups, int potentials, int *slots, int *maxrows,
+                                    int *row0, int *cut, int *kernel_slots, int *kernel_rows, long *smem) {
+  using namespace x2g;
+  ColPlan p;
+  if (potentials < 0 || potentials > 2 || (groups != 1 && groups != 2) || nnu < 31 || nmu < 31 ||
+      !column_plan(nnu, nmu, csize, groups, p))
+    return set_status(X2G_ERR_SCHEDULE, "no such band plan");
+  int pitch = 0;
+  const ColKernel k = column_kernel(p, potentials > 0, potentials == 2, std::max(p.pitch, p.warps * 32), pitch);
+  if (slots) *slots = p.slots;
+  if (maxrows) *maxrows = p.maxrows;
+  if (row0) std::copy(p.row0, p.row0 + csize + 1, row0);
+  if (cut) std::copy(p.cut, p.cut + csize, cut);
+  const int rows = k.fn ? column_rows(p, k.slots) : 0;
+  if (kernel_slots) *kernel_slots = k.fn ? k.slots : 0;
+  if (kernel_rows) *kernel_rows = rows;
+  if (smem) *smem = k.fn ? long(column_smem(rows, pitch, potentials > 0, p.warps * p.groups * 32)) : 0;
+  return set_status(X2G_OK, "");
+}
