@@ -22,12 +22,6 @@ constexpr int kMaxLevels = 8;
 // sweep's per-block phase counts from word kPhaseWords (kPhaseBlocks, one
 // 128-byte line each)
 constexpr int kMomentTickets = 288;
-// most warps per CTA of the potentials' cluster variant (two CTAs per SM:
-// the register file holds 2 x 32 x warps threads at <= 65536 / that
-// registers each): 16 with the reference colouring (measured faster than 20
-// at 48 registers), 20 with the seam-free one, whose two segments then take
-// every chunk of a colour in one pass
-constexpr int kPotWarpsRef = 16, kPotWarpsFree = 20;
 constexpr int kPhaseWords = 352, kPhaseBlocks = 320, kPhaseStride = 32;
 constexpr int kBarWords = kPhaseWords + kPhaseBlocks * kPhaseStride;
 
@@ -95,30 +89,6 @@ struct HostGrid {
   std::vector<int> tile_row0, tile_row1;
   std::vector<int> pts;  // ext indices grouped [tile][colour][level]
   std::vector<int> off;  // (ntiles*5*nlev + 1) offsets into pts
-  std::vector<int> pts_rc;  // same points as (ext row << 16) | ext col
-  // plan of whole tiles for one cluster per job (host only, for inspection;
-  // the on-chip sweep's are in columns): cl_size CTAs per job, CTA k owns
-  // tiles [cl_tile0[k], cl_tile0[k+1]) = ext rows [cl_row0[k], cl_row0[k+1])
-  int cl_size = 0, cl_maxrows = 0, cl_maxchunks = 0, cl_wa = 1, cl_wb = 1, cl_ws = 1;
-  // warps per role of the potentials' variant (two CTAs per SM, at most kPotWarpsRef)
-  int cl_pa = 1, cl_pb = 1, cl_ps = 1;
-  // the same CTA bands with the seam-free colouring of the mixed form,
-  // colour (col - row) mod 5 in ext coordinates (no two points of a colour
-  // within 4 rows or columns of each other on the stencil's cross): per
-  // (CTA, colour) the segments A (off the shared band edges), B (within 4
-  // rows of one) and an empty seam segment, chunks packed as in cl_pts
-  int cf_maxchunks = 0, cf_wa = 1, cf_wb = 1, cf_ws = 0, cf_pa = 1, cf_pb = 1, cf_ps = 0;
-  std::vector<int> cf_pts, cf_off;
-  size_t cl_smem = 0;
-  std::vector<int> cl_tile0, cl_row0;
-  // the CTAs' points regrouped [cta][colour][segment] as chunks of up to 4
-  // points of one row at stride 5, packed (band row << 19) | (col << 2) |
-  // (count - 1); segments: level-0 points off the band edges, level-0 points
-  // within 4 rows of an edge shared with another CTA, level-0 seam points
-  // (same-colour neighbours of higher levels), then levels 1..nlev-1; cl_off
-  // has cl_size * 5 * (nlev + 2) + 1 chunk offsets; cl_wa/wb/ws warps per
-  // CTA work on the three kinds
-  std::vector<int> cl_pts, cl_off;
   // persistent-band FP32 sweep of grids beyond one cluster: the same points
   // regrouped [colour][level][tile] (st_pts, packed (ext row << 16) | ext
   // col), so that the points of one colour and level in any run of

@@ -188,82 +188,6 @@ void build_march(HostGrid &g) {
 
 }  // namespace
 
-// Chunks of one segment appended to `chunks`: the segment's points (ext
-// row, col) of one CTA band starting at ext row r0 grouped into runs of up to
-// 4 points of one row at stride 5, packed (band row << 19) | (col << 2) |
-// (count - 1), and dealt round-robin over buckets of the shared-memory bank
-// of their first correction value, so that a warp's 32 chunks start on
-// distinct banks where the buckets allow.
-static void append_chunks(std::vector<std::pair<int, int>> &pts, int r0, int n8, std::vector<int> &chunks) {
-  std::sort(pts.begin(), pts.end());
-  std::vector<std::vector<int>> bank(32);
-  for (size_t i = 0; i < pts.size();) {
-    size_t n = 1;
-    while (n < 4 && i + n < pts.size() && pts[i + n].first == pts[i].first &&
-           pts[i + n].second == pts[i + n - 1].second + 5)
-      ++n;
-    const int lr = pts[i].first - r0;
-    bank[((lr + 4) * n8 + pts[i].second) % 32].push_back(
-        int((unsigned(lr) << 19) | (unsigned(pts[i].second) << 2) | unsigned(n - 1)));
-    i += n;
-  }
-  for (size_t depth = 0, left = 1; left;) {
-    left = 0;
-    for (auto &bk : bank)
-      if (depth < bk.size()) {
-        chunks.push_back(bk[depth]);
-        left = 1;
-      }
-    ++depth;
-  }
-}
-
-// Seam-free colouring of the mixed form's cluster sweep on the CTA bands r0:
-// colour (col - row) mod 5 of the ext point, so the stencil's neighbours at
-// distance 1..4 along a row or a column always have another colour and the
-// points of one colour are independent.  No level chain: per (CTA, colour)
-// segment A (no halo read or write), B (within 4 rows of a shared band
-// edge), and an empty seam segment.
-template <class Fit>
-static void build_free_plan(HostGrid &g, const std::vector<int> &r0, Fit fit) {
-  const int C = int(r0.size()) - 1, S = 3;
-  g.cf_pts.clear();
-  g.cf_off.assign(size_t(C) * 5 * S + 1, 0);
-  int maxchunks = 0, maxa = 0, maxb = 0;
-  for (int k = 0; k < C; ++k) {
-    const int first = int(g.cf_pts.size());
-    auto edge = [&](int row) { return (k > 0 && row < r0[k] + 4) || (k < C - 1 && row >= r0[k + 1] - 4); };
-    const int ra = std::max(r0[k], 5), rb = std::min(r0[k + 1], g.nmu);
-    for (int c = 0; c < 5; ++c)
-      for (int seg = 0; seg < S; ++seg) {
-        const int seg0 = int(g.cf_pts.size());
-        g.cf_off[(size_t(k) * 5 + c) * S + seg] = seg0;
-        if (seg == 2) continue;
-        std::vector<std::pair<int, int>> pts;
-        for (int row = ra; row < rb; ++row) {
-          if (edge(row) != (seg == 1)) continue;
-          for (int col = 5; col <= g.nni + 2; ++col)
-            if (((col - row) % 5 + 5) % 5 == c) pts.push_back({row, col});
-        }
-        append_chunks(pts, r0[k], g.n8, g.cf_pts);
-        const int n = int(g.cf_pts.size()) - seg0;
-        if (seg == 0) maxa = std::max(maxa, n);
-        else maxb = std::max(maxb, n);
-      }
-    maxchunks = std::max(maxchunks, int(g.cf_pts.size()) - first);
-  }
-  g.cf_off[size_t(C) * 5 * S] = int(g.cf_pts.size());
-  g.cf_maxchunks = maxchunks;
-  g.cf_wa = std::max(1, (maxa + 31) / 32);
-  g.cf_wb = std::max(1, (maxb + 31) / 32);
-  g.cf_ws = 0;
-  g.cf_pa = g.cf_wa;
-  g.cf_pb = g.cf_wb;
-  g.cf_ps = 0;
-  fit(g.cf_wa, g.cf_wb, g.cf_ws, 24);
-  fit(g.cf_pa, g.cf_pb, g.cf_ps, kPotWarpsFree);
-}
-
 std::string attach_schedule(HostGrid &g);
 
 std::string build_host_grid(HostGrid &g, int nni, int nmu, double r, double rinf, double z1, double z2,
@@ -420,7 +344,7 @@ std::string build_host_grid(HostGrid &g, int nni, int nmu, double r, double rinf
 }
 
 // The sweep schedules of a grid -- "middle" ordering, colour levels, tiles,
-// cluster plans, persistent-band and SOR schedules -- depend on N_nu and
+// band plans, persistent-band and wavefront schedules -- depend on N_nu and
 // N_mu only.  build_schedule makes them; attach_schedule copies them from a
 // process-wide cache of the most recent grid sizes (they take tens of
 // milliseconds to build; a serving loop or repeated solves on one grid size
@@ -545,120 +469,6 @@ static std::string build_schedule(HostGrid &g) {
     }
     g.st_rows[G] = most + 8;
   }
-  g.pts_rc.resize(g.pts.size());
-  for (size_t k = 0; k < g.pts.size(); ++k) g.pts_rc[k] = ((g.pts[k] / g.n8) << 16) | (g.pts[k] % g.n8);
-  // cluster plan for the on-chip FP32 sweep: contiguous tile ranges, ~30
-  // rows per CTA, 2..16 CTAs; each CTA keeps its FP32 band with 4-row halos
-  // plus the band's residual, omega/lhs, coefficient rows and point list in
-  // shared memory
-  g.cl_size = 0;
-  {
-    const int rows = nmu - 4;
-    int C = std::max(2, std::min(16, (rows + 29) / 30));
-    C = std::min(C, g.ntiles);
-    if (C >= 2) {
-      std::vector<int> t0(C + 1), r0(C + 1);
-      int t = 0;
-      t0[0] = 0;
-      for (int k = 1; k < C; ++k) {
-        const int target = 4 + (rows * k + C / 2) / C;
-        while (t < g.ntiles - (C - k) && g.tile_row1[t] <= target) ++t;
-        if (t <= t0[k - 1]) t = t0[k - 1] + 1;
-        t0[k] = t;
-      }
-      t0[C] = g.ntiles;
-      bool ok = true;
-      int maxrows = 0;
-      for (int k = 0; k < C; ++k) {
-        if (t0[k + 1] <= t0[k]) ok = false;
-        r0[k] = g.tile_row0[t0[k]];
-        maxrows = std::max(maxrows, g.tile_row1[t0[k + 1] - 1] - g.tile_row0[t0[k]]);
-      }
-      r0[C] = nmu;
-      // Per (CTA, colour) nlev+2 segments, each processed by its own warps:
-      //   A  level-0 points off the band edges (no halo read or write),
-      //   B  level-0 points within 4 rows of an edge shared with another CTA,
-      //   S0 level-0 points with a same-colour stencil neighbour of a higher
-      //      level (seam points), S1.. the levels 1..nlev-1.
-      // A and B points have no same-colour neighbour at all, so A, B and S0
-      // run concurrently and only the seam warps step through the levels.
-      // Each segment is stored as chunks of up to 4 of its points on one row
-      // at stride 5 (same-colour points of a row are 5 columns apart),
-      // packed (band row << 19) | (col << 2) | (count - 1).
-      const int S = g.nlev + 2;
-      std::vector<char> seam0(g.next, 0);
-      for (auto &d : deps)
-        if (lev[d.first] == 0) seam0[g.order[d.first]] = 1;
-      std::vector<int> chunks, coff(size_t(C) * 5 * S + 1, 0);
-      int maxchunks = 0, maxa = 0, maxb = 0, maxs = 0;
-      for (int k = 0; k < C; ++k) {
-        const int first = int(chunks.size());
-        auto edge = [&](int row) { return (k > 0 && row < r0[k] + 4) || (k < C - 1 && row >= r0[k + 1] - 4); };
-        for (int c = 0; c < 5; ++c)
-          for (int seg = 0; seg < S; ++seg) {
-            const int seg0 = int(chunks.size());
-            coff[(size_t(k) * 5 + c) * S + seg] = seg0;
-            const int l = (seg < 2) ? 0 : seg - 2;
-            std::vector<std::pair<int, int>> pts;
-            for (int t = t0[k]; t < t0[k + 1]; ++t) {
-              const int o = (t * 5 + c) * g.nlev + l;
-              for (int q = g.off[o]; q < g.off[o + 1]; ++q) {
-                const int row = g.pts_rc[q] >> 16, col = g.pts_rc[q] & 0xffff;
-                const bool s0 = seam0[row * g.n8 + col] != 0;
-                if (seg == 0 && (s0 || edge(row))) continue;
-                if (seg == 1 && (s0 || !edge(row))) continue;
-                if (seg == 2 && !s0) continue;
-                pts.push_back({row, col});
-              }
-            }
-            append_chunks(pts, r0[k], g.n8, chunks);
-            const int n = int(chunks.size()) - seg0;
-            if (seg == 0) maxa = std::max(maxa, n);
-            else if (seg == 1) maxb = std::max(maxb, n);
-            else maxs = std::max(maxs, n);
-          }
-        maxchunks = std::max(maxchunks, int(chunks.size()) - first);
-      }
-      coff[size_t(C) * 5 * S] = int(chunks.size());
-      // shared memory: (residual, omega/lhs) pairs, correction band with
-      // 4-row halos, b(mu) of the band's rows, d(nu) by column, the segment
-      // offsets, then the CTA's chunk list
-      const size_t smem = 2 * size_t(maxrows) * g.n8 * sizeof(float) + size_t(maxrows + 8) * g.n8 * sizeof(float) +
-                          size_t(maxrows + g.n8) * sizeof(float) + size_t(5 * S + 1) * sizeof(int) +
-                          size_t(maxchunks) * sizeof(int);
-      // a band must be at least 4 rows (halo pushes go to the next CTA only)
-      for (int k = 0; k < C; ++k)
-        if (r0[k + 1] - r0[k] < 4) ok = false;
-      if (ok && maxrows < 4096 && g.n8 < (1 << 17) && smem <= 200 * 1024) {
-        g.cl_size = C;
-        g.cl_maxrows = maxrows;
-        g.cl_maxchunks = maxchunks;
-        // warps per role: enough for one pass over the largest segment, at
-        // most 24 warps in all (the roles loop when a segment is larger)
-        g.cl_wa = std::max(1, (maxa + 31) / 32);
-        g.cl_wb = std::max(1, (maxb + 31) / 32);
-        g.cl_ws = std::max(1, (maxs + 31) / 32);
-        auto fit = [](int &a, int &b, int &c, int most) {
-          while (a + b + c > most) {
-            if (a >= b && a >= c) --a;
-            else if (b >= c) --b;
-            else --c;
-          }
-        };
-        g.cl_pa = g.cl_wa;
-        g.cl_pb = g.cl_wb;
-        g.cl_ps = g.cl_ws;
-        fit(g.cl_wa, g.cl_wb, g.cl_ws, 24);
-        fit(g.cl_pa, g.cl_pb, g.cl_ps, kPotWarpsRef);
-        g.cl_smem = smem;
-        g.cl_tile0 = t0;
-        g.cl_row0 = r0;
-        g.cl_pts = chunks;
-        g.cl_off = coff;
-        build_free_plan(g, r0, fit);
-      }
-    }
-  }
   // final check: no two points of one (tile,colour,level) bucket interact,
   // and every dependency is inside a tile with a strictly larger level
   for (auto &d : deps) {
@@ -700,30 +510,6 @@ void copy_schedule(HostGrid &to, const HostGrid &from) {
   to.tile_row1 = from.tile_row1;
   to.pts = from.pts;
   to.off = from.off;
-  to.pts_rc = from.pts_rc;
-  to.cl_size = from.cl_size;
-  to.cl_maxrows = from.cl_maxrows;
-  to.cl_maxchunks = from.cl_maxchunks;
-  to.cl_wa = from.cl_wa;
-  to.cl_wb = from.cl_wb;
-  to.cl_ws = from.cl_ws;
-  to.cl_pa = from.cl_pa;
-  to.cl_pb = from.cl_pb;
-  to.cl_ps = from.cl_ps;
-  to.cl_smem = from.cl_smem;
-  to.cl_tile0 = from.cl_tile0;
-  to.cl_row0 = from.cl_row0;
-  to.cl_pts = from.cl_pts;
-  to.cl_off = from.cl_off;
-  to.cf_maxchunks = from.cf_maxchunks;
-  to.cf_wa = from.cf_wa;
-  to.cf_wb = from.cf_wb;
-  to.cf_ws = from.cf_ws;
-  to.cf_pa = from.cf_pa;
-  to.cf_pb = from.cf_pb;
-  to.cf_ps = from.cf_ps;
-  to.cf_pts = from.cf_pts;
-  to.cf_off = from.cf_off;
   to.st_pts = from.st_pts;
   to.st_off = from.st_off;
   for (int k = 0; k <= HostGrid::kBandRuns; ++k) to.st_rows[k] = from.st_rows[k];
@@ -820,22 +606,6 @@ extern "C" int x2g_host_schedule(int nnu, int nmu, int *npoints, int *ntiles, in
   return X2G_OK;
 }
 
-// Cluster plan of the on-chip FP32 sweep (no CUDA call): CTAs per job,
-// rows per CTA, shared memory bytes; row0[C+1] when non-NULL.
-extern "C" int x2g_host_cluster_plan(int nnu, int nmu, int *csize, int *maxrows, long *smem, int *row0) {
-  x2g::HostGrid g;
-  std::string msg = x2g::build_host_grid(g, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
-  if (!msg.empty()) return X2G_ERR_SCHEDULE;
-  if (csize) *csize = g.cl_size;
-  if (maxrows) *maxrows = g.cl_maxrows;
-  if (smem) *smem = long(g.cl_smem);
-  if (row0 && g.cl_size > 0) std::copy(g.cl_row0.begin(), g.cl_row0.end(), row0);
-  return X2G_OK;
-}
-
-// Chunk lists of the on-chip sweep: nchunks packed chunks and noff segment
-// offsets (CTA-major, 5 colours x (nlevels + 1) segments per CTA, plus the
-// end).  Call with null arrays for the counts.
 extern "C" int x2g_host_band_schedule(int nnu, int nmu, int *npoints, int *ntiles, int *nlevels, int *pts, int *off,
                                       int *rows, int *tile_row0, int *tile_row1) {
   x2g::HostGrid g;
@@ -849,30 +619,6 @@ extern "C" int x2g_host_band_schedule(int nnu, int nmu, int *npoints, int *ntile
   if (rows) std::copy(g.st_rows, g.st_rows + x2g::HostGrid::kBandRuns + 1, rows);
   if (tile_row0) std::copy(g.tile_row0.begin(), g.tile_row0.end(), tile_row0);
   if (tile_row1) std::copy(g.tile_row1.begin(), g.tile_row1.end(), tile_row1);
-  return X2G_OK;
-}
-
-extern "C" int x2g_host_cluster_chunks(int nnu, int nmu, int *nchunks, int *noff, int *chunks, int *off) {
-  x2g::HostGrid g;
-  std::string msg = x2g::build_host_grid(g, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
-  if (!msg.empty()) return X2G_ERR_SCHEDULE;
-  if (nchunks) *nchunks = int(g.cl_pts.size());
-  if (noff) *noff = int(g.cl_off.size());
-  if (chunks) std::copy(g.cl_pts.begin(), g.cl_pts.end(), chunks);
-  if (off) std::copy(g.cl_off.begin(), g.cl_off.end(), off);
-  return X2G_OK;
-}
-
-// The same for the seam-free colouring of the mixed form (colour (col - row)
-// mod 5; per CTA and colour the segments A, B and an empty seam segment).
-extern "C" int x2g_host_free_chunks(int nnu, int nmu, int *nchunks, int *noff, int *chunks, int *off) {
-  x2g::HostGrid g;
-  std::string msg = x2g::build_host_grid(g, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
-  if (!msg.empty()) return X2G_ERR_SCHEDULE;
-  if (nchunks) *nchunks = int(g.cf_pts.size());
-  if (noff) *noff = int(g.cf_off.size());
-  if (chunks) std::copy(g.cf_pts.begin(), g.cf_pts.end(), chunks);
-  if (off) std::copy(g.cf_off.begin(), g.cf_off.end(), off);
   return X2G_OK;
 }
 
