@@ -309,8 +309,8 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
   d.m8 = h.m8;
   d.next = h.next;
   d.mxsize = h.mxsize;
-  d.ntiles = h.ntiles;
-  d.nlev = h.nlev;
+  d.ntiles = h.s->ntiles;
+  d.nlev = h.s->nlev;
   d.mpole = h.mpole;
   d.r2 = h.r2;
   std::memcpy(d.dmu1, h.dmu1, sizeof d.dmu1);
@@ -367,11 +367,6 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
     }
     return w;
   };
-  std::vector<int> place(h.st_pts.size());
-  for (size_t k = 0; k < place.size(); ++k) {
-    const int row = h.st_pts[k] >> 16, col = h.st_pts[k] & 0xffff;
-    place[size_t(row - 5) * (h.nni - 2) + col - 5] = int(k);
-  }
   const void *tmp;
   int rc = X2G_OK;
 #define UPTO(vec, dest)                                                                 \
@@ -409,20 +404,18 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
   UP(h.vxisq, vxisq);
   UP(h.veta, veta);
   UP(h.vetasq, vetasq);
-  UP(h.tile_row0, tile_row0);
-  UP(h.tile_row1, tile_row1);
-  UP(h.pts, pts);
-  UP(h.off, off);
-  UP(h.st_pts, st_pts);
-  UP(h.st_off, st_off);
-  const WaveHost *waves[2] = {&h.sor, &h.mcsor};
+  UP(h.s->tile_row0, tile_row0);
+  UP(h.s->tile_row1, tile_row1);
+  UP(h.s->pts, pts);
+  UP(h.s->off, off);
+  UP(h.s->st_pts, st_pts);
+  UP(h.s->st_off, st_off);
+  const WaveHost *waves[2] = {&h.s->sor, &h.s->mcsor};
   WaveDev *wave_dev[2] = {&d.sor, &d.mcsor};
   for (int k = 0; k < 2; ++k) {
     const WaveHost &w = *waves[k];
     WaveDev &wd = *wave_dev[k];
-    std::vector<int2> e(w.pts.size());
-    for (size_t q = 0; q < e.size(); ++q) e[q] = make_int2(w.pts[q], w.mask[q]);
-    UPTO(e, wd.pts);
+    UPTO(w.pts, wd.pts);
     UPTO(w.off, wd.off);
     UPTO(w.bpts, wd.bpts);
     UPTO(w.boff, wd.boff);
@@ -430,11 +423,9 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
     wd.nblev = w.nblev;
     wd.delta = w.delta;
   }
-  std::vector<int2> march(h.march_pts.size());
-  for (size_t k = 0; k < march.size(); ++k) march[k] = make_int2(h.march_pts[k], h.march_mask[k]);
-  UPTO(march, d.march.pts);
-  UPTO(h.march_off, d.march.off);
-  for (int k = 0; k <= HostGrid::kBandRuns; ++k) d.st_rows[k] = h.st_rows[k];
+  UPTO(h.s->march_pts, d.march.pts);
+  UPTO(h.s->march_off, d.march.off);
+  for (int k = 0; k <= Schedule::kBandRuns; ++k) d.st_rows[k] = h.s->st_rows[k];
   UP(b32, borb_mu32);
   UP(p32, bpot_mu32);
   UP(d32, d_nu32);
@@ -444,7 +435,7 @@ int x2g_grid_create(x2g_ctx *ctx, int nnu, int nmu, double r, double rinf, doubl
   const std::vector<int2> fixed_mp = fixed(cmp), fixed_nu = fixed(cnu);
   UP(fixed_mp, wmu_pot);
   UP(fixed_nu, wnu);
-  UP(place, st_place);
+  UP(h.s->st_place, st_place);
 #undef UP
 #undef UPTO
   {
@@ -509,9 +500,9 @@ int x2g_grid_info(x2g_grid *gr, int *nnu, int *nmu, int *ntiles, int *nlevels, i
   if (!gr) return set_status(X2G_ERR_ARG, "null grid");
   if (nnu) *nnu = gr->h.nni;
   if (nmu) *nmu = gr->h.nmu;
-  if (ntiles) *ntiles = gr->h.ntiles;
-  if (nlevels) *nlevels = gr->h.nlev;
-  if (npoints) *npoints = int(gr->h.order.size());
+  if (ntiles) *ntiles = gr->h.s->ntiles;
+  if (nlevels) *nlevels = gr->h.s->nlev;
+  if (npoints) *npoints = int(gr->h.s->order.size());
   return X2G_OK;
 }
 

@@ -130,7 +130,7 @@ void mcsor_common(int *isym, double *wk2, double *lhs, double *rhs) {
 // partition of the "middle" list by position mod 5), i.e. single-thread
 // MCSOR; 0 the "middle" list itself, i.e. list-order SOR; -1 neither.
 int sor_list_order() {
-  const std::vector<int> &mid = g_grid->h.order;  // 0-based ext indices, middle order
+  const std::vector<int> &mid = g_grid->h.s->order;  // 0-based ext indices, middle order
   const int n = int(mid.size());
   const int *lst = c_sorptr_.p + (c_iadex_.iadextc - 1);
   bool is_mid = true, is_col = true;

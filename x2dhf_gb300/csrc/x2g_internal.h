@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <string>
+#include <memory>
 #include <vector>
 
 #include "../../include/x2dhf_gpu.h"
@@ -36,11 +37,11 @@ constexpr int kBarWords = kPhaseWords + kPhaseBlocks * kPhaseStride;
 // ----------------------------------------------------------------------
 struct WaveHost {
   int nlev = 0, nblev = 0, delta = 0;
+  // pts: interior points as pairs (packed point, mask); mask: the stencil
+  // neighbours earlier in the list, bit 4 (k-1) + {0: -k, 1: +k, 2: -k rows, 3:
+  // +k rows}; bits 16..18: the point is the fifth of the extrapolation of the
+  // mu=1 row, nu=1 or nu=nni column
   std::vector<int> pts, off, bpts, boff;
-  // per entry of pts the stencil neighbours earlier in the list, bit 4 (k-1)
-  // + {0: -k, 1: +k, 2: -k rows, 3: +k rows}; bits 16..18: the point is the
-  // fifth of the extrapolation of the mu=1 row, nu=1 or nu=nni column
-  std::vector<int> mask;
 };
 
 // ----------------------------------------------------------------------
@@ -64,6 +65,46 @@ struct ColPlan {
 };
 
 // ----------------------------------------------------------------------
+// What the sweeps of a grid size follow: depends on N_nu and N_mu only, and is
+// shared by the grids of a size (attach_schedule).
+// ----------------------------------------------------------------------
+struct Schedule {
+  int nni = 0, nmu = 0, n8 = 0, next = 0;
+  // "middle" ordering of interior points (ext indices, reference list order)
+  std::vector<int> order;
+  // sweep schedule: tiles = bands of ext rows [row0,row1)
+  int ntiles = 0, nlev = 0;
+  std::vector<int> tile_row0, tile_row1;
+  std::vector<int> pts;  // ext indices grouped [tile][colour][level]
+  std::vector<int> off;  // (ntiles*5*nlev + 1) offsets into pts
+  // persistent-band FP32 sweep of grids beyond one cluster: the same points
+  // regrouped [colour][level][tile] (st_pts, packed (ext row << 16) | ext
+  // col), so that the points of one colour and level in any run of
+  // consecutive tiles are one contiguous range; st_off[(c * nlev + l) *
+  // (ntiles + 1) + t] is the start of tile t.  st_rows[G] = most rows of any
+  // run of G consecutive tiles plus the 4-row halos on both sides (G =
+  // 1..kBandRuns)
+  static constexpr int kBandRuns = 16;
+  std::vector<int> st_pts, st_off;
+  // the place of interior point (mu, nu) in st_pts, (nni - 2) (mu - 1) + nu - 1
+  std::vector<int> st_place;
+  int st_rows[kBandRuns + 1] = {};
+  // bands of the on-chip FP32 sweep, by cluster size and threads per column
+  std::vector<ColPlan> columns;
+  // SOR's points of ext rows 4..nmu-1 (4: the mu=1 axis) by row and side of
+  // the middle column, in list order: row r's left (right) points are entries
+  // [march_off[2(r-4)], march_off[2(r-4)+1]) (then up to march_off[2(r-4)+2])
+  // of march_pts, pairs of the ext index and a mask (sor's, kMarchAxis... for
+  // axis points and the stride to what they read); a side ends with its axis
+  // point
+  std::vector<int> march_pts, march_off;
+  // the FP64 sweeps' wavefront schedules (build_wave_schedule): list-order
+  // SOR over the "middle" list (sor, sormcsor.F90:20-132), and MCSOR as the
+  // same sweep over the list colour after colour (mcsor, :143-386)
+  WaveHost sor, mcsor;
+};
+
+// ----------------------------------------------------------------------
 // Host-side grid: every table the relaxation path reads, built with the
 // reference's formulas (initCBAllocArrays.F90 initCBlocks:813-858,
 // initSuppl:1636-2051).  Indices are 0-based: nu j in [0,nni), mu i in
@@ -82,35 +123,7 @@ struct HostGrid {
   std::vector<double> d_nu;                     // nu-only
   std::vector<double> e, f0, f1, f2, f4, g, wgt1, wgt2;  // plain 2-D tables
   std::vector<double> leg;                      // mpole tables P_k(cos th) r^k, plain
-  // "middle" ordering of interior points (ext indices, reference list order)
-  std::vector<int> order;
-  // sweep schedule: tiles = bands of ext rows [row0,row1)
-  int ntiles = 0, nlev = 0;
-  std::vector<int> tile_row0, tile_row1;
-  std::vector<int> pts;  // ext indices grouped [tile][colour][level]
-  std::vector<int> off;  // (ntiles*5*nlev + 1) offsets into pts
-  // persistent-band FP32 sweep of grids beyond one cluster: the same points
-  // regrouped [colour][level][tile] (st_pts, packed (ext row << 16) | ext
-  // col), so that the points of one colour and level in any run of
-  // consecutive tiles are one contiguous range; st_off[(c * nlev + l) *
-  // (ntiles + 1) + t] is the start of tile t.  st_rows[G] = most rows of any
-  // run of G consecutive tiles plus the 4-row halos on both sides (G =
-  // 1..kBandRuns)
-  static constexpr int kBandRuns = 16;
-  std::vector<int> st_pts, st_off;
-  int st_rows[kBandRuns + 1] = {};
-  // bands of the on-chip FP32 sweep, by cluster size and threads per column
-  std::vector<ColPlan> columns;
-  // SOR's points of ext rows 4..nmu-1 (4: the mu=1 axis) by row and side of
-  // the middle column, in list order: row r's left (right) points are entries
-  // [march_off[2(r-4)], march_off[2(r-4)+1]) (then up to march_off[2(r-4)+2])
-  // of march_pts (ext index) and march_mask (sor.mask, kMarchAxis... for axis
-  // points and the stride to what they read); a side ends with its axis point
-  std::vector<int> march_pts, march_mask, march_off;
-  // the FP64 sweeps' wavefront schedules (build_wave_schedule): list-order
-  // SOR over the "middle" list (sor, sormcsor.F90:20-132), and MCSOR as the
-  // same sweep over the list colour after colour (mcsor, :143-386)
-  WaveHost sor, mcsor;
+  std::shared_ptr<const Schedule> s;            // of this grid size
 };
 
 std::string build_host_grid(HostGrid &g, int nni, int nmu, double r, double rinf, double z1, double z2, int mpole);
@@ -126,7 +139,7 @@ struct WaveDev {
   int nlev, nblev, delta;
 };
 
-// SOR's points by row and side (HostGrid::march_pts): (ext index, mask)
+// SOR's points by row and side (Schedule::march_pts): (ext index, mask)
 struct MarchDev {
   const int2 *pts;
   const int *off;
@@ -253,7 +266,7 @@ struct x2g_ctx {
   int mixed_free = 0;           // cluster sweep colouring: 0 the reference's list order mod 5, 1 seam-free
   // kernels of the cluster sweep that run a grid size's band plans here
   struct ColumnShape {
-    int plan;  // place in HostGrid::columns
+    int plan;  // place in Schedule::columns
     const void *fn;
     bool sep;
     int rows;

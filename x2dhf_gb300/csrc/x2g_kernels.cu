@@ -450,7 +450,7 @@ struct WaveWait {
 struct WaveItem {
   int kind, jb, s;
   int rc;         // (ext row << 16) | ext col
-  unsigned mask;  // interior points: the bits of HostGrid::sor_mask
+  unsigned mask;  // interior points: the mask of WaveHost::pts
   __device__ __forceinline__ int row() const { return rc >> 16; }
   __device__ __forceinline__ int col() const { return rc & 0xffff; }
 };
@@ -589,7 +589,7 @@ __device__ __forceinline__ bool wave_axis(const GridDev &g, const JobTable &jobs
 
 // the axis value five points from a point, or 0: an extrapolation's last
 // point is the only one that does not read it back (flags of
-// HostGrid::sor_mask); which: 0 along mu, 1 along nu
+// WaveHost::pts); which: 0 along mu, 1 along nu
 __device__ __forceinline__ int fifth_reader(const GridDev &g, unsigned mask, int ij, int which) {
   if (which == 0) return (mask & 0x10000u) ? ij - 5 * g.n8 : 0;
   return (mask & 0x20000u) ? ij - 5 : (mask & 0x40000u) ? ij + 5 : 0;
@@ -2543,9 +2543,9 @@ static const std::vector<x2g_ctx::ColumnShape> &column_shapes(x2g_ctx *ctx, cons
   for (const auto &s : ctx->columns)
     if (s.nni == h.nni && s.nmu == h.nmu) return s.shapes;
   x2g_ctx::ColumnShapes out{h.nni, h.nmu, {}};
-  for (size_t i = 0; i < h.columns.size(); ++i)
+  for (size_t i = 0; i < h.s->columns.size(); ++i)
     for (int kind = 0; kind < 3; ++kind) {
-      const ColPlan &p = h.columns[i];
+      const ColPlan &p = h.s->columns[i];
       int pitch = 0;
       const ColKernel k = column_kernel(p, kind > 0, kind == 2, std::max(p.pitch, p.warps * 32), pitch);
       if (!k.fn) continue;
@@ -2582,7 +2582,7 @@ static ColChoice choose_columns(x2g_ctx *ctx, const HostGrid &h, int njobs, bool
   if (ctx->no_cluster) return best;
   for (const x2g_ctx::ColumnShape &c : column_shapes(ctx, h)) {
     if (c.sep != sep) continue;
-    const ColPlan &p = h.columns[size_t(c.plan)];
+    const ColPlan &p = h.s->columns[size_t(c.plan)];
     const int wave = std::min(c.active, kParamJobs);
     const double time = njobs / wave * column_time(p, wave, ctx->num_sms) +
                         (njobs % wave ? column_time(p, njobs % wave, ctx->num_sms) : 0.0);
@@ -2631,7 +2631,7 @@ static int persistent_shape(x2g_ctx *ctx, const GridDev &g, int most, int *nj, i
   }
   for (int n = most; n >= 1; --n)
     for (int bpsm = 2; bpsm >= 1; --bpsm)
-      for (int r = 1; r <= HostGrid::kBandRuns; ++r) {
+      for (int r = 1; r <= Schedule::kBandRuns; ++r) {
         const size_t sm = band_smem_bytes(g, r);
         if (sm > size_t(ctx->band_attr) || int(size_t(ctx->band_sm_smem) / (sm + 1024)) < bpsm) break;
         const int items = n * ((g.ntiles + r - 1) / r), nt = kBandThreads * (bpsm == 1 ? 2 : 1);

@@ -45,24 +45,33 @@ std::vector<double> newton_cotes(int n, double h) {
 // sweep's values of those later in the list and of the axis, and delta makes
 // every such previous-sweep value final before it is read and not yet
 // overwritten.  The ghost cells and the mu >= nmu-3 rows stay fixed during a
-// relaxation call.  Every dependency is checked here; a violation refuses
-// the grid.
-std::string build_wave_schedule(const HostGrid &g, const std::vector<int> &order, const int *offs, WaveHost &w) {
+// relaxation call.
+//
+// One pass over the list: a point's neighbours earlier in it are those that have
+// a level already.  Its level is above theirs, so that it reads their new values
+// and they its old one, if delta exceeds the difference; the same holds for an
+// axis point and the five it reads, among which are the only points that read
+// it.
+std::string build_wave_schedule(const Schedule &g, const std::vector<int> &order, const std::vector<int> &packed,
+                                const int *offs, WaveHost &w) {
   const int npts = int(order.size()), n8 = g.n8, nni = g.nni, nmu = g.nmu;
-  std::vector<int> pos(g.next, -1);
-  for (int p = 0; p < npts; ++p) pos[order[p]] = p;
-  std::vector<int> L(npts, 0);
-  int nlev = 0;
+  std::vector<int> level(g.next, -1), mask(npts);  // level by ext index
+  int nlev = 0, delta = 1;
   for (int p = 0; p < npts; ++p) {
-    const int ij = order[p];
-    int l = 0;
+    // an interior point's 16 neighbours all lie in the extended array
+    const int *at = level.data() + order[p];
+    int most = -1;
+    unsigned least = ~0u, m = 0;
     for (int k = 0; k < 16; ++k) {
-      const int q = ij + offs[k];
-      if (q < 0 || q >= g.next || pos[q] < 0 || pos[q] >= p) continue;
-      l = std::max(l, L[pos[q]] + 1);
+      const int l = at[offs[k]];
+      most = std::max(most, l);
+      least = std::min(least, unsigned(l));
+      m |= unsigned(l >= 0) << k;
     }
-    L[p] = l;
-    nlev = std::max(nlev, l + 1);
+    if (m) delta = std::max(delta, most + 1 - int(least) + 1);  // the earlier one's old value
+    level[order[p]] = most + 1;
+    mask[p] = int(m);
+    nlev = std::max(nlev, most + 2);
   }
   // axis points (sormcsor.F90:94-129, lists of mesh:2823-2842): the mu=1
   // row (ext row 4, cols 5..nni+2) from rows 5..9, then the nu=1 and nu=nni
@@ -77,112 +86,67 @@ std::string build_wave_schedule(const HostGrid &g, const std::vector<int> &order
     ax.push_back({r * n8 + 4, 1});
     ax.push_back({r * n8 + nni + 3, -1});
   }
-  std::vector<int> B(g.next, -1);  // axis level by ext index
   int nblev = 0;
   for (const Axis &a : ax) {
-    int b = 0;
+    int most = -1, least = 0x7fffffff;
     for (int k = 1; k <= 5; ++k) {
-      const int q = a.ij + k * a.st;
-      const int lq = (pos[q] >= 0) ? L[pos[q]] : B[q];
-      if (lq < 0) return "schedule: an axis point reads neither an interior nor an axis point";
-      b = std::max(b, lq + 1);
+      const int l = level[a.ij + k * a.st];
+      if (l < 0) return "schedule: an axis point reads neither an interior nor an axis point";
+      most = std::max(most, l);
+      least = std::min(least, l);
     }
-    B[a.ij] = b;
-    nblev = std::max(nblev, b + 1);
+    level[a.ij] = most + 1;
+    delta = std::max(delta, most + 1 - least + 1);  // read before the next sweep overwrites it
+    nblev = std::max(nblev, most + 2);
   }
-  // delta: every value a step reads from the previous sweep is final and
-  // not yet overwritten by the next
-  int delta = 1;
-  for (int p = 0; p < npts; ++p) {
-    const int ij = order[p];
-    for (int k = 0; k < 16; ++k) {
-      const int q = ij + offs[k];
-      if (q < 0 || q >= g.next) continue;
-      if (pos[q] > p) delta = std::max(delta, L[pos[q]] - L[p] + 1);  // a later point's old value
-      if (B[q] >= 0) delta = std::max(delta, B[q] - L[p] + 1);        // an axis value
-    }
-  }
-  for (const Axis &a : ax)
-    for (int k = 1; k <= 5; ++k) {
-      const int q = a.ij + k * a.st;
-      const int lq = (pos[q] >= 0) ? L[pos[q]] : B[q];
-      delta = std::max(delta, B[a.ij] - lq + 1);  // read before the next sweep overwrites it
-    }
-  // check every dependency at sweeps s and s+1 (step = level + s * delta)
-  for (int p = 0; p < npts; ++p) {
-    const int ij = order[p];
-    for (int k = 0; k < 16; ++k) {
-      const int q = ij + offs[k];
-      if (q < 0 || q >= g.next) continue;
-      if (pos[q] >= 0 && pos[q] < p && !(L[pos[q]] < L[p])) return "schedule: new value read too early";
-      if (pos[q] > p && !(L[pos[q]] > L[p] && L[pos[q]] < L[p] + delta))
-        return "schedule: old value of a later point not preserved";
-      if (B[q] >= 0 && !(B[q] > L[p] && B[q] < L[p] + delta)) return "schedule: axis value out of order";
-    }
-  }
-  for (const Axis &a : ax)
-    for (int k = 1; k <= 5; ++k) {
-      const int q = a.ij + k * a.st;
-      const int lq = (pos[q] >= 0) ? L[pos[q]] : B[q];
-      if (!(lq < B[a.ij] && B[a.ij] < lq + delta)) return "schedule: extrapolation out of order";
-    }
   w.nlev = nlev;
   w.nblev = nblev;
   w.delta = delta;
   w.off.assign(nlev + 1, 0);
-  for (int p = 0; p < npts; ++p) w.off[L[p] + 1]++;
+  for (int p = 0; p < npts; ++p) w.off[level[order[p]] + 1]++;
   for (int l = 0; l < nlev; ++l) w.off[l + 1] += w.off[l];
-  w.pts.assign(npts, 0);
+  w.pts.resize(size_t(npts) * 2);
   {
     std::vector<int> fill(w.off.begin(), w.off.end() - 1);
-    w.mask.assign(npts, 0);
     for (int p = 0; p < npts; ++p) {
-      const int ij = order[p], at = fill[L[p]]++;
-      w.pts[at] = ((ij / n8) << 16) | (ij % n8);
-      for (int k = 0; k < 16; ++k)  // an interior point's 16 neighbours all lie in the extended array
-        if (pos[ij + offs[k]] >= 0 && pos[ij + offs[k]] < p) w.mask[at] |= 1 << k;
-      // the fifth point of an axis extrapolation
-      if (ij / n8 == 9) w.mask[at] |= 1 << 16;
-      if (ij % n8 == 9) w.mask[at] |= 1 << 17;
-      if (ij % n8 == nni - 2) w.mask[at] |= 1 << 18;
+      const int at = fill[level[order[p]]]++, rc = packed[p], row = rc >> 16, col = rc & 0xffff;
+      w.pts[2 * size_t(at)] = rc;
+      // and whether it is the fifth point of an axis extrapolation
+      w.pts[2 * size_t(at) + 1] = mask[p] | (row == 9) << 16 | (col == 9) << 17 | (col == nni - 2) << 18;
     }
   }
   w.boff.assign(nblev + 1, 0);
-  for (const Axis &a : ax) w.boff[B[a.ij] + 1]++;
+  for (const Axis &a : ax) w.boff[level[a.ij] + 1]++;
   for (int l = 0; l < nblev; ++l) w.boff[l + 1] += w.boff[l];
   w.bpts.assign(ax.size(), 0);
   {
     std::vector<int> fill(w.boff.begin(), w.boff.end() - 1);
-    for (const Axis &a : ax) w.bpts[fill[B[a.ij]]++] = ((a.ij / n8) << 16) | (a.ij % n8);
+    for (const Axis &a : ax) w.bpts[fill[level[a.ij]]++] = ((a.ij / n8) << 16) | (a.ij % n8);
   }
   return "";
 }
 
 // SOR's points by row and side, from the wavefront schedule (whose entries are
 // sorted by level, so every row and side is in list order).
-void build_march(HostGrid &g) {
-  const int rows = g.nmu - 4, n8 = g.n8, last = g.nni + 3, middle = (g.n8 - 1) / 2 - 1;  // last column of the first half
-  std::vector<std::vector<int>> pts(size_t(rows) * 2), mask(size_t(rows) * 2);
-  auto add = [&](int ij, int col, unsigned m) {
-    const size_t k = size_t(ij / n8 - 4) * 2 + (col > middle);
-    pts[k].push_back(ij);
-    mask[k].push_back(int(m));
+void build_march(Schedule &g) {
+  const int sides = (g.nmu - 4) * 2, n8 = g.n8, last = g.nni + 3, middle = (g.n8 - 1) / 2 - 1;  // last column of the first half
+  const int npts = int(g.sor.pts.size() / 2), naxis = int(g.sor.bpts.size());
+  auto side = [&](int rc) { return ((rc >> 16) - 4) * 2 + ((rc & 0xffff) > middle); };
+  g.march_off.assign(sides + 1, 0);
+  for (int k = 0; k < npts; ++k) g.march_off[side(g.sor.pts[2 * size_t(k)]) + 1]++;
+  for (int k = 0; k < naxis; ++k) g.march_off[side(g.sor.bpts[k]) + 1]++;
+  for (int k = 0; k < sides; ++k) g.march_off[k + 1] += g.march_off[k];
+  g.march_pts.resize(size_t(npts + naxis) * 2);
+  std::vector<int> fill(g.march_off.begin(), g.march_off.end() - 1);
+  auto add = [&](int rc, int mask) {
+    const size_t at = size_t(fill[side(rc)]++) * 2;
+    g.march_pts[at] = (rc >> 16) * n8 + (rc & 0xffff);
+    g.march_pts[at + 1] = mask;
   };
-  for (size_t k = 0; k < g.sor.pts.size(); ++k) {
-    const int row = g.sor.pts[k] >> 16, col = g.sor.pts[k] & 0xffff;
-    add(row * n8 + col, col, unsigned(g.sor.mask[k]));
-  }
-  for (size_t k = 0; k < g.sor.bpts.size(); ++k) {
-    const int row = g.sor.bpts[k] >> 16, col = g.sor.bpts[k] & 0xffff;
-    add(row * n8 + col, col, col == 4 ? kMarchAxisUp : col == last ? kMarchAxisDown : kMarchAxisMu);
-  }
-  g.march_pts.clear();
-  g.march_mask.clear();
-  g.march_off.assign(1, 0);
-  for (size_t k = 0; k < pts.size(); ++k) {
-    g.march_pts.insert(g.march_pts.end(), pts[k].begin(), pts[k].end());
-    g.march_mask.insert(g.march_mask.end(), mask[k].begin(), mask[k].end());
-    g.march_off.push_back(int(g.march_pts.size()));
+  for (int k = 0; k < npts; ++k) add(g.sor.pts[2 * size_t(k)], g.sor.pts[2 * size_t(k) + 1]);
+  for (int k = 0; k < naxis; ++k) {
+    const int col = g.sor.bpts[k] & 0xffff;
+    add(g.sor.bpts[k], int(col == 4 ? kMarchAxisUp : col == last ? kMarchAxisDown : kMarchAxisMu));
   }
 }
 
@@ -345,59 +309,57 @@ std::string build_host_grid(HostGrid &g, int nni, int nmu, double r, double rinf
 
 // The sweep schedules of a grid -- "middle" ordering, colour levels, tiles,
 // band plans, persistent-band and wavefront schedules -- depend on N_nu and
-// N_mu only.  build_schedule makes them; attach_schedule copies them from a
+// N_mu only.  build_schedule makes them; attach_schedule takes them from a
 // process-wide cache of the most recent grid sizes (they take tens of
 // milliseconds to build; a serving loop or repeated solves on one grid size
-// build them once).
-static std::string build_schedule(HostGrid &g) {
+// build them once, and the grids of a size share them).
+static std::string build_schedule(Schedule &g) {
   const int nni = g.nni, nmu = g.nmu;
   // ------------------------------------------------------------------
   // "middle" ordering of the interior points (mesh:2503-2544), 1-based
   // ext rows ii in 6..nmu, cols jj in 6..nni+3, middle-outward.
   // ------------------------------------------------------------------
-  const int nmux = (g.m8 - 1) / 2, nnix = (g.n8 - 1) / 2;
-  g.order.clear();
-  g.order.reserve(size_t(nni - 2) * (nmu - 5));
-  for (int i = 6; i <= nmu; i++) {
-    int ii = (i <= nmux) ? nmux - i + 6 : i;
-    for (int j = 6; j <= nni + 3; j++) {
-      int jj = (j <= nnix) ? nnix - j + 6 : j;
-      g.order.push_back((ii - 1) * g.n8 + (jj - 1));
+  const int n8 = g.n8 = nni + 8, m8 = nmu + 8, nmux = (m8 - 1) / 2, nnix = (n8 - 1) / 2;
+  g.next = n8 * m8;
+  const int npts = (nni - 2) * (nmu - 5);
+  g.order.resize(npts);
+  std::vector<int> packed(npts);  // the same points as (ext row << 16) | ext col
+  std::vector<signed char> colour(g.next, -1);  // list position mod 5 (mcsor loops i=c,ngrid1,5)
+  for (int i = 6, p = 0; i <= nmu; i++) {
+    const int row = ((i <= nmux) ? nmux - i + 6 : i) - 1;
+    for (int j = 6; j <= nni + 3; j++, p++) {
+      const int col = ((j <= nnix) ? nnix - j + 6 : j) - 1;
+      g.order[p] = row * n8 + col;
+      packed[p] = (row << 16) | col;
+      colour[row * n8 + col] = (signed char)(p % 5);
     }
   }
-  const int npts = int(g.order.size());
-  // colour = list position mod 5 (mcsor loops i=c,ngrid1,5)
-  std::vector<int> pos(g.next, -1);
-  for (int p = 0; p < npts; p++) pos[g.order[p]] = p;
   // colour level: a point waits for every same-colour stencil neighbour
   // earlier in the list (new value read) and, by symmetry, is waited on by
   // every same-colour neighbour later in the list (old value read).
-  std::vector<int> lev(npts, 0);
-  std::vector<std::pair<int, int>> deps;
+  std::vector<signed char> lev(g.next, -1);  // by ext index
+  std::vector<std::pair<int, int>> deps;     // ext indices
   int offs[16];
   for (int k = 1; k <= 4; k++) {
     offs[4 * (k - 1) + 0] = -k;
     offs[4 * (k - 1) + 1] = k;
-    offs[4 * (k - 1) + 2] = -k * g.n8;
-    offs[4 * (k - 1) + 3] = k * g.n8;
+    offs[4 * (k - 1) + 2] = -k * n8;
+    offs[4 * (k - 1) + 3] = k * n8;
   }
   int maxlev = 0;
   for (int p = 0; p < npts; p++) {
-    int ij = g.order[p], L = 0;
+    const int ij = g.order[p], c = colour[ij];
+    int L = 0;
     for (int o : offs) {
-      int q = ij + o;
-      if (q < 0 || q >= g.next) continue;
-      int pq = pos[q];
-      if (pq < 0 || pq % 5 != p % 5) continue;
-      if (pq < p) {
-        L = std::max(L, lev[pq] + 1);
-        deps.push_back({pq, p});
-      }
+      const int q = ij + o;
+      if (colour[q] != c || lev[q] < 0) continue;
+      L = std::max(L, lev[q] + 1);
+      deps.push_back({q, ij});
     }
-    lev[p] = L;
+    if (L >= kMaxLevels) return "colour level depth exceeds the schedule limit";
+    lev[ij] = (signed char)L;
     maxlev = std::max(maxlev, L);
   }
-  if (maxlev + 1 > kMaxLevels) return "colour level depth exceeds the schedule limit";
   g.nlev = maxlev + 1;
   // row bands: 0-based ext rows [4, nmu); band 0 must hold rows 4..9 (the
   // mu=1 extrapolation reads rows 5..9), ~4 rows each, merged until every
@@ -420,7 +382,7 @@ static std::string build_schedule(HostGrid &g) {
   for (bool changed = true; changed;) {
     changed = false;
     for (auto &d : deps) {
-      int ra = g.order[d.first] / g.n8, rb = g.order[d.second] / g.n8;
+      int ra = d.first / n8, rb = d.second / n8;
       int ta = band_of(ra), tb = band_of(rb);
       if (ta != tb) {
         int lo = std::min(ta, tb), hi = std::max(ta, tb);
@@ -434,22 +396,22 @@ static std::string build_schedule(HostGrid &g) {
   g.tile_row0.assign(bounds.begin(), bounds.end() - 1);
   g.tile_row1.assign(bounds.begin() + 1, bounds.end());
   // bucket points by (tile, colour, level), list order inside each bucket
+  std::vector<int> tile(nmu);  // by ext row
+  for (int row = 4; row < nmu; ++row) tile[row] = band_of(row);
+  auto bucket = [&](int p) { return (tile[packed[p] >> 16] * 5 + colour[g.order[p]]) * g.nlev + lev[g.order[p]]; };
   const int nb = g.ntiles * 5 * g.nlev;
-  std::vector<int> cnt(nb + 1, 0);
+  g.off.assign(nb + 1, 0);
+  for (int p = 0; p < npts; p++) g.off[bucket(p) + 1]++;
+  for (int k = 0; k < nb; k++) g.off[k + 1] += g.off[k];
+  g.pts.resize(npts);
+  std::vector<int> rc(npts), fill(g.off.begin(), g.off.end() - 1);
   for (int p = 0; p < npts; p++) {
-    int t = band_of(g.order[p] / g.n8);
-    cnt[(t * 5 + p % 5) * g.nlev + lev[p] + 1]++;
+    const int at = fill[bucket(p)]++;
+    g.pts[at] = g.order[p];
+    rc[at] = packed[p];
   }
-  for (int k = 0; k < nb; k++) cnt[k + 1] += cnt[k];
-  g.off = cnt;
-  g.pts.assign(npts, 0);
-  std::vector<int> fill(cnt.begin(), cnt.end() - 1);
-  for (int p = 0; p < npts; p++) {
-    int t = band_of(g.order[p] / g.n8);
-    g.pts[fill[(t * 5 + p % 5) * g.nlev + lev[p]]++] = g.order[p];
-  }
-  g.st_pts.clear();
-  g.st_pts.reserve(g.pts.size());
+  g.st_pts.reserve(npts);
+  g.st_place.resize(npts);
   g.st_off.assign(size_t(5) * g.nlev * (g.ntiles + 1), 0);
   for (int c = 0; c < 5; ++c)
     for (int l = 0; l < g.nlev; ++l) {
@@ -457,11 +419,14 @@ static std::string build_schedule(HostGrid &g) {
       for (int t = 0; t < g.ntiles; ++t) {
         so[t] = int(g.st_pts.size());
         const int o = (t * 5 + c) * g.nlev + l;
-        for (int k = g.off[o]; k < g.off[o + 1]; ++k) g.st_pts.push_back(((g.pts[k] / g.n8) << 16) | (g.pts[k] % g.n8));
+        for (int k = g.off[o]; k < g.off[o + 1]; ++k) {
+          g.st_place[((rc[k] >> 16) - 5) * (nni - 2) + (rc[k] & 0xffff) - 5] = int(g.st_pts.size());
+          g.st_pts.push_back(rc[k]);
+        }
       }
       so[g.ntiles] = int(g.st_pts.size());
     }
-  for (int G = 1; G <= HostGrid::kBandRuns; ++G) {
+  for (int G = 1; G <= Schedule::kBandRuns; ++G) {
     int most = 0;
     for (int t0 = 0; t0 < g.ntiles; t0 += G) {
       const int t1 = std::min(t0 + G, g.ntiles);
@@ -472,53 +437,38 @@ static std::string build_schedule(HostGrid &g) {
   // final check: no two points of one (tile,colour,level) bucket interact,
   // and every dependency is inside a tile with a strictly larger level
   for (auto &d : deps) {
-    int ra = g.order[d.first] / g.n8, rb = g.order[d.second] / g.n8;
+    int ra = d.first / n8, rb = d.second / n8;
     if (band_of(ra) != band_of(rb)) return "schedule check: dependency crosses a tile";
     if (!(lev[d.second] > lev[d.first])) return "schedule check: level order violated";
   }
-  g.columns.clear();
   for (int size = 1; size <= kMaxCluster; ++size)
     for (int groups = 1; groups <= 2; ++groups) {
       ColPlan cp;
       if (column_plan(nni, nmu, size, groups, cp)) g.columns.push_back(cp);
     }
-  std::string msg = build_wave_schedule(g, g.order, offs, g.sor);
+  std::string msg = build_wave_schedule(g, g.order, packed, offs, g.sor);
   if (!msg.empty()) return msg;
   build_march(g);
-  std::vector<int> by_colour;
-  by_colour.reserve(g.order.size());
+  std::vector<int> order, at;
+  order.reserve(npts);
+  at.reserve(npts);
   for (int c = 0; c < 5; ++c)
-    for (int p = c; p < npts; p += 5) by_colour.push_back(g.order[p]);
-  return build_wave_schedule(g, by_colour, offs, g.mcsor);
+    for (int p = c; p < npts; p += 5) {
+      order.push_back(g.order[p]);
+      at.push_back(packed[p]);
+    }
+  return build_wave_schedule(g, order, at, offs, g.mcsor);
 }
 
 
 namespace {
 struct ScheduleCache {
   std::mutex m;
-  std::vector<std::shared_ptr<const HostGrid>> entries;  // most recent last
+  std::vector<std::shared_ptr<const Schedule>> entries;  // most recent last
 };
 ScheduleCache &schedule_cache() {
   static ScheduleCache c;
   return c;
-}
-void copy_schedule(HostGrid &to, const HostGrid &from) {
-  to.order = from.order;
-  to.ntiles = from.ntiles;
-  to.nlev = from.nlev;
-  to.tile_row0 = from.tile_row0;
-  to.tile_row1 = from.tile_row1;
-  to.pts = from.pts;
-  to.off = from.off;
-  to.st_pts = from.st_pts;
-  to.st_off = from.st_off;
-  for (int k = 0; k <= HostGrid::kBandRuns; ++k) to.st_rows[k] = from.st_rows[k];
-  to.columns = from.columns;
-  to.sor = from.sor;
-  to.march_pts = from.march_pts;
-  to.march_mask = from.march_mask;
-  to.march_off = from.march_off;
-  to.mcsor = from.mcsor;
 }
 constexpr size_t kScheduleCacheEntries = 8;
 }  // namespace
@@ -529,18 +479,18 @@ std::string attach_schedule(HostGrid &g) {
     std::lock_guard<std::mutex> lock(c.m);
     for (auto &e : c.entries)
       if (e->nni == g.nni && e->nmu == g.nmu) {
-        copy_schedule(g, *e);
+        g.s = e;
         return "";
       }
   }
-  std::string msg = build_schedule(g);
+  auto made = std::make_shared<Schedule>();
+  made->nni = g.nni;
+  made->nmu = g.nmu;
+  std::string msg = build_schedule(*made);
   if (!msg.empty()) return msg;
-  auto keep = std::make_shared<HostGrid>();
-  keep->nni = g.nni;
-  keep->nmu = g.nmu;
-  copy_schedule(*keep, g);
+  g.s = made;
   std::lock_guard<std::mutex> lock(c.m);
-  c.entries.push_back(std::move(keep));
+  c.entries.push_back(std::move(made));
   if (c.entries.size() > kScheduleCacheEntries) c.entries.erase(c.entries.begin());
   return "";
 }
@@ -583,9 +533,10 @@ extern "C" int x2g_host_table(int nnu, int nmu, double r, double rinf, double z1
 // 0-based, reference list order), tile/colour/level of every point.
 extern "C" int x2g_host_schedule(int nnu, int nmu, int *npoints, int *ntiles, int *nlevels, int *order,
                                  int *tile, int *colour, int *level) {
-  x2g::HostGrid g;
-  std::string msg = x2g::build_host_grid(g, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
+  x2g::HostGrid grid;
+  std::string msg = x2g::build_host_grid(grid, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
   if (!msg.empty()) return X2G_ERR_SCHEDULE;
+  const x2g::Schedule &g = *grid.s;
   if (npoints) *npoints = int(g.order.size());
   if (ntiles) *ntiles = g.ntiles;
   if (nlevels) *nlevels = g.nlev;
@@ -608,15 +559,16 @@ extern "C" int x2g_host_schedule(int nnu, int nmu, int *npoints, int *ntiles, in
 
 extern "C" int x2g_host_band_schedule(int nnu, int nmu, int *npoints, int *ntiles, int *nlevels, int *pts, int *off,
                                       int *rows, int *tile_row0, int *tile_row1) {
-  x2g::HostGrid g;
-  std::string msg = x2g::build_host_grid(g, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
+  x2g::HostGrid grid;
+  std::string msg = x2g::build_host_grid(grid, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
   if (!msg.empty()) return X2G_ERR_SCHEDULE;
+  const x2g::Schedule &g = *grid.s;
   if (npoints) *npoints = int(g.st_pts.size());
   if (ntiles) *ntiles = g.ntiles;
   if (nlevels) *nlevels = g.nlev;
   if (pts) std::copy(g.st_pts.begin(), g.st_pts.end(), pts);
   if (off) std::copy(g.st_off.begin(), g.st_off.end(), off);
-  if (rows) std::copy(g.st_rows, g.st_rows + x2g::HostGrid::kBandRuns + 1, rows);
+  if (rows) std::copy(g.st_rows, g.st_rows + x2g::Schedule::kBandRuns + 1, rows);
   if (tile_row0) std::copy(g.tile_row0.begin(), g.tile_row0.end(), tile_row0);
   if (tile_row1) std::copy(g.tile_row1.begin(), g.tile_row1.end(), tile_row1);
   return X2G_OK;
@@ -629,14 +581,15 @@ extern "C" int x2g_host_band_schedule(int nnu, int nmu, int *npoints, int *ntile
 // Null arrays: counts only.
 extern "C" int x2g_host_sor_schedule(int nnu, int nmu, int *npoints, int *nlev, int *nblev, int *delta, int *pts,
                                      int *off, int *bpts, int *boff) {
-  x2g::HostGrid g;
-  std::string msg = x2g::build_host_grid(g, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
+  x2g::HostGrid grid;
+  std::string msg = x2g::build_host_grid(grid, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4);
   if (!msg.empty()) return X2G_ERR_SCHEDULE;
-  if (npoints) *npoints = int(g.sor.pts.size());
+  const x2g::Schedule &g = *grid.s;
+  if (npoints) *npoints = int(g.sor.pts.size() / 2);
   if (nlev) *nlev = g.sor.nlev;
   if (nblev) *nblev = g.sor.nblev;
   if (delta) *delta = g.sor.delta;
-  if (pts) std::copy(g.sor.pts.begin(), g.sor.pts.end(), pts);
+  for (size_t k = 0; pts && k < g.sor.pts.size() / 2; ++k) pts[k] = g.sor.pts[2 * k];
   if (off) std::copy(g.sor.off.begin(), g.sor.off.end(), off);
   if (bpts) std::copy(g.sor.bpts.begin(), g.sor.bpts.end(), bpts);
   if (boff) std::copy(g.sor.boff.begin(), g.sor.boff.end(), boff);

@@ -55,7 +55,7 @@ static void append_chunks(std::vector<std::pair<int, int>> &pts, int r0, int n8,
 // along a row or a column always have another colour and the points of one
 // colour are independent.  Per (CTA, colour) segment A (no halo read or write),
 // B (within 4 rows of a shared band edge), and an empty seam segment.
-void free_chunks(const HostGrid &g, const std::vector<int> &r0, TilePlan &plan) {
+void free_chunks(const Schedule &g, const std::vector<int> &r0, TilePlan &plan) {
   const int C = int(r0.size()) - 1;
   plan.free_off.push_back(0);
   for (int k = 0; k < C; ++k) {
@@ -79,7 +79,7 @@ void free_chunks(const HostGrid &g, const std::vector<int> &r0, TilePlan &plan) 
 // (halos come from the next CTA only); shared memory per CTA for (residual,
 // omega/lhs) pairs, the correction band with 4-row halos, b(mu) of the band's
 // rows, d(nu) by column, the segment offsets and the CTA's chunks.
-TilePlan tile_plan(const HostGrid &g) {
+TilePlan tile_plan(const Schedule &g) {
   TilePlan plan;
   const int rows = g.nmu - 4, C = std::min(std::max(2, std::min(16, (rows + 29) / 30)), g.ntiles);
   if (C < 2) return plan;
@@ -156,7 +156,7 @@ TilePlan tile_plan(const HostGrid &g) {
 int host_tile_plan(int nnu, int nmu, TilePlan &plan) {
   HostGrid g;
   if (!build_host_grid(g, nnu, nmu, 2.0, 40.0, 1.0, 1.0, 4).empty()) return X2G_ERR_SCHEDULE;
-  plan = tile_plan(g);
+  plan = tile_plan(*g.s);
   return X2G_OK;
 }
 
