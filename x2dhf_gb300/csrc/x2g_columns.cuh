@@ -129,11 +129,9 @@ __device__ __forceinline__ void push_halo(unsigned addr, float v, unsigned bar) 
 }
 // (negative: nothing)
 __device__ __forceinline__ void expect_bytes(unsigned bar, int bytes) {
-  asm volatile(
-      "{\n\t.reg .b64 t;\n\t.reg .pred p;\n\tsetp.ge.s32 p, %1, 0;\n\t"
-      "@p mbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(bar),
-      "r"(bytes)
-      : "memory");
+  if (bytes >= 0)
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes)
+                 : "memory");
 }
 __device__ __forceinline__ bool poll_bar(unsigned bar, unsigned parity) {
   unsigned ok;
@@ -155,7 +153,7 @@ __device__ __forceinline__ bool test_bar(unsigned bar, unsigned parity) {
 // a wait for a neighbour's halo values, a few polls as a rule; false: it ran
 // out (now recorded), or another one did
 __device__ __forceinline__ bool wait_halo(unsigned bar, unsigned parity, const BarrierDev &b) {
-  if (test_bar(bar, parity)) return true;
+  if (b.limit_ns != 0 ? poll_bar(bar, parity) : test_bar(bar, parity)) return true;
   unsigned long long t0 = 0;
   for (unsigned k = 1; b.limit_ns != 0; ++k) {
     if (poll_bar(bar, parity)) return true;
