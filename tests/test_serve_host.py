@@ -107,3 +107,18 @@ def test_other_errors_stop_the_run():
     with pytest.raises(RuntimeError):
         serve.Server(slots=2, backend=Broken()).run(serve.make_requests(TEMPLATES, 4, rate=0.0, seed=1),
                                                    realtime=False)
+
+
+def test_footprint_holds_the_relaxations_workspace():
+    """N2 on 331 x 481: the FP64 forms keep a 16-byte copy and two 16-byte
+    pairs per point of each of its 22 potentials, the mixed form 12 bytes; no
+    form, the larger.  A large grid's launches share 256 MiB or one function's."""
+    deck = serve.request_deck(TEMPLATES["n2"], 2.068, 331, 481)
+    c = xg.parse_deck(deck)
+    bare = (3 * 6 + 22) * 339 * 489 * 8 + 60 * 331 * 481 * 8
+    fp64, mixed, either = (serve.footprint_bytes(c, p) for p in (xg.FP64, xg.MIXED, None))
+    assert fp64 >= bare + 22 * (16 * 339 * 489 + 32 * 331 * 481)
+    assert mixed >= bare + 22 * 12 * 331 * 481
+    assert either == max(fp64, mixed)
+    assert serve.scratch_bytes(781, 1201, 33, xg.FP64) <= 1.25 * (256 << 20)
+    assert serve.scratch_bytes(2401, 2401, 4, xg.FP64) >= 48 * 2401 * 2401

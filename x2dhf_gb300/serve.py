@@ -88,19 +88,35 @@ def request_deck(template_deck, r, nnu, nmu, maxscf=3000):
     return "\n".join(out) + "\n"
 
 
-def footprint_bytes(case):
-    """Device bytes of one solve: orbitals, Coulomb and exchange potentials
-    and per-orbital work arrays in the extended layout, plus the grid's
-    tables (the closed-shell pair rule: one exchange potential per pair, two
-    for a pair of non-sigma orbitals, one self-exchange per non-sigma
-    orbital)."""
+def scratch_bytes(nnu, nmu, jobs, precision=None):
+    """Device workspace of a context after relaxing `jobs` functions in one
+    call: in the FP64 forms a tagged copy of each function and its (lhs, rhs)
+    pairs with reciprocals, for at most 32 functions and 256 MiB a launch (or
+    one function's), in the mixed form the FP32 correction, residual and omega /
+    lhs of each; grown by a quarter more than asked for.  precision None: the
+    larger."""
+    ext, plain = (nnu + 8) * (nmu + 8), nnu * nmu
+    wave = -(-16 * ext // 256) * 256 + -(-32 * plain // 256) * 256
+    fp64 = wave * max(1, min(jobs, 32, (256 << 20) // wave))
+    mixed = (4 * ext + 8 * plain + 512) * jobs
+    need = max(fp64, mixed) if precision is None else mixed if precision == MIXED else fp64
+    return need + need // 4
+
+
+def footprint_bytes(case, precision=None):
+    """Device bytes of one solve: orbitals, Coulomb and exchange potentials in
+    the extended layout (the closed-shell pair rule: one exchange potential per
+    pair, two for a pair of non-sigma orbitals, one self-exchange per non-sigma
+    orbital), the per-orbital work arrays, the grid's tables and schedules, and
+    the relaxations' workspace with every potential in one call.  precision:
+    the form the solve relaxes in (None: whichever takes more)."""
     m = [int(case.m[i]) for i in range(case.norb)]
     n = len(m)
     pots = n + sum(1 + (1 if (m[i] > 0 and m[j] > 0) else 0) for i in range(n) for j in range(i + 1, n))
     pots += sum(1 for x in m if x > 0)
     ext = (case.nnu + 8) * (case.nmu + 8) * 8
     plain = case.nnu * case.nmu * 8
-    return (3 * n + pots) * ext + 60 * plain
+    return (3 * n + pots) * ext + (2 * n + 66) * plain + scratch_bytes(case.nnu, case.nmu, pots, precision)
 
 
 def make_requests(templates, n, rate, seed=42):
