@@ -273,7 +273,8 @@ int x2g_putout(x2g_ctx *ctx, x2g_grid *grid, const double *work_ext, double *fun
 
 /* Host-buffer form of one relaxation call, the unit the reference's
  * mcsor_pthread_ performs (mcsor_pthread.c:32): copies wk2/lhs/rhs to the
- * device, relaxes, copies wk2 back.  kind as in x2g_job. */
+ * device, relaxes, copies wk2 back.  kind as in x2g_job.  Threads that make it
+ * on one context at the same time take turns. */
 int x2g_mcsor_host(x2g_ctx *ctx, x2g_grid *grid, int isym, int kind, double omega, int nsweeps,
                    double *wk2_ext_host, const double *lhs_host, const double *rhs_host);
 

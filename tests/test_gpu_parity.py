@@ -965,3 +965,41 @@ def test_tall_and_flat_grids_run_on_chip(ctx, nnu, nmu):
     assert min(g.cluster_occupancy()) > 0
     g.close()
     test_column_sweep_matches_band_sweep(ctx, nnu, nmu, 2, 3)
+
+
+def test_host_calls_of_threads_on_one_context(ctx):
+    """mcsor_host calls of several threads on one context, which share its
+    device arrays, on grids of growing size: each as alone, bit for bit."""
+    import threading
+    rng = np.random.default_rng(17)
+    cases = []
+    for nnu, nmu in ((31, 61), (91, 121), (151, 181), (181, 241)):
+        oc = Case(_grid_deck(nnu, nmu))
+        u = oc.putin(1, rng.standard_normal(nnu * nmu))
+        lhs, rhs = oc.fock(1)[0] + oc.coeffs()[5], rng.standard_normal(nnu * nmu)
+        cases.append((_grid(ctx, _grid_deck(nnu, nmu))[1], oc.omega()[0], u, lhs, rhs))
+
+    def call(g, omega, u, lhs, rhs):
+        return xg.mcsor_host(ctx, g, 1, 0, omega, 10, u.copy(), lhs, rhs)
+
+    alone = [call(*c) for c in cases]
+    fresh = xg.Context(0)  # whose arrays are still to grow
+    grids = [xg.Grid(fresh, g.nnu, g.nmu, 2.0, 25.0, 1.0, 1.0) for g, *_ in cases]
+    got = [[] for _ in cases]
+
+    def work(k):
+        g, omega, u, lhs, rhs = cases[k]
+        for _ in range(8):
+            got[k].append(xg.mcsor_host(ctx, g, 1, 0, omega, 10, u.copy(), lhs, rhs))
+            xg.mcsor_host(fresh, grids[k], 1, 0, omega, 2, u.copy(), lhs, rhs)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(cases))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k, outs in enumerate(got):
+        assert len(outs) == 8 and all(np.array_equal(x, alone[k]) for x in outs), k
+    for g in grids + [c[0] for c in cases]:
+        g.close()
+    fresh.close()

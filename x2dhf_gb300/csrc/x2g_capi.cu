@@ -532,13 +532,15 @@ int x2g_putout(x2g_ctx *ctx, x2g_grid *grid, const double *work, double *fun) {
 
 // The device arrays belong to the context: allocated from the stream-ordered
 // pool and given back in every call, they cost 170 us of the 480 that ten sweeps
-// of 91 x 121 took (the pool returns its memory at each synchronisation).
+// of 91 x 121 took (the pool returns its memory at each synchronisation).  One
+// call of a context at a time has them; other threads' wait.
 int x2g_mcsor_host(x2g_ctx *ctx, x2g_grid *grid, int isym, int kind, double omega, int nsweeps, double *wk2,
                    const double *lhs, const double *rhs) {
   if (!ctx || !grid || !wk2 || !lhs || !rhs) return set_status(X2G_ERR_ARG, "null argument");
   if (kind != 0 && kind != 1) return set_status(X2G_ERR_ARG, "kind must be 0 or 1");
   const GridDev &g = grid->d;
   const size_t eb = size_t(g.next) * sizeof(double), pb = size_t(g.mxsize) * sizeof(double);
+  std::lock_guard<std::mutex> lock(ctx->host_call);
   double *buf = static_cast<double *>(ctx_buffer(ctx, ctx->host_arrays, ctx->host_arrays_bytes, eb + 2 * pb));
   if (!buf) return set_status(X2G_ERR_CUDA, "mcsor buffers: out of memory");
   double *du = buf, *dl = buf + g.next, *dr = dl + g.mxsize;

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <string>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "../../include/x2dhf_gpu.h"
@@ -252,6 +253,7 @@ struct x2g_ctx {
   // reusable device workspace
   void *work = nullptr;
   size_t work_bytes = 0;
+  std::mutex host_call;         // held by a call on host arrays, which shares the next two
   void *host_arrays = nullptr;  // device copies of a host call's arrays
   size_t host_arrays_bytes = 0;
   void *red = nullptr;  // reduction partials
