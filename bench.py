@@ -40,15 +40,22 @@ UNIT = "SCF solves/s"
 BYTES_PER_PT = {0: 32.0, 1: 16.0}
 FLOPS_PER_PT = 54.0
 # DRAM bytes (read + write) per point-update of the on-chip cluster sweep,
-# from ncu (dram__bytes_read.sum + dram__bytes_write.sum = 2 765 824 + 0) of
-# one single-job, 10-sweep launch on 331x481 (1 566 040 point-updates): the
-# correction, residual and omega/lhs stay in shared memory, so DRAM sees only
-# the band load (the u += e writeback was still in L2 when the launch ended)
-CLUSTER_DRAM_BYTES_PER_PT = 2765824.0 / 1566040.0
+# from ncu (dram__bytes_read.sum + dram__bytes_write.sum = 43.5 MB) of one
+# launch of 22 potentials, 10 sweeps, on 331x481 (34 452 880 point-updates): the
+# correction stays in shared memory, so DRAM sees the residual, u and omega / lhs
+# once
+CLUSTER_DRAM_BYTES_PER_PT = 43.5e6 / 34452880.0
 # the same for the persistent-band sweep of grids beyond one cluster, from
 # ncu of two 6-job, 10-sweep launches on 781x1201 (71.38 + 1.57 MB read + write
 # per launch, 55 901 040 point-updates)
 BAND_DRAM_BYTES_PER_PT = (71379200.0 + 1573120.0) / 55901040.0
+
+
+def sweeps_on_chip(occupancy):
+    """Whether the mixed form's sweeps of a grid run on chip, from its
+    co-resident clusters of the plain kernel (0: it takes the persistent-band
+    sweep) and of the potentials' variant."""
+    return occupancy[0] > 0
 
 
 def n2_deck(grid="337 481 40.0"):
@@ -405,12 +412,10 @@ def run_gpu(args):
     rate = {n: world * len(lat[n]) * per_step / tot[n] for n in names}
     value = rate[head[0]]
     e2e_value = world * len(late2e) * per_step / tote2e
-    on_chip = xg.host_cluster_plan(c.nnu, c.nmu)[0] > 0
-    occ = (0, 0)
-    if on_chip:
-        g = xg.Grid(ctx, c.nnu, c.nmu, c.r, c.rinf, c.z1, c.z2)
-        occ = g.cluster_occupancy()
-        g.close()
+    g = xg.Grid(ctx, c.nnu, c.nmu, c.r, c.rinf, c.z1, c.z2)
+    occ = g.cluster_occupancy()
+    g.close()
+    on_chip = sweeps_on_chip(occ)
     hs = sorted(lat[head[0]])
     p99 = hs[min(len(hs) - 1, int(round(0.99 * (len(hs) - 1))))]
     # bytes the library copied per timed e2e step (grid tables up; per-iteration
@@ -484,7 +489,7 @@ def run_gpu(args):
             "bytes_per_point_update": BYTES_PER_PT[1],
             "note": ("achieved = 16 algorithmic B per point-update / launch time; the correction lives in shared "
                      "memory during the sweeps, so DRAM traffic is far below it and the launch is bound by "
-                     "instruction issue and the latency of a colour phase, not by HBM" if on_chip else
+                     "the latency of a colour phase (its loads, halo values and barrier), not by HBM" if on_chip else
                      "achieved = 16 algorithmic B per point-update / launch time; the correction stays in shared "
                      "memory for the whole launch, so DRAM traffic stays far below the algorithmic bytes and the "
                      "launch is bound by phase latency (neighbour wait, halo round trip, level chain), not by HBM"),

@@ -4,6 +4,8 @@ import os
 import subprocess
 import sys
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
@@ -79,3 +81,20 @@ def test_sweeps_leg_deck_sets_maxsor():
     assert (c40.maxsor_orb, c40.maxsor_pot) == (40, 40)
     assert (c40.orb_scheme, c40.pot_scheme) == (c0.orb_scheme, c0.pot_scheme) == (1, 1)
     assert (c40.nnu, c40.nmu, c40.r) == (c0.nnu, c0.nmu, c0.r)
+
+
+@pytest.mark.parametrize("nnu,nmu,on_chip", [(331, 481, True), (451, 541, True), (91, 901, True), (781, 1201, False)])
+def test_kernel_named_is_the_one_that_runs(nnu, nmu, on_chip):
+    """The bench names the sweep kernel by the clusters of the kernels that run,
+    as their band plans have them (one cluster where a plan's kernel fits an SM)."""
+    import bench
+    import x2dhf_gb300 as xg
+
+    fits = [0, 0]
+    for potentials in (0, 1):
+        for size in range(1, 17):
+            for groups in (1, 2):
+                p = xg.host_column_plan(nnu, nmu, size, groups, potentials)
+                if p and p["kernel_slots"] and p["smem"] <= 227 * 1024:
+                    fits[potentials] += 1
+    assert bench.sweeps_on_chip(tuple(fits)) == on_chip
