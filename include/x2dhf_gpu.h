@@ -177,7 +177,10 @@ int x2g_set_mixed_on_chip(x2g_ctx *ctx, int on);
  * lhs from a row and a column term instead of keeping it on chip, so that two
  * CTAs fit each SM and twice the clusters are co-resident.
  * mode 0 never, 1 always, 2 (default) for batches larger than the clusters
- * of the plain kernel co-resident on the device.  No reference counterpart. */
+ * of the plain kernel co-resident on the device.  Its FP64 residuals, and in
+ * modes 1 and 2 those of grids of 2^16 points or more that no on-chip kernel
+ * holds, are summed in fixed point; mode 0 and the plain kernel use FMAs.  No
+ * reference counterpart. */
 int x2g_set_potential_clusters(x2g_ctx *ctx, int mode);
 /* Batch mode 2, no orbital frozen: the orthonormalisation of an SCF
  * iteration (normOrtho.F90:14-59,103-207 for every orbital in the

@@ -958,7 +958,8 @@ def test_large_band_blocks_match_single_jobs(ctx, njobs, nsweeps):
 
 # grids of few columns and many rows (more points of a colour per thread, three row pitches) and of many columns and few
 # rows (25 warps)
-@pytest.mark.parametrize("nnu,nmu", [(241, 901), (271, 811), (151, 1201), (121, 1831), (91, 2431), (541, 31), (781, 31)])
+@pytest.mark.parametrize("nnu,nmu", [(241, 901), (271, 811), (331, 931), (241, 1591), (151, 1201),
+                                     (121, 1831), (91, 2431), (541, 31), (781, 31), (571, 241), (511, 631)])
 def test_tall_and_flat_grids_run_on_chip(ctx, nnu, nmu):
     torch = pytest.importorskip("torch")
     g = xg.Grid(ctx, nnu, nmu, 2.0, 25.0, 1.0, 1.0)

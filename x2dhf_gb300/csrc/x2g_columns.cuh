@@ -28,14 +28,20 @@
 // counted on the receiver's barrier: a cluster barrier per phase took 440
 // cycles, 665 with plain stores into the neighbours' memory to drain.
 //
-// What bounds it: instruction issue (per slot of 32 points 17 loads and stores
-// and 20 packed operations of two roundings each, 12 for potentials), at 0.45
-// per cycle and SM quarter, and a fifth of a phase at its barrier; where a launch
-// is small, the latency of a phase (0.9 us at three slots).  Against the sweep
-// with a list of points per warp and a cluster barrier per colour and level (10
-// sweeps, us): one orbital of 151 x 241 58 (106), of 331 x 481 97 (132), six 101
-// (132), 22 potentials of 331 x 481 173 (two waves, 382; 210 with relax_f32's
-// order of operations).
+// Every wait is bounded by the context's limit and looks at its error word.
+// After one that runs out (or where the word is set before the launch) a block
+// leaves the sweeps at the next sweep's start, tells its cluster, and no block of
+// it writes u.
+//
+// What bounds it: waiting.  An instruction issues in two cycles of five (70 of a
+// warp per slot of 32 points: 17 loads and stores, 20 packed operations of two
+// roundings each, 12 for potentials, addresses and moves), no pipe is above 52 %:
+// the warps wait for their loads, for the instruction before and, 1.5 stalls per
+// issue, at the phase's barrier; where a launch is small, for the latency of a
+// phase (0.9 us at three slots).  Against the sweep with a list of points per warp
+// and a cluster barrier per colour and level (10 sweeps, us): one orbital of 151 x
+// 241 58 (106), of 331 x 481 98 (132), six 101 (132), 22 potentials of 331 x 481 174
+// (two waves, 382; 210 with relax_f32's order of operations).
 #pragma once
 
 #include <cooperative_groups.h>

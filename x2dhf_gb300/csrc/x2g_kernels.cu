@@ -2565,7 +2565,7 @@ static const std::vector<x2g_ctx::ColumnShape> &column_shapes(x2g_ctx *ctx, cons
 // one group of SMs).  Measured, us: 151x241, two threads per column: 3 slots
 // 57, 4 66, 5 74; 331x481 likewise: 4 slots 96, 5 114; one thread per column,
 // one CTA on an SM: 7 slots 117, 9 139, two: 7 160, 9 207.  So 22 potentials
-// of 331x481 run as one wave of 12-CTA clusters (209) and not as two of 16-CTA
+// of 331x481 run as one wave of 11-CTA clusters (209) and not as two of 16-CTA
 // ones (320), 64 of 151x241 as two launches of 32 (214; 287 on the kernel with
 // fixed clusters of 8).
 static double column_time(const ColPlan &p, int jobs, int num_sms) {
@@ -2833,8 +2833,8 @@ static bool march_fits(x2g_ctx *ctx, size_t smem) {
 // FP64 relaxation over the wavefront schedule w, in cooperative launches of
 // at most kParamJobs jobs and kWaveScratch bytes of scratch (the tagged copy
 // and the (lhs, rhs) pairs of a launch's jobs, used by the launches in turn;
-// 32 jobs of 331 x 481 are 167 MB, about what L2 holds, and a launch of one
-// 781 x 1201 job already has points enough in a step to fill the GPU).
+// 32 jobs of 331 x 481 are 248 MB, and a launch of one 781 x 1201 job already has
+// points enough in a step to fill the GPU).
 constexpr size_t kWaveScratch = size_t(256) << 20;
 static int relax_wave(x2g_ctx *ctx, const GridDev &g, const WaveDev &w, const x2g_job *jobs, int njobs, int nsweeps,
                       bool profile, const MarchDev *march = nullptr) {

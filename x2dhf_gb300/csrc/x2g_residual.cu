@@ -110,9 +110,11 @@ __global__ void k_residual(GridDev g, const __grid_constant__ JobTable jobs, int
 // points of 331 x 481 and 15 % of 151 x 241, that lie in 20 and 44 % of a warp's
 // rows).
 //
-// What bounds it: its warps wait for the tile and the orbitals, then for the
-// products, about 300 instructions a point of which 96 are the products (two
-// each); 8 rows per warp share the column's weights and its values.
+// What bounds it: waiting (issue in two cycles of five, the FP64 pipe 39 % busy):
+// for the tile and the orbitals, then for the products one after the other, about
+// 300 instructions a point of which 96 are the products (two each); 8 rows per
+// warp share the column's weights and its values.  22 potentials of 331 x 481: 75
+// us in an SCF, 90 with a third of them of azimuthal number 2; with FMAs 149.
 constexpr int kTile = 32;           // columns and rows of a block's tile
 constexpr int kSpan = kTile + 8;    // with the stencil's four on each side
 constexpr int kRowsPerWarp = 8;
