@@ -2975,8 +2975,11 @@ int launch_relax(x2g_ctx *ctx, x2g_grid *grid, const x2g_job *jobs, int njobs, i
     set_status(X2G_OK, "");
   }
   // their stencil sums in fixed point with the potentials' kernel, and on grids
-  // that no on-chip kernel holds, where a function alone has tiles enough (22 of
-  // 331x481 80 us, FMAs 149; 22 of 151x241 42 and 54; one of 331x481 13 and 14).
+  // that no on-chip kernel holds, where a function alone has tiles enough (smooth
+  // functions, us, and by FMAs: 22 of 331x481 61 and 149, one of 811x121 9.0 and
+  // 10.1, seven of 781x1201 116 and 345; one of 151x241 8.8 and 6.5.  Points left
+  // to FMAs make a tail of some us: with the plain kernel, four of 301x481 with
+  // azimuthal numbers 0 to 2 take 4 us longer so than by FMAs alone).
   // The kernel and the grid decide, not the number of jobs, so that a function's
   // result does not depend on its batch, and the plain kernel's results (mode 0,
   // SCFs in the reference's order) stay the persistent-band sweep's
